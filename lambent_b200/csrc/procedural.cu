@@ -90,7 +90,8 @@ LAM_DEV void proc_trace(const DevScene& S, const lam_ray* __restrict__ rays, uin
         hits[i] = h;
     };
     trace_persistent<ANY, true>(S, tl, in, n, counter, err, load, store);
-    if (err) atomicOr(err_out, err);
+    if (err) *err_out = err;  // mapped host memory; one flag only, so a plain store
+    trace_done(counter);
 }
 
 extern "C" __global__ void __launch_bounds__(TRACE_BLOCK)

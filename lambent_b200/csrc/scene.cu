@@ -60,6 +60,23 @@ static int upload(lam_scene* s, const T* host, size_t count, const T** dev, cuda
 static void free_scene(lam_scene* s) {
     for (void* p : s->allocations) cudaFree(p);
     s->allocations.clear();
+    if (s->trace_flags) cudaFreeHost(s->trace_flags);
+    s->trace_flags = nullptr;
+}
+
+static int alloc_trace_slots(lam_scene* s, cudaStream_t st) {
+    cudaError_t e = cudaHostAlloc((void**)&s->trace_flags, TRACE_SLOTS * sizeof(uint32_t), cudaHostAllocMapped);
+    if (e == cudaSuccess) {
+        std::memset(s->trace_flags, 0, TRACE_SLOTS * sizeof(uint32_t));
+        e = cudaHostGetDevicePointer((void**)&s->trace_flags_dev, s->trace_flags, 0);
+    }
+    const size_t bytes = TRACE_SLOTS * TRACE_SLOT_WORDS * sizeof(uint32_t);
+    if (e == cudaSuccess) e = cudaMalloc((void**)&s->trace_words, bytes);
+    if (e == cudaSuccess) {
+        s->allocations.push_back(s->trace_words);
+        e = cudaMemsetAsync(s->trace_words, 0, bytes, st);
+    }
+    return e == cudaSuccess ? LAM_OK : cuda_error(e, "ray query scratch");
 }
 
 }  // namespace lam
@@ -287,12 +304,14 @@ extern "C" int lam_scene_create(const lam_scene_desc* d, void* stream, lam_scene
 
     lam_scene* s = new lam_scene();
     cudaGetDevice(&s->device);
+    cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->device);
     DevScene& D = s->dev;
     auto fail = [&](int code) {
         free_scene(s);
         delete s;
         return code;
     };
+    if ((rc = alloc_trace_slots(s, st))) return fail(rc);
     if ((rc = upload(s, reinterpret_cast<const uint4*>(blas_nodes.data()), blas_nodes.size() * 5, &D.blas_nodes, st))) return fail(rc);
     if ((rc = upload(s, reinterpret_cast<const uint4*>(tlas.nodes.data()), tlas.nodes.size() * 5, &D.tlas_nodes, st))) return fail(rc);
     if ((rc = upload(s, tris.data(), tris.size(), &D.tris, st))) return fail(rc);
@@ -425,7 +444,60 @@ __global__ void __launch_bounds__(TRACE_BLOCK) trace_rays_kernel(DevScene S, con
         hits[i] = h;
     };
     trace_persistent<ANY, ALPHA>(S, tl, in, n, counter, err, load, store);
-    if (err) atomicOr(err_out, err);
+    if (err) *err_out = err;  // possibly mapped host memory; one flag only, so a plain store
+    trace_done(counter);
+}
+
+static cudaError_t launch_trace(const lam_scene* s, const lam_ray* rays, uint32_t n, uint32_t mode, lam_hit* hits,
+                                uint32_t* words, uint32_t* flags, cudaStream_t st) {
+    const dim3 grid(s->sms * 8), block(TRACE_BLOCK);
+    const bool alpha = !s->dev.all_opaque;
+    if (mode == LAM_TRACE_ANY) {
+        if (alpha) trace_rays_kernel<true, true><<<grid, block, 0, st>>>(s->dev, rays, n, hits, words, flags);
+        else trace_rays_kernel<true, false><<<grid, block, 0, st>>>(s->dev, rays, n, hits, words, flags);
+    } else {
+        if (alpha) trace_rays_kernel<false, true><<<grid, block, 0, st>>>(s->dev, rays, n, hits, words, flags);
+        else trace_rays_kernel<false, false><<<grid, block, 0, st>>>(s->dev, rays, n, hits, words, flags);
+    }
+    return cudaGetLastError();
+}
+
+int run_trace(const lam_scene* s, cudaStream_t st, const char* who, TraceLaunch launch, const void* arg) {
+    uint64_t busy = s->trace_busy.load(std::memory_order_relaxed);
+    int slot = -1;
+    while (~busy) {
+        const int k = __builtin_ctzll(~busy);
+        if (s->trace_busy.compare_exchange_weak(busy, busy | (1ull << k), std::memory_order_acquire)) {
+            slot = k;
+            break;
+        }
+    }
+    static_assert(TRACE_SLOTS == 64, "one bit of trace_busy per slot");
+    if (slot < 0) {  // 64 queries in flight: scratch of this call's own
+        uint32_t* own = nullptr;
+        cudaError_t e = cudaMallocAsync((void**)&own, 3 * sizeof(uint32_t), st);
+        if (e != cudaSuccess) return cuda_error(e, who);
+        cudaMemsetAsync(own, 0, 3 * sizeof(uint32_t), st);
+        uint32_t flags = 0;
+        e = launch(own, own + 2, arg);
+        if (e == cudaSuccess) cudaMemcpyAsync(&flags, own + 2, sizeof(flags), cudaMemcpyDeviceToHost, st);
+        cudaFreeAsync(own, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        if (e != cudaSuccess) return cuda_error(e, who);
+        return flags & ERR_STACK_OVERFLOW ? set_error(LAM_ERR_STACK_OVERFLOW, "traversal stack overflow") : LAM_OK;
+    }
+    volatile uint32_t* flags = s->trace_flags + slot;
+    cudaError_t e = launch(s->trace_words + slot * TRACE_SLOT_WORDS, s->trace_flags_dev + slot, arg);
+    if (e == cudaSuccess) {
+        e = cudaStreamSynchronize(st);
+        // a wait that failed (a stream being captured) says nothing about the kernel: the slot stays taken
+        if (e != cudaSuccess) return cuda_error(e, who);
+    }
+    const uint32_t got = *flags;
+    *flags = 0u;
+    s->trace_busy.fetch_and(~(1ull << slot), std::memory_order_release);
+    if (e != cudaSuccess) return cuda_error(e, who);  // the launch failed: nothing ran
+    return got & ERR_STACK_OVERFLOW ? set_error(LAM_ERR_STACK_OVERFLOW, "traversal stack overflow") : LAM_OK;
 }
 
 int check_trace_call(const lam_scene* s, uint32_t n, const char* who) {
@@ -448,35 +520,17 @@ extern "C" int lam_trace_rays(const lam_scene* s, const lam_ray* rays, uint32_t 
         return set_error(LAM_ERR_INVALID_ARGUMENT, "lam_trace_rays: unknown mode");
     if (n == 0) return LAM_OK;
     if (int rc = check_trace_call(s, n, "lam_trace_rays")) return rc;
-    cudaStream_t st = (cudaStream_t)stream;
-    uint32_t* scratch = nullptr;  // [0] work counter, [1] error flags
-    cudaError_t e = cudaMallocAsync((void**)&scratch, 8, st);
-    if (e != cudaSuccess) return cuda_error(e, "lam_trace_rays scratch");
-    cudaMemsetAsync(scratch, 0, 8, st);
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
-    int per_sm = 8;
-    dim3 grid(sms * per_sm), block(TRACE_BLOCK);
-    const bool alpha = !s->dev.all_opaque;
-    if (mode == LAM_TRACE_ANY) {
-        if (alpha) trace_rays_kernel<true, true><<<grid, block, 0, st>>>(s->dev, rays, n, hits, scratch, scratch + 1);
-        else trace_rays_kernel<true, false><<<grid, block, 0, st>>>(s->dev, rays, n, hits, scratch, scratch + 1);
-    } else {
-        if (alpha) trace_rays_kernel<false, true><<<grid, block, 0, st>>>(s->dev, rays, n, hits, scratch, scratch + 1);
-        else trace_rays_kernel<false, false><<<grid, block, 0, st>>>(s->dev, rays, n, hits, scratch, scratch + 1);
-    }
-    e = cudaGetLastError();
-    if (e != cudaSuccess) {
-        cudaFreeAsync(scratch, st);
-        return cuda_error(e, "trace_rays_kernel launch");
-    }
-    uint32_t err_flags = 0;
-    cudaMemcpyAsync(&err_flags, scratch + 1, 4, cudaMemcpyDeviceToHost, st);
-    cudaFreeAsync(scratch, st);
-    e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return cuda_error(e, "lam_trace_rays");
-    if (err_flags & ERR_STACK_OVERFLOW) return set_error(LAM_ERR_STACK_OVERFLOW, "traversal stack overflow");
-    return LAM_OK;
+    struct Call {
+        const lam_scene* s;
+        const lam_ray* rays;
+        uint32_t n, mode;
+        lam_hit* hits;
+        cudaStream_t st;
+    } c{s, rays, n, mode, hits, (cudaStream_t)stream};
+    return run_trace(s, c.st, "lam_trace_rays", [](uint32_t* words, uint32_t* flags, const void* arg) {
+        const Call& a = *static_cast<const Call*>(arg);
+        return launch_trace(a.s, a.rays, a.n, a.mode, a.hits, words, flags, a.st);
+    }, &c);
 }
 
 // ---------------------------------------------------------------- allocation-free ray query
@@ -493,7 +547,7 @@ extern "C" int lam_trace_rays(const lam_scene* s, const lam_ray* rays, uint32_t 
 //     claim per warp of the grid and must not wrap;
 //   * every call uses the same array: calls that overlap on the GPU (different streams, or
 //     several host threads) race on the counter and give wrong results; serialise them;
-//   * the array keeps the last call's contents; each call clears the two words it uses first;
+//   * the array keeps the last call's contents; each call clears the three words it uses first;
 //   * the first call on a device resolves the array's device address with cudaGetSymbolAddress
 //     (once per device, in the CUDA runtime's primary context of that device) and keeps it for the
 //     life of the process; make that first call before any stream capture.  After cudaDeviceReset
@@ -501,7 +555,7 @@ extern "C" int lam_trace_rays(const lam_scene* s, const lam_ray* rays, uint32_t 
 //   * every call reads the error flags back and synchronises its stream before it returns.
 namespace lam {
 
-constexpr uint32_t STATIC_TRACE_WORDS = 64;  // 256 bytes; words 0 (work counter) and 1 (error flags) used
+constexpr uint32_t STATIC_TRACE_WORDS = 64;  // 256 bytes; words 0 (work counter), 1 (finished blocks) and 2 (error flags) used
 static __device__ __align__(256) uint32_t g_static_trace_scratch[STATIC_TRACE_WORDS];
 
 constexpr int STATIC_TRACE_MAX_DEVICES = 64;
@@ -543,23 +597,12 @@ extern "C" int lam_trace_rays_static(const lam_scene* s, const lam_ray* rays, ui
     int rc = static_trace_scratch(device, &scratch);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    e = cudaMemsetAsync(scratch, 0, 2 * sizeof(uint32_t), st);
+    e = cudaMemsetAsync(scratch, 0, 3 * sizeof(uint32_t), st);
     if (e != cudaSuccess) return cuda_error(e, "lam_trace_rays_static: clearing the scratch words");
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    dim3 grid(sms * 8), block(TRACE_BLOCK);
-    const bool alpha = !s->dev.all_opaque;
-    if (mode == LAM_TRACE_ANY) {
-        if (alpha) trace_rays_kernel<true, true><<<grid, block, 0, st>>>(s->dev, rays, n, hits, scratch, scratch + 1);
-        else trace_rays_kernel<true, false><<<grid, block, 0, st>>>(s->dev, rays, n, hits, scratch, scratch + 1);
-    } else {
-        if (alpha) trace_rays_kernel<false, true><<<grid, block, 0, st>>>(s->dev, rays, n, hits, scratch, scratch + 1);
-        else trace_rays_kernel<false, false><<<grid, block, 0, st>>>(s->dev, rays, n, hits, scratch, scratch + 1);
-    }
-    e = cudaGetLastError();
+    e = launch_trace(s, rays, n, mode, hits, scratch, scratch + 2, st);
     if (e != cudaSuccess) return cuda_error(e, "lam_trace_rays_static: launch");
     uint32_t err_flags = 0;
-    e = cudaMemcpyAsync(&err_flags, scratch + 1, sizeof(err_flags), cudaMemcpyDeviceToHost, st);
+    e = cudaMemcpyAsync(&err_flags, scratch + 2, sizeof(err_flags), cudaMemcpyDeviceToHost, st);
     if (e != cudaSuccess) return cuda_error(e, "lam_trace_rays_static: reading the error flags");
     e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_error(e, "lam_trace_rays_static");

@@ -694,6 +694,16 @@ LAM_DEV void trace_persistent_multi(uint32_t n, uint32_t* __restrict__ work, uin
     }
 }
 
+// End of a ray-query kernel: the last block to finish clears the work counter words[0] and the
+// finished-block count words[1] for the next query that uses them.
+LAM_DEV void trace_done(uint32_t* words) {
+    __syncthreads();
+    if (threadIdx.x == 0u) {
+        __threadfence();
+        if (atomicAdd(words + 1, 1u) + 1u == gridDim.x) words[0] = words[1] = 0u;
+    }
+}
+
 constexpr int TRACE_BLOCK = 128;
 constexpr uint32_t SMEM_INSTANCES = 128;
 

@@ -2756,28 +2756,19 @@ extern "C" int lam_pipeline_trace_rays(lam_pipeline* pl, const lam_scene* s, con
     if (int rc = check_trace_call(s, n, "lam_pipeline_trace_rays")) return rc;
     int rc = ensure_handler(pl);
     if (rc) return rc;
-    cudaStream_t st = (cudaStream_t)stream;
-    uint32_t* scratch = nullptr;  // [0] work counter, [1] error flags
-    cudaError_t e = cudaMallocAsync((void**)&scratch, 8, st);
-    if (e != cudaSuccess) return cuda_error(e, "lam_pipeline_trace_rays scratch");
-    cudaMemsetAsync(scratch, 0, 8, st);
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
-    DevScene S = s->dev;
-    uint32_t* counter = scratch;
-    uint32_t* err = scratch + 1;
-    void* kargs[] = {&S, &rays, &n, &hits, &counter, &err};
-    cudaKernel_t k = mode == LAM_TRACE_ANY ? pl->handler->trace_any : pl->handler->trace_closest;
-    e = cudaLaunchKernel((const void*)k, dim3(sms * 8), dim3(TRACE_BLOCK), kargs, 0, st);
-    if (e != cudaSuccess) {
-        cudaFreeAsync(scratch, st);
-        return cuda_error(e, "procedural trace launch");
-    }
-    uint32_t err_flags = 0;
-    cudaMemcpyAsync(&err_flags, err, 4, cudaMemcpyDeviceToHost, st);
-    cudaFreeAsync(scratch, st);
-    e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return cuda_error(e, "lam_pipeline_trace_rays");
-    if (err_flags & ERR_STACK_OVERFLOW) return set_error(LAM_ERR_STACK_OVERFLOW, "traversal stack overflow");
-    return LAM_OK;
+    struct Call {
+        DevScene S;
+        const lam_ray* rays;
+        uint32_t n;
+        lam_hit* hits;
+        cudaKernel_t kernel;
+        dim3 grid;
+        cudaStream_t st;
+    } c{s->dev, rays, n, hits, mode == LAM_TRACE_ANY ? pl->handler->trace_any : pl->handler->trace_closest,
+        dim3(s->sms * 8), (cudaStream_t)stream};
+    return run_trace(s, c.st, "lam_pipeline_trace_rays", [](uint32_t* words, uint32_t* flags, const void* arg) {
+        Call a = *static_cast<const Call*>(arg);
+        void* kargs[] = {&a.S, &a.rays, &a.n, &a.hits, &words, &flags};
+        return cudaLaunchKernel((const void*)a.kernel, a.grid, dim3(TRACE_BLOCK), kargs, 0, a.st);
+    }, &c);
 }
