@@ -82,7 +82,24 @@ LAM_DEV uint32_t f2u(float f) {
     return (uint32_t)f;
 }
 
+// Correctly rounded quotients by a constant, without the general division (about ten instructions and
+// a branch each, and a bounce has some twenty of them): q = x * (1 / c), then one correction by the
+// exact residual x - q * c (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. R&D 34, 1990).  Whether one correction rounds correctly depends on
+// c: checked against the IEEE quotient for every byte / 255 and every 24-bit mantissa / pi.
+LAM_DEV float byte_over_255(uint32_t b) {
+    const float x = (float)b, rc = 1.0f / 255.0f;
+    const float q = __fmul_rn(x, rc);
+    return __fmaf_rn(__fmaf_rn(-q, 255.0f, x), rc, q);
+}
+
 constexpr float PI_F = 3.14159265358979323846f;
+LAM_DEV float over_pi(float x) {
+    if (!(fabsf(x) > 1.0e-30f)) return x / PI_F;  // zeros, NaN, and residuals that could be subnormal
+    const float rc = 1.0f / PI_F;
+    const float q = __fmul_rn(x, rc);
+    return __fmaf_rn(__fmaf_rn(-q, PI_F, x), rc, q);
+}
 constexpr float HALF_PI_F = 3.14159265358979323846f / 2.0f;
 constexpr float TAU_F = 2.0f * 3.14159265358979323846f;
 constexpr uint32_t TY_DIFFUSE = 0u, TY_METALLIC = 1u, TY_TRANSPARENT = 2u, TY_SKY = 0xFFu;
@@ -145,17 +162,11 @@ LAM_DEV v3 u32_to_normalised(uint32_t u) {
     return normalize(v);
 }
 
-// IEEE binary16 -> f32 (exact), used by unpack2x16float
+// IEEE binary16 -> f32 (exact), used by unpack2x16float: one conversion instruction.
 LAM_DEV float f16_bits_to_f32(uint32_t h) {
-    uint32_t sign = (h & 0x8000u) << 16;
-    uint32_t exp = (h >> 10) & 0x1Fu;
-    uint32_t man = h & 0x3FFu;
-    if (exp == 0u) {
-        float v = (float)man * 5.9604644775390625e-08f;  // man * 2^-24, exact
-        return __uint_as_float(__float_as_uint(v) | sign);
-    }
-    if (exp == 0x1Fu) return __uint_as_float(sign | 0x7F800000u | (man << 13));
-    return __uint_as_float(sign | ((exp + 112u) << 23) | (man << 13));
+    float f;
+    asm("cvt.f32.f16 %0, %1;" : "=f"(f) : "h"((unsigned short)h));
+    return f;
 }
 LAM_DEV float2 unpack2x16float(uint32_t u) { return make_float2(f16_bits_to_f32(u & 0xFFFFu), f16_bits_to_f32(u >> 16)); }
 

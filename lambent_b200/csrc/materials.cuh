@@ -26,10 +26,8 @@ LAM_DEV lam_material load_material(const DevScene& S, uint32_t inst, uint32_t pr
 }
 
 LAM_DEV float4 unpack_texel(uint32_t t) {
-    const float s = 1.0f / 255.0f;
-    return make_float4((float)(t & 0xFFu) / 255.0f, (float)((t >> 8) & 0xFFu) / 255.0f,
-                       (float)((t >> 16) & 0xFFu) / 255.0f, (float)(t >> 24) / 255.0f);
-    (void)s;
+    return make_float4(byte_over_255(t & 0xFFu), byte_over_255((t >> 8) & 0xFFu), byte_over_255((t >> 16) & 0xFFu),
+                       byte_over_255(t >> 24));
 }
 
 // Nearest, clamp-to-edge sample of layer `layer` of a texture array [first, first + count).

@@ -122,6 +122,16 @@ LAM_DEV bool wbw_f32(const TravRay& r, float4 a, float4 b, float4 c, float limit
     return true;
 }
 
+// a / b rounded to nearest from b's rounded reciprocal: the quotient estimate is corrected twice by its
+// exact residual (P. Markstein, IBM J. R&D 34, 1990).  For a and b that came from f32, whose quotients
+// and residuals stay far inside the FP64 range; a zero keeps the sign that the first product gives.
+LAM_DEV double quotient_f64(double a, double b, double rcp_b) {
+    const double q0 = __dmul_rn(a, rcp_b);
+    const double q1 = __fma_rn(__fma_rn(-b, q0, a), rcp_b, q0);
+    const double q2 = __fma_rn(__fma_rn(-b, q1, a), rcp_b, q1);
+    return a == 0.0 ? q0 : q2;
+}
+
 // FP64 re-evaluation of the committed hit (same formulas as the oracle, never contracted).
 LAM_DEV void wbw_f64(float3 of, float3 df, float4 p0, float4 p1, float4 p2, float* t, float* u, float* v,
                      bool* front) {
@@ -152,7 +162,7 @@ LAM_DEV void wbw_f64(float3 of, float3 df, float4 p0, float4 p1, float4 p2, floa
     double dky = ky == 0 ? d[0] : (ky == 1 ? d[1] : d[2]);
     double dkz = kz == 0 ? d[0] : (kz == 1 ? d[1] : d[2]);
     auto pick = [&](const double* q, int k) { return k == 0 ? q[0] : (k == 1 ? q[1] : q[2]); };
-    double Sx = __ddiv_rn(dkx, dkz), Sy = __ddiv_rn(dky, dkz), Sz = __ddiv_rn(1.0, dkz);
+    const double Sz = __ddiv_rn(1.0, dkz), Sx = quotient_f64(dkx, dkz, Sz), Sy = quotient_f64(dky, dkz, Sz);
     double Ax = __dsub_rn(pick(a, kx), __dmul_rn(Sx, pick(a, kz))), Ay = __dsub_rn(pick(a, ky), __dmul_rn(Sy, pick(a, kz)));
     double Bx = __dsub_rn(pick(b, kx), __dmul_rn(Sx, pick(b, kz))), By = __dsub_rn(pick(b, ky), __dmul_rn(Sy, pick(b, kz)));
     double Cx = __dsub_rn(pick(c, kx), __dmul_rn(Sx, pick(c, kz))), Cy = __dsub_rn(pick(c, ky), __dmul_rn(Sy, pick(c, kz)));

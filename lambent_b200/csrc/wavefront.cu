@@ -375,9 +375,10 @@ __global__ void __launch_bounds__(WAVE_BLOCK) extend_kernel(Args A) {
 // ---------------------------------------------------------------- shade (one bounce of rt_sample)
 template <int Q, bool GUIDE>
 struct Shader {
-    LAM_DEV static v3 get_normal(v3 rd, v3 n, v3 t, uint32_t seed, float2 rough) {
+    // view: to_onb(rd, n, t)
+    LAM_DEV static v3 get_normal(v3 view, v3 n, v3 t, uint32_t seed, float2 rough) {
         if (Q == LAM_QUALITY_LOW) return n;
-        return from_onb(sample_vndf_ggx(seed, to_onb(rd, n, t), rough), n, t);
+        return from_onb(sample_vndf_ggx(seed, view, rough), n, t);
     }
     LAM_DEV static v3 make_diffuse(v3 hit_color, v3 rd, v3 n, v3 t, float rough, v3 new_dir) {
         if (Q == LAM_QUALITY_LOW) return splat(1.0f);
@@ -653,7 +654,8 @@ __global__ void __launch_bounds__(WAVE_BLOCK) shade_scatter_kernel(const __grid_
     }
 }
 
-template <int Q, bool GUIDE, bool LEARN, bool BATCH>
+// REC: out-radiance, primary and visible vertices are recorded (ReSTIR, Markov guiding).
+template <int Q, bool GUIDE, bool LEARN, bool BATCH, bool REC = GUIDE>
 // Six CTAs per SM for the unguided forms: the kernel waits on chains of dependent gathers (queue ->
 // hit -> triangle -> material -> texture), so resident warps matter more than the few registers
 // that spill (measured: 79 ms against 87 ms per 16-spp step at 1080p).  The Markov-guided forms keep
@@ -667,7 +669,6 @@ __global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(cons
     G.len = A.world_len;
     G.mod_m = A.world_mod_m;
     G.camera_loc = A.camera_pos;
-    const bool rec = A.ort != nullptr;
     // learned guiding without Markov chains: what the bounce decides for a deferred vertex (normal and
     // roughness, tangent and seed, albedo or the metal's reflection), held per thread until the append
     // at the end gives the vertex its slot in the guide kernel's queue, where it is then written
@@ -738,7 +739,7 @@ __global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(cons
             v3 orc = splat(1.0f), orad = splat(0.0f);
             float sum_mc = 0.0f;
             float4 pp = make_float4(0, 0, 0, 0), pn = make_float4(0, 0, 0, 0);
-            if (rec) {
+            if (REC) {
                 float4 t0 = A.ort[path], t1 = A.orad[path];
                 orc = mk(t0.x, t0.y, t0.z);
                 sum_mc = t0.w;
@@ -766,33 +767,40 @@ __global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(cons
                 make_isect(S, S.inst, h, make_float3(ro.x, ro.y, ro.z), make_float3(rd.x, rd.y, rd.z), is, A.phit_a,
                            A.phit_b, path);
                 new_pos = fma3(rd, splat(is.t), ro);
-                if (depth != 0u) {
-                    v3 est = GUIDE ? grid_radiance(G, new_pos, is.normal, rd) : splat(0.0f);
+                if (GUIDE && depth != 0u) {
+                    v3 est = grid_radiance(G, new_pos, is.normal, rd);
                     v3 rad_refl = strip_nan3(((is.color * est) * cached_brdf) / cached_pdf);
                     v3 rad_out = (is.emission * cached_brdf) / cached_pdf;
                     g_rad = rad_out + rad_refl;
                     g_out = rad_out;
                     g_nvmf = last_not_vmf;
+                } else if (depth != 0u && (is.emission.x != 0.0f || is.emission.y != 0.0f || is.emission.z != 0.0f)) {
+                    // without a grid the reflected estimate is zero, and a surface that emits nothing
+                    // has no weight whatever the sample's pdf (0 / pdf is 0 or NaN): six divisions
+                    // and a square root that only light sources need
+                    g_rad = (is.emission * cached_brdf) / cached_pdf;
                 }
             } else {
                 bg = sky_sample(S, rd);
                 new_pos = fma3(rd, splat(A.tmax), ro);
-                if (depth == 1u && rec) {
+                if (depth == 1u && REC) {
                     A.vpoint[path] = make_float4(new_pos.x, new_pos.y, new_pos.z, 0.0f);
                     A.vnormal[path] = make_float4(-rd.x, -rd.y, -rd.z, 0.0f);
                 }
                 if (depth == 0u && last_sample) {
                     if (out_normal) out_normal[pixel] = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
                     if (out_albedo) out_albedo[pixel] = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-                    if (A.pix_emission) {
+                    if (REC && A.pix_emission) {
                         A.pix_emission[pixel] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                         A.pix_albedo[pixel] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     }
                 }
                 if (depth != 0u) {
-                    orad = fma3(orc, bg, orad);
-                    g_rad = (bg * cached_brdf) / cached_pdf;
-                    g_out = g_rad;
+                    if (REC) orad = fma3(orc, bg, orad);
+                    if (GUIDE) {
+                        g_rad = (bg * cached_brdf) / cached_pdf;
+                        g_out = g_rad;
+                    }
                 }
             }
             // one call site for the chain updates of hit and sky lanes (general.wesl:677-684 and
@@ -817,35 +825,46 @@ __global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(cons
                 last_not_vmf = false;
                 ro = new_pos;
                 if (depth == 0u) {
-                    if (rec) {
+                    if (REC) {
                         pp = make_float4(ro.x, ro.y, ro.z, __uint_as_float(is.ty));
                         pn = make_float4(is.normal.x, is.normal.y, is.normal.z, pn.w);
                     }
                     if (last_sample) {
                         if (out_normal) out_normal[pixel] = make_float4(is.normal.x, is.normal.y, is.normal.z, 1.0f);
                         if (out_albedo) out_albedo[pixel] = make_float4(is.color.x, is.color.y, is.color.z, 1.0f);
-                        if (A.pix_emission) {
+                        if (REC && A.pix_emission) {
                             A.pix_emission[pixel] = make_float4(is.emission.x, is.emission.y, is.emission.z, 0.0f);
                             A.pix_albedo[pixel] = make_float4(is.color.x, is.color.y, is.color.z, 0.0f);
                         }
                     }
-                } else if (depth == 1u && rec) {
+                } else if (depth == 1u && REC) {
                     A.vpoint[path] = make_float4(ro.x, ro.y, ro.z, 0.0f);
                     A.vnormal[path] = make_float4(is.normal.x, is.normal.y, is.normal.z, 0.0f);
                 }
                 scol = fma3(color, is.emission, scol);
-                if (depth != 0u) orad = fma3(orc, is.emission, orad);
-                v3 assign_normal = Shader<Q, GUIDE>::get_normal(rd, is.normal, is.tangent, seed, is.roughness);
-                v3 normal = Shader<Q, GUIDE>::get_normal(rd, is.normal, is.tangent, seed, is.roughness_transparent);
+                if (REC && depth != 0u) orad = fma3(orc, is.emission, orad);
+                // The microfacet normals are drawn where something reads them: the surface's at metals and
+                // refractions, the coat's for the Fresnel choice.  A diffuse vertex without a Fresnel
+                // choice needs neither (250 instructions each of the 2,700 of a bounce).  The frame's view
+                // vector stays outside the branch, and the two draws inside one: the products that the
+                // compiler contracts, and with them the last bits, are then those of the plain sequence.
+                const uint32_t normal_seed = seed;
+                const v3 view = Q == LAM_QUALITY_LOW ? splat(0.0f) : to_onb(rd, is.normal, is.tangent);
                 bool should_reflect = false;
                 seed += 1u;
                 float4 cri = Shader<Q, GUIDE>::pick_ref_idx(&picked, is.ior_low, is.ior_high, seed);
                 float ri = cri.w;
                 seed += 1u;
                 if (!(!is.front_face && is.ty == TY_TRANSPARENT)) ri = 1.0f / ri;
+                v3 assign_normal = splat(0.0f), normal = splat(0.0f);
+                if (Q == LAM_QUALITY_LOW || ri != 1.0f || is.ty == TY_METALLIC || is.ty == TY_TRANSPARENT) {
+                    assign_normal = Shader<Q, GUIDE>::get_normal(view, is.normal, is.tangent, normal_seed, is.roughness);
+                    if (Q == LAM_QUALITY_LOW || ri != 1.0f)
+                        normal = Shader<Q, GUIDE>::get_normal(view, is.normal, is.tangent, normal_seed, is.roughness_transparent);
+                }
                 v3 cw = mk(cri.x, cri.y, cri.z);
                 color = color * cw;
-                orc = orc * cw;
+                if (REC) orc = orc * cw;
                 if (ri != 1.0f) {
                     float cos_theta = fminf(dot(-rd, normal), 1.0f);
                     float sin_theta = sqrtf(1.0f - (cos_theta * cos_theta));
@@ -856,7 +875,7 @@ __global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(cons
                 }
                 if (!should_reflect || is.ty == TY_TRANSPARENT) {
                     color = color * is.color;
-                    if (depth != 0u) orc = orc * is.color;
+                    if (REC && depth != 0u) orc = orc * is.color;
                 }
                 if (!should_reflect) {
                     normal = assign_normal;
@@ -922,7 +941,7 @@ __global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(cons
                         seed += 3u;
                     } else if (is.ty == TY_DIFFUSE) {
                         v3 dir_cos = cosine_hemisphere(seed, is.normal, is.tangent);
-                        float cos_pdf = fmaxf(dot(dir_cos, is.normal) / PI_F, 0.0f);
+                        float cos_pdf = fmaxf(over_pi(dot(dir_cos, is.normal)), 0.0f);
                         float theta = rand_f32(seed) * TAU_F;
                         seed += 1u;
                         float xi = rand_f32(seed);
@@ -968,7 +987,7 @@ __global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(cons
                         }
                         // general.wesl:840 weights by the cosine pdf of the cosine branch's draw even when
                         // dir is the vMF draw; LAM_GUIDE_PDF_AT_SAMPLE evaluates it at dir (unbiased)
-                        const float cos_term = GUIDE && A.pdf_at_sample ? fmaxf(dot(dir, is.normal) / PI_F, 0.0f) : cos_pdf;
+                        const float cos_term = GUIDE && A.pdf_at_sample ? fmaxf(over_pi(dot(dir, is.normal)), 0.0f) : cos_pdf;
                         float avg_pdf = (c0 * cos_term) + (c1 == 0.0f ? 0.0f : c1 * fmaxf(mix_pdf, 0.0f));
                         if (GUIDE && LEARN && depth + 1u < A.max_depth) {
                             // learned + Markov: the guide kernel mixes this draw with the network's.  It
@@ -977,7 +996,7 @@ __global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(cons
                             // kernel evaluates), with the cosine term at the drawn direction
                             deferred = true;
                             A.def_kind[path] = DEF_DIFFUSE;
-                            float pref = c0 * fmaxf(dot(dir, is.normal) / PI_F, 0.0f);
+                            float pref = c0 * fmaxf(over_pi(dot(dir, is.normal)), 0.0f);
                             float4* lobe = A.def_lobe + (size_t)path * MIX_LOBES;
                             float* lw = A.def_lw + (size_t)path * MIX_LOBES;
 #pragma unroll 1
@@ -998,10 +1017,10 @@ __global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(cons
                         } else {
                             v3 diffuse = Shader<Q, GUIDE>::make_diffuse(is.color, rd, is.normal, is.tangent, is.roughness.x, dir);
                             cached_pdf = avg_pdf;
-                            cached_brdf = fmaxf(dot(dir, is.normal) / PI_F, 0.0f);
+                            cached_brdf = fmaxf(over_pi(dot(dir, is.normal)), 0.0f);
                             float nf = fabsf(cached_brdf) / fmaxf(avg_pdf, 0.001f);
                             color = (color * nf) * diffuse;
-                            orc = (orc * nf) * diffuse;
+                            if (REC) orc = (orc * nf) * diffuse;
                             rd = dir;
                         }
                     } else if (is.ty == TY_TRANSPARENT) {
@@ -1068,7 +1087,7 @@ __global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(cons
             // live state at its slot in the guide kernel's queue, and a continuing one its state at its
             // slot in the next queue (both below)
             if (!cont) A.acc[path] = o_acc;
-            if (rec) {
+            if (REC) {
                 A.ort[path] = make_float4(orc.x, orc.y, orc.z, sum_mc);
                 A.orad[path] = make_float4(orad.x, orad.y, orad.z, 0.0f);
                 A.ppoint[path] = pp;
@@ -1138,7 +1157,7 @@ constexpr uint32_t GUIDE_TMEM_COLS = 128;  // accumulators of tiles A (columns 0
 // The Markov sampler's mixture pdf at w from the lobes the shade kernel kept for the path:
 // c0 cos/pi + sum_k w_k vMF_k(w), where w_k already includes the vMF branch's probability.
 LAM_DEV float markov_mixture_pdf(const Args& A, uint32_t path, float c0, v3 n, v3 w) {
-    float p = c0 * fmaxf(dot(w, n) / PI_F, 0.0f);
+    float p = c0 * fmaxf(over_pi(dot(w, n)), 0.0f);
     const float4* lobe = A.def_lobe + (size_t)path * MIX_LOBES;
     const float* lw = A.def_lw + (size_t)path * MIX_LOBES;
 #pragma unroll 1
@@ -1257,7 +1276,7 @@ LAM_DEV void guide_finish(const Args& A, uint32_t q, uint32_t path, const net::L
     } else {
         const v3 dir_cos = cosine_hemisphere(seed0, n, t);
         dir = dir_cos;
-        pdf = fmaxf(dot(dir_cos, n) / PI_F, 0.0f);
+        pdf = fmaxf(over_pi(dot(dir_cos, n)), 0.0f);
     }
     if (NET && !MARKOV) {
         const float f = A.guide_frac;
@@ -1272,10 +1291,10 @@ LAM_DEV void guide_finish(const Args& A, uint32_t q, uint32_t path, const net::L
             const float u2 = rand_f32(h);
             dir = net::mixture_sample(*L, u0, u1, u2);
         }
-        pdf = (1.0f - f) * fmaxf(dot(dir, n) / PI_F, 0.0f) + f * net::mixture_pdf(*L, dir);
+        pdf = (1.0f - f) * fmaxf(over_pi(dot(dir, n)), 0.0f) + f * net::mixture_pdf(*L, dir);
     }
     const v3 diffuse = Shader<Q, false>::make_diffuse(mk(dc.x, dc.y, dc.z), rd, n, t, dn.w, dir);
-    const float cached_brdf = fmaxf(dot(dir, n) / PI_F, 0.0f);
+    const float cached_brdf = fmaxf(over_pi(dot(dir, n)), 0.0f);
     const float nf = fabsf(cached_brdf) / fmaxf(pdf, 0.001f);
     const v3 color_pre = color;
     color = (color * nf) * diffuse;
@@ -1751,6 +1770,7 @@ static void launch_shade(bool guide, bool learned, dim3 g, dim3 b, cudaStream_t 
     if (guide && learned) shade_kernel<Q, true, true, false><<<g, b, GUIDE_SHADE_SMEM, st>>>(A);
     else if (guide) shade_kernel<Q, true, false, false><<<g, b, GUIDE_SHADE_SMEM, st>>>(A);
     else if (learned) shade_kernel<Q, false, true, false><<<g, b, 0, st>>>(A);
+    else if (A.ort) shade_kernel<Q, false, false, false, true><<<g, b, 0, st>>>(A);
     else shade_kernel<Q, false, false, false><<<g, b, 0, st>>>(A);
 }
 
