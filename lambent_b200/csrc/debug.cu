@@ -26,6 +26,8 @@ __global__ void __launch_bounds__(128) debug_kernel(DebugArgs A) {
     const uint4* tl;
     const DevInstance* in;
     stage_tlas(A.S, sm, tl, in);
+    __shared__ CoopScratch<false> scratch[4];  // one per warp of a 128-thread block
+    CoopScratch<false>& ws = scratch[threadIdx.x >> 5];
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= A.width * A.height) return;
     const uint32_t x = p % A.width, y = p / A.width;
@@ -46,8 +48,8 @@ __global__ void __launch_bounds__(128) debug_kernel(DebugArgs A) {
     uint2 stack[TRAVERSAL_STACK];
     uint32_t err = 0;
     T.transparent_passes = false;
-    T.init(A.S, o, d, A.tmin, A.tmax);
-    while (T.step(A.S, tl, in, stack, err)) {
+    T.init(A.S, ws, o, d, A.tmin, A.tmax);
+    while (T.step(A.S, tl, in, stack, ws, err)) {
     }
     float3 c = make_float3(0.0f, 0.0f, 0.0f);
     const TraceResult& r = T.res;
@@ -72,14 +74,15 @@ __global__ void __launch_bounds__(128) debug_kernel(DebugArgs A) {
         const float4* tp = A.S.tris + 3u * r.tri;
         float t, bu, bv;
         bool front;
-        wbw_f64(oo, od, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), &t, &bu, &bv, &front);
+        const float4 va = __ldg(tp);
+        wbw_f64(oo, od, va, __ldg(tp + 1), __ldg(tp + 2), &t, &bu, &bv, &front);
         if (A.mode == LAM_DEBUG_FRONT_FACE) {
             float g = 1.0f / (t + 1.0f);
             c = front ? make_float3(0.0f, g, 0.0f) : make_float3(g, 0.0f, 0.0f);
         } else {
             // reflectance.wesl:88 indexes the material tables by geometry_index (always 0 here), not
             // by the instance index
-            lam_material mt = load_material(A.S, 0u, r.prim);
+            lam_material mt = load_material(A.S, 0u, __float_as_uint(va.w));
             float2 ior = unpack2x16float(mt.refractive_index);
             c = make_float3(ior.x / 5.0f, ior.y / 5.0f, 0.0f);
         }

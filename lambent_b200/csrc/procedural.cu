@@ -69,7 +69,7 @@ LAM_DEV void proc_trace(const DevScene& S, const lam_ray* __restrict__ rays, uin
             h.kind = LAM_HIT_NONE;
         } else if (in[tr.inst].flags & INST_PROCEDURAL) {
             h.t = tr.t; h.u = 0.0f; h.v = 0.0f;
-            h.primitive_index = tr.prim;
+            h.primitive_index = __float_as_uint(__ldg(S.tris + 3u * tr.tri).w);
             h.instance_index = tr.inst;
             h.kind = LAM_HIT_BACK;
         } else {
@@ -82,8 +82,9 @@ LAM_DEV void proc_trace(const DevScene& S, const lam_ray* __restrict__ rays, uin
             object_ray(m, o, d, &oo, &od);
             const float4* tp = S.tris + 3u * tr.tri;
             bool front;
-            wbw_f64(oo, od, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), &h.t, &h.u, &h.v, &front);
-            h.primitive_index = tr.prim;
+            const float4 a = __ldg(tp);
+            wbw_f64(oo, od, a, __ldg(tp + 1), __ldg(tp + 2), &h.t, &h.u, &h.v, &front);
+            h.primitive_index = __float_as_uint(a.w);
             h.instance_index = tr.inst;
             h.kind = front ? LAM_HIT_FRONT : LAM_HIT_BACK;
         }

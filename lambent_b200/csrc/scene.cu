@@ -402,8 +402,9 @@ extern "C" int lam_scene_destroy(lam_scene* s) {
 namespace lam {
 
 template <bool ANY, bool ALPHA>
-__global__ void __launch_bounds__(TRACE_BLOCK) trace_rays_kernel(DevScene S, const lam_ray* __restrict__ rays,
-                                                                 uint32_t n, lam_hit* __restrict__ hits,
+__global__ void __launch_bounds__(TRACE_BLOCK) trace_rays_kernel(const __grid_constant__ DevScene S,
+                                                                 const lam_ray* __restrict__ rays, uint32_t n,
+                                                                 lam_hit* __restrict__ hits,
                                                                  uint32_t* __restrict__ counter,
                                                                  uint32_t* __restrict__ err_out) {
     __shared__ TraceSmem sm;
@@ -420,32 +421,45 @@ __global__ void __launch_bounds__(TRACE_BLOCK) trace_rays_kernel(DevScene S, con
         t1 = r1.w;
     };
     auto store = [&](uint32_t i, const TraceResult& tr) {
-        const float4 r0 = __ldg(reinterpret_cast<const float4*>(rays + i));
-        const float4 r1 = __ldg(reinterpret_cast<const float4*>(rays + i) + 1);
-        const float3 o = make_float3(r0.x, r0.y, r0.z), d = make_float3(r1.x, r1.y, r1.z);
-        lam_hit h;
-        if (tr.tri == NO_HIT) {
-            h.t = 0.0f; h.u = 0.0f; h.v = 0.0f;
-            h.primitive_index = NO_HIT;
-            h.instance_index = NO_HIT;
-            h.kind = LAM_HIT_NONE;
-        } else {
-            float m[12];
-            for (int q = 0; q < 12; ++q) m[q] = in[tr.inst].inv[q];
-            float3 oo, od;
-            object_ray(m, o, d, &oo, &od);
-            const float4* tp = S.tris + 3u * tr.tri;
-            bool front;
-            wbw_f64(oo, od, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), &h.t, &h.u, &h.v, &front);
-            h.primitive_index = tr.prim;
-            h.instance_index = tr.inst;
-            h.kind = front ? LAM_HIT_FRONT : LAM_HIT_BACK;
-        }
-        hits[i] = h;
+        hits[i].primitive_index = tr.tri;
+        hits[i].instance_index = tr.inst;
     };
     trace_persistent<ANY, ALPHA>(S, tl, in, n, counter, err, load, store);
     if (err) *err_out = err;  // possibly mapped host memory; one flag only, so a plain store
     trace_done(counter);
+}
+
+// The public hit records, from the triangle slots and instances that the traversal left in them: the
+// FP64 re-evaluation of each hit's triangle.  Inside the traversal loop it ran for the one or two lanes
+// whose rays had finished, and its registers (96) cost two CTAs per SM: 4.2M rays 2,490 -> 1,890 us.
+__global__ void __launch_bounds__(TRACE_BLOCK) finish_hits_kernel(const __grid_constant__ DevScene S,
+                                                                  const lam_ray* __restrict__ rays, uint32_t n,
+                                                                  lam_hit* hits) {
+    const uint32_t i = blockIdx.x * TRACE_BLOCK + threadIdx.x;
+    if (i >= n) return;
+    const uint32_t tri = hits[i].primitive_index, inst = hits[i].instance_index;
+    lam_hit h;
+    if (tri == NO_HIT) {
+        h.t = 0.0f; h.u = 0.0f; h.v = 0.0f;
+        h.primitive_index = NO_HIT;
+        h.instance_index = NO_HIT;
+        h.kind = LAM_HIT_NONE;
+    } else {
+        const float4 r0 = __ldg(reinterpret_cast<const float4*>(rays + i));
+        const float4 r1 = __ldg(reinterpret_cast<const float4*>(rays + i) + 1);
+        float m[12];
+        for (int q = 0; q < 12; ++q) m[q] = S.inst[inst].inv[q];
+        float3 oo, od;
+        object_ray(m, make_float3(r0.x, r0.y, r0.z), make_float3(r1.x, r1.y, r1.z), &oo, &od);
+        const float4* tp = S.tris + 3u * tri;
+        const float4 a = __ldg(tp);
+        bool front;
+        wbw_f64(oo, od, a, __ldg(tp + 1), __ldg(tp + 2), &h.t, &h.u, &h.v, &front);
+        h.primitive_index = __float_as_uint(a.w);
+        h.instance_index = inst;
+        h.kind = front ? LAM_HIT_FRONT : LAM_HIT_BACK;
+    }
+    hits[i] = h;
 }
 
 static cudaError_t launch_trace(const lam_scene* s, const lam_ray* rays, uint32_t n, uint32_t mode, lam_hit* hits,
@@ -459,6 +473,7 @@ static cudaError_t launch_trace(const lam_scene* s, const lam_ray* rays, uint32_
         if (alpha) trace_rays_kernel<false, true><<<grid, block, 0, st>>>(s->dev, rays, n, hits, words, flags);
         else trace_rays_kernel<false, false><<<grid, block, 0, st>>>(s->dev, rays, n, hits, words, flags);
     }
+    finish_hits_kernel<<<(n + TRACE_BLOCK - 1) / TRACE_BLOCK, block, 0, st>>>(s->dev, rays, n, hits);
     return cudaGetLastError();
 }
 

@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(WAVE_BLOCK) generate_kernel(Args A) {
 
 // ---------------------------------------------------------------- extend
 template <bool ALPHA>
-__global__ void __launch_bounds__(WAVE_BLOCK) extend_kernel(Args A) {
+__global__ void __launch_bounds__(WAVE_BLOCK) extend_kernel(const __grid_constant__ Args A) {
     __shared__ TraceSmem sm;
     const uint4* tl;
     const DevInstance* in;
@@ -1860,8 +1860,8 @@ __global__ void __launch_bounds__(WAVE_BLOCK) extend_batch_kernel(const __grid_c
         atomicAdd(A.segments + 1, (unsigned long long)n);
     }
     uint32_t err = 0u;
-    trace_persistent_multi<false, ALPHA>(
-        n, A.work, err,
+    trace_persistent<false, ALPHA, true>(
+        A.S, nullptr, nullptr, n, A.work, err,
         [&](uint32_t i, float3& o, float3& d, float& t0, float& t1, const DevScene*& sp) {
             const float4 o4 = A.ray_o[i], d4 = A.ray_d[i];
             o = make_float3(o4.x, o4.y, o4.z);
