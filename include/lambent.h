@@ -488,12 +488,12 @@ int lam_render_profile_get(lam_pipeline* pipeline, lam_stage_times* out);
 int lam_pipeline_set_wave_paths(lam_pipeline* pipeline, uint64_t max_paths);
 /* Shading order (no counterpart in the reference, whose rt_main shades one pixel's path per
  * thread).  LAM_SHADE_ORDER_QUEUE shades the queued hits in the order extend found them;
- * LAM_SHADE_ORDER_MATERIAL first sorts them (stable) by what the bounce runs: sky, diffuse,
- * metallic, transparent, so that a warp's lanes take the same branch.  LAM_SHADE_ORDER_AUTO, the
- * default, sorts every render except Markov-guided ones, which run slower in class order.  A plain
- * render's image does not depend on the order;
+ * LAM_SHADE_ORDER_MATERIAL first groups them by what the bounce runs: sky, diffuse, metallic,
+ * transparent, so that a warp's lanes take the same branch.  LAM_SHADE_ORDER_AUTO, the default, does
+ * so in waves of at least 2^18 paths, except in Markov-guided renders, which run slower in class
+ * order.  A plain render's image does not depend on the order;
  * under guiding, the world-grid and training updates land in another order, as they already may
- * between two runs.  The sort keeps 5 bytes per path of device state.  Takes effect at the next
+ * between two runs.  The order keeps 8 bytes per path of device state.  Takes effect at the next
  * lam_render or lam_batch_render. */
 #define LAM_SHADE_ORDER_AUTO 0u
 #define LAM_SHADE_ORDER_QUEUE 1u

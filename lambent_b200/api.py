@@ -435,9 +435,10 @@ class Pipeline:
         check(lib().lam_pipeline_set_wave_paths(self._h, int(max_paths)))
 
     def set_shade_order(self, order=_abi.SHADE_ORDER_AUTO):
-        """SHADE_ORDER_MATERIAL sorts each bounce's hits by class (sky, diffuse, metallic,
+        """SHADE_ORDER_MATERIAL groups each bounce's hits by class (sky, diffuse, metallic,
         transparent) before shading; SHADE_ORDER_QUEUE shades them in traversal order;
-        SHADE_ORDER_AUTO (the default) sorts except under Markov guiding."""
+        SHADE_ORDER_AUTO (the default) groups them in waves of at least 2^18 paths, except under
+        Markov guiding."""
         check(lib().lam_pipeline_set_shade_order(self._h, int(order)))
 
     def profile(self):

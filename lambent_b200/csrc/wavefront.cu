@@ -243,10 +243,8 @@ struct WaveBuffers {
     float* def_lw = nullptr;
     uint32_t* def_kind = nullptr;                  // DEF_DIFFUSE / DEF_METAL
     float4 *phit_a = nullptr, *phit_b = nullptr;  // procedural hits (allocated on first use)
-    uint8_t* shade_key = nullptr;                  // material-ordered shading (allocated on first use)
-    uint32_t *shade_order = nullptr, *shade_bc = nullptr;
-    uint32_t* ctr = nullptr;  // [0..1] queue counts, [2..3] work counters, [4] error flags,
-                              // [8..11] segment counters, [12] diffuse-queue count, [13] records
+    uint32_t *order_a = nullptr, *order_b = nullptr;  // material-ordered shading (allocated on first use)
+    uint32_t* ctr = nullptr;                       // CTR_WORDS counters
     std::vector<void*> allocs;
     int sms = 148, grid_extend = 0, grid_shade = 0, grid_guide = 0, grid_sort = 0;
 };
@@ -294,9 +292,19 @@ LAM_DEV uint32_t advance_fill_seed(uint32_t s) {
 }
 
 // ---------------------------------------------------------------- generate
+// Clears a wave's counters and queues its `paths` at depth 0 (by block 0 of a generate kernel).
+LAM_DEV void start_wave(const Args& A, uint32_t paths) {
+    for (uint32_t k = CTR_WAVE + threadIdx.x; k < CTR_WORDS; k += blockDim.x) A.ctr[k] = k == CTR_COUNT ? paths : 0u;
+}
+
 __global__ void __launch_bounds__(WAVE_BLOCK) generate_kernel(Args A) {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p == 0) *A.count_in = A.npix * A.wave_count;
+    if (blockIdx.x == 0u) {
+        start_wave(A, A.npix * A.wave_count);
+        // a render's error flags and segment count; its training records are counted per wave
+        if (A.wave_first == 0u && threadIdx.x < CTR_TOTAL) A.ctr[threadIdx.x] = 0u;
+        if (threadIdx.x == 0u) A.ctr[CTR_RECORDS] = 0u;
+    }
     if (p >= A.npix) return;
     const uint32_t x = p % A.width, y = p / A.width;
     uint32_t st;
@@ -484,43 +492,34 @@ LAM_DEV void finalize_records(const Args& A, uint32_t path, v3 scol) {
 }
 
 // ---------------------------------------------------------------- material-ordered shading
-// A stable counting sort of the queue by shading class (sky, diffuse, metallic, transparent), so that
-// the shade kernel runs one class at a time across the whole GPU: its warps take one branch, and
-// every SM's caches hold one class's code, materials and textures.  (A sort within blocks, whose
-// warps are as uniform, gave no gain: the grid-wide order is what pays.)  The three kernels split
-// the queue into one contiguous chunk per block: count the classes of the chunk, scan the counts
-// (class major, then block), and write each position to its slot in the order.  Within a class the
-// queue order is kept, so the shade kernel's reads stay nearly sequential.  A procedural hit's
-// leaf record holds its primitive in the same word as a triangle's.
-
-// The chunk of queue positions [*beg, *end) of block b of nb (a multiple of the block size).
-LAM_DEV void sort_chunk(uint32_t n, uint32_t b, uint32_t nb, uint32_t* beg, uint32_t* end) {
-    const uint32_t per = (n + nb - 1u) / nb;
-    const uint32_t c = (per + WAVE_BLOCK - 1u) / WAVE_BLOCK * WAVE_BLOCK;
-    *beg = min(n, b * c);
-    *end = min(n, *beg + c);
-}
-
+// The queue positions by shading class (sky, diffuse, metallic, transparent), so that the shade kernel
+// runs one class at a time across the whole GPU: its warps take one branch, and every SM's caches hold
+// one class's code, materials and textures.  (An order within blocks, whose warps are as uniform, gave
+// no gain: the grid-wide order is what pays.)  One pass: a block finds the classes of a tile of
+// positions, reserves room in the classes' lists and writes the positions there.  A tile's positions
+// stay together and in order, so the shade kernel's reads stay nearly sequential.  (Counting, scanning
+// and scattering in three kernels kept the whole queue in order, which no result depends on: 1,560 us of
+// a 16-spp frame of the icosphere field at 1080p, and 7% of a 16-spp frame of the Cornell box at 256x256.)
+// A procedural hit's leaf record holds its primitive in the same word as a triangle's.
 // BATCH: each path's scene is its request's (lam_batch_render).
 template <bool BATCH>
-__global__ void __launch_bounds__(WAVE_BLOCK) shade_keys_kernel(const __grid_constant__ Args A) {
-    __shared__ uint32_t cnt[SHADE_CLASSES];
-    if (threadIdx.x < SHADE_CLASSES) cnt[threadIdx.x] = 0u;
-    __syncthreads();
-    uint32_t beg, end;
-    sort_chunk(*A.count_in, blockIdx.x, gridDim.x, &beg, &end);
-    const uint32_t lane = threadIdx.x & 31u;
-    // U tiles per step, each stage's loads issued for all of them before the next stage's: a class
+__global__ void __launch_bounds__(WAVE_BLOCK) shade_order_kernel(const __grid_constant__ Args A) {
+    // U positions per thread, each stage's loads issued for all of them before the next stage's: a class
     // is a chain of four dependent loads (hit; triangle word and instance; material index; material)
-    constexpr uint32_t U = 4;
-    for (uint32_t t = beg; t < end; t += U * WAVE_BLOCK) {
+    constexpr uint32_t NW = WAVE_BLOCK / 32, U = 4;
+    __shared__ uint32_t wcnt[U * NW][SHADE_CLASSES];  // positions of each class per row of 32
+    __shared__ uint32_t first[SHADE_CLASSES];         // the tile's first entry in each class's list
+    const uint32_t n = *A.count_in;
+    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    const uint32_t below = (1u << lane) - 1u;
+    for (uint32_t t = blockIdx.x * U * WAVE_BLOCK; t < n; t += gridDim.x * U * WAVE_BLOCK) {
         bool v[U];
         uint2 h[U];
         const DevScene* S[U];
 #pragma unroll
         for (uint32_t q = 0; q < U; ++q) {
             const uint32_t j = t + q * WAVE_BLOCK + threadIdx.x;
-            v[q] = j < end;
+            v[q] = j < n;
             S[q] = &A.S;
             // plain loads: the shade kernel reads the hit (and a batched path's flags) again next
             if (BATCH && v[q]) S[q] = &A.reqs[A.segs[A.qmisc[j].z >> 16].req].S;
@@ -539,116 +538,48 @@ __global__ void __launch_bounds__(WAVE_BLOCK) shade_keys_kernel(const __grid_con
         for (uint32_t q = 0; q < U; ++q)
             mi[q] = clamp_idx(mcount[q] ? __ldg(S[q]->mat_idx + moff[q] + clamp_idx(prim[q], mcount[q])) : 0u,
                               S[q]->material_count);
-        uint32_t k[U];
+        uint32_t k[U], rank[U];
 #pragma unroll
         for (uint32_t q = 0; q < U; ++q) {
-            const uint32_t j = t + q * WAVE_BLOCK + threadIdx.x;
             k[q] = SHADE_CLASSES;
             if (v[q]) {
-                if (h[q].x == NO_HIT) {
-                    k[q] = SHADE_SKY;
-                } else {
+                k[q] = SHADE_SKY;
+                if (h[q].x != NO_HIT) {
                     // tex_idx_attributes_ty: the type in its upper half (as load_material reads it)
                     const uint32_t ty = __ldg(reinterpret_cast<const uint32_t*>(S[q]->materials + mi[q]) + 5) >> 16;
                     k[q] = ty == TY_METALLIC ? SHADE_METALLIC : (ty == TY_TRANSPARENT ? SHADE_TRANSPARENT : SHADE_DIFFUSE);
                 }
-                A.shade_key[j] = (uint8_t)k[q];
             }
         }
-#pragma unroll
-        for (uint32_t q = 0; q < U; ++q)
-#pragma unroll
-            for (uint32_t c = 0; c < SHADE_CLASSES; ++c) {
-                const uint32_t m = __ballot_sync(0xFFFFFFFFu, k[q] == c);
-                if (lane == 0u && m) atomicAdd(&cnt[c], (uint32_t)__popc(m));
-            }
-    }
-    __syncthreads();
-    if (threadIdx.x < SHADE_CLASSES) A.shade_bc[blockIdx.x * SHADE_CLASSES + threadIdx.x] = cnt[threadIdx.x];
-}
-
-// One block of SORT_BLOCKS_MAX threads: thread b turns block b's counts into its first slot per
-// class (exclusive, class-major: all of class 0, then class 1, ...).
-__global__ void __launch_bounds__(SORT_BLOCKS_MAX) shade_scan_kernel(const __grid_constant__ Args A, uint32_t nb) {
-    __shared__ uint32_t warp_sum[SORT_BLOCKS_MAX / 32];
-    __shared__ uint32_t class_base;
-    const uint32_t b = threadIdx.x, lane = b & 31u, wid = b >> 5;
-    if (b == 0u) class_base = 0u;
-    for (uint32_t c = 0; c < SHADE_CLASSES; ++c) {
-        const uint32_t v = b < nb ? A.shade_bc[b * SHADE_CLASSES + c] : 0u;
-        uint32_t x = v;  // inclusive scan within the warp
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-            if (lane >= (uint32_t)o) x += y;
-        }
-        if (lane == 31u) warp_sum[wid] = x;
-        __syncthreads();
-        if (wid == 0u) {
-            uint32_t s = warp_sum[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, s, o);
-                if (lane >= (uint32_t)o) s += y;
-            }
-            warp_sum[lane] = s;  // inclusive over warps
-        }
-        __syncthreads();
-        const uint32_t before = (wid ? warp_sum[wid - 1u] : 0u) + x - v;
-        if (b < nb) A.shade_bc[b * SHADE_CLASSES + c] = class_base + before;
-        __syncthreads();
-        if (b == 0u) class_base += warp_sum[SORT_BLOCKS_MAX / 32 - 1];
-        __syncthreads();
-    }
-}
-
-__global__ void __launch_bounds__(WAVE_BLOCK) shade_scatter_kernel(const __grid_constant__ Args A) {
-    // U tiles per step: their ranks come from one pass of ballots, so that a step takes three
-    // barriers instead of three per tile
-    constexpr uint32_t NW = WAVE_BLOCK / 32, U = 4;
-    __shared__ uint32_t wcnt[U][NW][SHADE_CLASSES];
-    __shared__ uint32_t next[SHADE_CLASSES];
-    if (threadIdx.x < SHADE_CLASSES) next[threadIdx.x] = A.shade_bc[blockIdx.x * SHADE_CLASSES + threadIdx.x];
-    __syncthreads();
-    uint32_t beg, end;
-    sort_chunk(*A.count_in, blockIdx.x, gridDim.x, &beg, &end);
-    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
-    const uint32_t below = (1u << lane) - 1u;
-    for (uint32_t t = beg; t < end; t += U * WAVE_BLOCK) {
-        uint32_t k[U], rank[U];
 #pragma unroll
         for (uint32_t q = 0; q < U; ++q) {
-            const uint32_t j = t + q * WAVE_BLOCK + threadIdx.x;
-            k[q] = j < end ? (uint32_t)A.shade_key[j] : SHADE_CLASSES;
             rank[q] = 0u;
 #pragma unroll
             for (uint32_t c = 0; c < SHADE_CLASSES; ++c) {
                 const uint32_t m = __ballot_sync(0xFFFFFFFFu, k[q] == c);
                 if (k[q] == c) rank[q] = (uint32_t)__popc(m & below);
-                if (lane == 0u) wcnt[q][wid][c] = (uint32_t)__popc(m);
+                if (lane == 0u) wcnt[q * NW + wid][c] = (uint32_t)__popc(m);
             }
         }
         __syncthreads();
-        // a position's slot: its class's next slot, then the earlier tiles' and earlier warps' lanes
-        // of its class, then its rank within its warp (stable: tiles, warps and lanes in order)
+        if (threadIdx.x < SHADE_CLASSES) {  // exclusive sums over the rows; room for the tile
+            uint32_t sum = 0u;
+#pragma unroll
+            for (uint32_t r = 0; r < U * NW; ++r) {
+                const uint32_t x = wcnt[r][threadIdx.x];
+                wcnt[r][threadIdx.x] = sum;
+                sum += x;
+            }
+            first[threadIdx.x] = sum ? atomicAdd(A.class_count + threadIdx.x, sum) : 0u;
+        }
+        __syncthreads();
 #pragma unroll
         for (uint32_t q = 0; q < U; ++q) {
             if (k[q] < SHADE_CLASSES) {
-                uint32_t slot = next[k[q]] + rank[q];
-                for (uint32_t p = 0; p < q; ++p)
-                    for (uint32_t w = 0; w < NW; ++w) slot += wcnt[p][w][k[q]];
-                for (uint32_t w = 0; w < wid; ++w) slot += wcnt[q][w][k[q]];
-                A.shade_order[slot] = t + q * WAVE_BLOCK + threadIdx.x;
+                const uint32_t slot = first[k[q]] + wcnt[q * NW + wid][k[q]] + rank[q];
+                uint32_t* list = k[q] < SHADE_METALLIC ? A.order_a : A.order_b;
+                list[(k[q] & 1u) ? n - 1u - slot : slot] = t + q * WAVE_BLOCK + threadIdx.x;
             }
-        }
-        __syncthreads();
-        if (threadIdx.x < SHADE_CLASSES) {
-            uint32_t add = 0u;
-#pragma unroll
-            for (uint32_t q = 0; q < U; ++q)
-#pragma unroll
-                for (uint32_t w = 0; w < NW; ++w) add += wcnt[q][w][threadIdx.x];
-            next[threadIdx.x] += add;
         }
         __syncthreads();
     }
@@ -674,16 +605,27 @@ __global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(cons
     // at the end gives the vertex its slot in the guide kernel's queue, where it is then written
     constexpr bool STASH = LEARN && !GUIDE;
     __shared__ float4 def_stash[STASH ? 3 : 1][STASH ? WAVE_BLOCK : 1];
+    // the classes' ends in work-item order
+    uint32_t end0 = 0u, end1 = 0u, end2 = 0u;
+    if (A.order_a) {
+        end0 = A.class_count[SHADE_SKY];
+        end1 = end0 + A.class_count[SHADE_DIFFUSE];
+        end2 = end1 + A.class_count[SHADE_METALLIC];
+    }
+    auto entry = [&](uint32_t j) -> const uint32_t* {
+        return j < end1 ? A.order_a + (j < end0 ? j : n - 1u - (j - end0))
+                        : A.order_b + (j < end2 ? j - end1 : n - 1u - (j - end2));
+    };
     for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u;; base += gridDim.x * blockDim.x) {
         if (base >= n) break;
         const uint32_t j = base + lane;  // work item; i: the queue position it shades
-        const uint32_t i = (A.shade_order && j < n) ? A.shade_order[j] : j;
+        const uint32_t i = (A.order_a && j < n) ? *entry(j) : j;
         {
             // the next iteration's queue-ordered inputs have known addresses: start them towards L2
             const uint32_t jnext = j + gridDim.x * blockDim.x;
             if (jnext < n) {
-                if (A.shade_order) {
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(A.shade_order + jnext));
+                if (A.order_a) {
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(entry(jnext)));
                 } else {
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(A.q_in + jnext));
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(A.hit + jnext));
@@ -1596,7 +1538,7 @@ static int alloc_wave(WaveBuffers* w, uint32_t npix, bool full, bool guide, bool
     rc |= walloc(w, &w->seed, P);
     rc |= walloc(w, &w->flags, P);
     rc |= walloc(w, &w->pix_color, npix);
-    rc |= walloc(w, &w->ctr, 64);
+    rc |= walloc(w, &w->ctr, CTR_WORDS);
     if (full) {
         rc |= walloc(w, &w->ort, P);
         rc |= walloc(w, &w->orad, P);
@@ -1680,7 +1622,7 @@ static int ensure_wave(lam_pipeline* pl, uint32_t width, uint32_t height, bool f
         capped = true;
     }
     w->mem_capped = capped;
-    cudaMemset(w->ctr, 0, 64 * sizeof(uint32_t));
+    cudaMemset(w->ctr, 0, CTR_WORDS * sizeof(uint32_t));
     pl->total_segments = 0;
     pl->prof_segments_base = 0;
     cudaDeviceGetAttribute(&w->sms, cudaDevAttrMultiProcessorCount, pl->device);
@@ -1690,7 +1632,7 @@ static int ensure_wave(lam_pipeline* pl, uint32_t width, uint32_t height, bool f
     occ = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, shade_kernel<LAM_QUALITY_MEDIUM, false, false, false>, WAVE_BLOCK, 0);
     w->grid_shade = w->sms * std::max(1, occ);
-    w->grid_sort = std::min(SORT_BLOCKS_MAX, w->sms * 6);
+    w->grid_sort = w->sms * 6;
     if (guide) {
         const void* ks[] = {(const void*)shade_kernel<LAM_QUALITY_LOW, true, false, false>,
                             (const void*)shade_kernel<LAM_QUALITY_MEDIUM, true, false, false>,
@@ -1740,6 +1682,22 @@ static int ensure_wave(lam_pipeline* pl, uint32_t width, uint32_t height, bool f
     }
     pl->wave = w;
     return LAM_OK;
+}
+
+static int ensure_order(WaveBuffers* w, size_t paths) {
+    if (w->order_a && w->order_b) return LAM_OK;
+    if ((!w->order_a && walloc(w, &w->order_a, paths)) || (!w->order_b && walloc(w, &w->order_b, paths)))
+        return LAM_ERR_CUDA;
+    return LAM_OK;
+}
+
+// The counters of one bounce.
+static void set_depth(Args& A, const WaveBuffers* w, uint32_t depth) {
+    A.count_in = w->ctr + CTR_COUNT + depth;
+    A.count_out = A.count_in + 1;
+    A.work = w->ctr + CTR_WORK + depth;
+    A.dq_count = w->ctr + CTR_DEFERRED + depth;
+    A.class_count = w->ctr + CTR_CLASS + 4u * depth;
 }
 
 int ensure_handler(lam_pipeline* pl) {
@@ -1811,8 +1769,10 @@ LAM_DEV void create_ray_req(const BatchReq& R, uint32_t x, uint32_t y, v3* o, v3
     *o = R.camera_pos;
 }
 
-// Zeroes the per-request completion counters and stamps the batch start.
-__global__ void batch_start_kernel(uint32_t* done, unsigned long long* times, uint32_t n) {
+// Zeroes the batch's error flags, its segment count and the per-request completion counters, and
+// stamps the batch start.
+__global__ void batch_start_kernel(uint32_t* ctr, uint32_t* done, unsigned long long* times, uint32_t n) {
+    if (threadIdx.x < CTR_TOTAL) ctr[threadIdx.x] = 0u;
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) done[i] = 0u;
     __syncthreads();
     if (threadIdx.x == 0) times[n] = global_timer_ns();
@@ -1822,7 +1782,7 @@ __global__ void batch_start_kernel(uint32_t* done, unsigned long long* times, ui
 // segment's samples (as generate_kernel does for a single render).
 __global__ void __launch_bounds__(WAVE_BLOCK) batch_generate_kernel(const __grid_constant__ Args A) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t == 0) *A.count_in = A.npix;  // paths of this wave
+    if (blockIdx.x == 0u) start_wave(A, A.npix);  // npix: paths of this wave
     if (t >= A.pix_threads) return;
     const uint32_t k = find_seg(A.segs, A.nsegs, t);
     const BatchSeg sg = A.segs[k];
@@ -2073,8 +2033,9 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
     A.ray_o = w->ray_o;
     A.ray_d = w->ray_d;
     A.hit = w->hit;
-    A.err = w->ctr + 4;
-    A.segments = reinterpret_cast<unsigned long long*>(w->ctr + 8);
+    A.ctr = w->ctr;
+    A.err = w->ctr + CTR_ERR;
+    A.segments = reinterpret_cast<unsigned long long*>(w->ctr + CTR_SEGMENTS);
     A.thr = w->thr;
     A.acc = w->acc;
     A.brdf = w->brdf;
@@ -2125,7 +2086,6 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
     lam_guide* gd = learned ? pl->guide : nullptr;
     if (gd) {
         A.dq = w->dq;
-        A.dq_count = w->ctr + 12;
         A.def_n = w->def_n;
         A.def_t = w->def_t;
         A.def_c = w->def_c;
@@ -2137,20 +2097,19 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
         A.def_lobe = w->def_lobe;
         A.def_lw = w->def_lw;
         A.rec_cap = gd->opts.record_capacity;
-        A.rec_count = w->ctr + 13;
+        A.rec_count = w->ctr + CTR_RECORDS;
         A.guide_w = gd->packed;
         std::memcpy(A.box, s->bounds, sizeof(A.box));
     }
     if (guide && !world) return set_error(LAM_ERR_INVALID_ARGUMENT, "Markov guiding needs MARKOV_CHAIN_WORLD_SPACE buffers");
-    // automatic order: sorted except under Markov guiding, which measured faster in queue order
-    const bool sorted = pl->shade_order == LAM_SHADE_ORDER_MATERIAL || (pl->shade_order == LAM_SHADE_ORDER_AUTO && !guide);
+    // automatic order: sorted except under Markov guiding, which measured faster in queue order, and in
+    // waves too small for it
+    const bool sorted = pl->shade_order == LAM_SHADE_ORDER_MATERIAL ||
+                        (pl->shade_order == LAM_SHADE_ORDER_AUTO && !guide && w->paths >= SORT_MIN_PATHS);
     if (sorted) {
-        if (!w->shade_order && (walloc(w, &w->shade_key, w->paths) || walloc(w, &w->shade_order, w->paths) ||
-                                walloc(w, &w->shade_bc, (size_t)SORT_BLOCKS_MAX * SHADE_CLASSES)))
-            return LAM_ERR_CUDA;
-        A.shade_key = w->shade_key;
-        A.shade_order = w->shade_order;
-        A.shade_bc = w->shade_bc;
+        if ((rc = ensure_order(w, w->paths))) return rc;
+        A.order_a = w->order_a;
+        A.order_b = w->order_b;
     }
     const bool alpha = !s->dev.all_opaque;
     const dim3 blk(WAVE_BLOCK);
@@ -2177,7 +2136,6 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
     auto end = [&](int h) {
         if (h >= 0) cudaEventRecord(pl->timed[h].end, st);
     };
-    cudaMemsetAsync(w->ctr, 0, 10 * sizeof(uint32_t), st);  // keeps the cumulative counter ctr[10..11]
     for (uint32_t first = 0; first < pl->opts.samples;) {
         // learned guiding: record training vertices while the guide has seen fewer than train_spp
         // samples per pixel; sample the network once it has taken a training step
@@ -2190,13 +2148,10 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
         A.wave_count = count;
         uint32_t* qa = w->queue0;
         uint32_t* qb = w->queue1;
-        uint32_t* ca = w->ctr + 0;
-        uint32_t* cb = w->ctr + 1;
         float4 *rao = w->ray_o, *rad = w->ray_d, *rbo = w->ray_o2, *rbd = w->ray_d2;  // rays of qa, qb
         float4 *tha = w->qthr0, *thb = w->qthr1, *aca = w->qacc0, *acb = w->qacc1;   // path state of qa, qb
         uint4 *mia = w->qmisc0, *mib = w->qmisc1;
         A.q_in = qa;
-        A.count_in = ca;
         A.ray_o = rao;
         A.ray_d = rad;
         A.qthr = tha;
@@ -2211,7 +2166,6 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
         }
         A.rec_head = training ? w->rec_head : nullptr;
         A.guide_frac = use_net ? gd->opts.guide_fraction : 0.0f;
-        if (training) cudaMemsetAsync(w->ctr + 13, 0, sizeof(uint32_t), st);
         int h = begin(0);
         generate_kernel<<<gpix, blk, 0, st>>>(A);
         end(h);
@@ -2219,8 +2173,7 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
         for (uint32_t depth = 0; depth < pl->opts.max_depth; ++depth) {
             A.q_in = qa;
             A.q_out = qb;
-            A.count_in = ca;
-            A.count_out = cb;
+            set_depth(A, w, depth);
             A.ray_o = rao;
             A.ray_d = rad;
             A.ray_o_out = rbo;
@@ -2231,9 +2184,6 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
             A.qthr_out = thb;
             A.qacc_out = acb;
             A.qmisc_out = mib;
-            A.work = w->ctr + 2;
-            cudaMemsetAsync(w->ctr + 2, 0, sizeof(uint32_t), st);
-            cudaMemsetAsync(cb, 0, sizeof(uint32_t), st);
             h = begin(1);
             if (proc) {
                 void* kargs[] = {&A};
@@ -2245,12 +2195,9 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
             }
             end(h);
             h = begin(2);
-            if (gd) cudaMemsetAsync(w->ctr + 12, 0, sizeof(uint32_t), st);
             if (sorted) {
-                shade_keys_kernel<false><<<w->grid_sort, blk, 0, st>>>(A);
-                shade_scan_kernel<<<1, SORT_BLOCKS_MAX, 0, st>>>(A, (uint32_t)w->grid_sort);
-                shade_scatter_kernel<<<w->grid_sort, blk, 0, st>>>(A);
-                launches += 3;
+                shade_order_kernel<false><<<w->grid_sort, blk, 0, st>>>(A);
+                ++launches;
             }
             switch (pl->quality) {
                 case LAM_QUALITY_LOW: launch_shade<LAM_QUALITY_LOW>(guide, learned, w->grid_shade, blk, st, A); break;
@@ -2269,7 +2216,6 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
             }
             end(h);
             std::swap(qa, qb);
-            std::swap(ca, cb);
             std::swap(rao, rbo);
             std::swap(rad, rbd);
             std::swap(tha, thb);
@@ -2288,7 +2234,7 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
         if (training) {
             h = begin(4);
             for (uint32_t k = 0; k < gd->opts.steps_per_wave; ++k) {
-                rc = guide_grad_and_update(gd, gd->records, GUIDE_RECORD_STRIDE, gd->opts.record_capacity, w->ctr + 13,
+                rc = guide_grad_and_update(gd, gd->records, GUIDE_RECORD_STRIDE, gd->opts.record_capacity, w->ctr + CTR_RECORDS,
                                            gd->opts.batch, false, 1.0f / (float)gd->opts.batch, s->bounds, 1u, nullptr,
                                            nullptr, st);
                 if (rc) return rc;
@@ -2442,12 +2388,12 @@ static int batch_wave_buffers(BatchState* b, uint32_t capacity) {
     rc |= walloc(w, &w->brdf, capacity);
     rc |= walloc(w, &w->seed, capacity);
     rc |= walloc(w, &w->flags, capacity);
-    rc |= walloc(w, &w->ctr, 64);
+    rc |= walloc(w, &w->ctr, CTR_WORDS);
     if (rc) {
         free_wave(w);
         return LAM_ERR_CUDA;
     }
-    cudaMemset(w->ctr, 0, 64 * sizeof(uint32_t));
+    cudaMemset(w->ctr, 0, CTR_WORDS * sizeof(uint32_t));
     b->wave = w;
     b->capacity = capacity;
     return LAM_OK;
@@ -2512,14 +2458,15 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
                                                           : (uint32_t)std::max(1, occ_e));
     const int grid_s = sms * (int)(t.shade_blocks_per_sm ? t.shade_blocks_per_sm : (uint32_t)std::max(1, occ_s));
     const BatchPlan P = plan_batch(reqs, n, t.wave_paths);
-    // material-ordered shading (no Markov guiding here, so the automatic order sorts)
-    const bool sorted = pl->shade_order != LAM_SHADE_ORDER_QUEUE;
-    const int grid_sort = std::min(SORT_BLOCKS_MAX, sms * 6);
-    if (sorted && !w->shade_order) {
+    // material-ordered shading: as lam_render chooses it for a wave of this size
+    uint64_t wave_most = 0;
+    for (uint32_t k : P.wave_paths) wave_most = std::max<uint64_t>(wave_most, k);
+    const bool sorted = pl->shade_order == LAM_SHADE_ORDER_MATERIAL ||
+                        (pl->shade_order == LAM_SHADE_ORDER_AUTO && wave_most >= SORT_MIN_PATHS);
+    const int grid_sort = sms * 6;
+    if (sorted && !w->order_a) {
         b->generation++;  // a captured graph does not know the new buffers
-        if (walloc(w, &w->shade_key, b->capacity) || walloc(w, &w->shade_order, b->capacity) ||
-            walloc(w, &w->shade_bc, (size_t)SORT_BLOCKS_MAX * SHADE_CLASSES))
-            return LAM_ERR_CUDA;
+        if ((rc = ensure_order(w, b->capacity))) return rc;
     }
     // device tables (uploaded before any capture)
     if (dgrow(b, &b->reqs, &b->reqs_cap, n) || dgrow(b, &b->segs, &b->segs_cap, P.segs.size()) ||
@@ -2567,8 +2514,9 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
     A.ray_o = w->ray_o;
     A.ray_d = w->ray_d;
     A.hit = w->hit;
-    A.err = w->ctr + 4;
-    A.segments = reinterpret_cast<unsigned long long*>(w->ctr + 8);
+    A.ctr = w->ctr;
+    A.err = w->ctr + CTR_ERR;
+    A.segments = reinterpret_cast<unsigned long long*>(w->ctr + CTR_SEGMENTS);
     A.thr = w->thr;
     A.acc = w->acc;
     A.brdf = w->brdf;
@@ -2580,15 +2528,13 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
     A.req_done = b->done;
     A.req_time = b->times;
     if (sorted) {
-        A.shade_key = w->shade_key;
-        A.shade_order = w->shade_order;
-        A.shade_bc = w->shade_bc;
+        A.order_a = w->order_a;
+        A.order_b = w->order_b;
     }
     const dim3 blk(WAVE_BLOCK);
     uint32_t launches = 0;
     auto record = [&]() {
-        cudaMemsetAsync(w->ctr, 0, 10 * sizeof(uint32_t), st);
-        batch_start_kernel<<<1, 256, 0, st>>>(b->done, b->times, n);
+        batch_start_kernel<<<1, 256, 0, st>>>(w->ctr, b->done, b->times, n);
         for (size_t wv = 0; wv < P.wave_begin.size(); ++wv) {
             A.segs = b->segs + P.wave_begin[wv];
             A.nsegs = P.wave_nsegs[wv];
@@ -2596,13 +2542,10 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
             A.npix = P.wave_paths[wv];
             uint32_t* qa = w->queue0;
             uint32_t* qb = w->queue1;
-            uint32_t* ca = w->ctr + 0;
-            uint32_t* cb = w->ctr + 1;
             float4 *rao = w->ray_o, *rad = w->ray_d, *rbo = w->ray_o2, *rbd = w->ray_d2;  // rays of qa, qb
             float4 *tha = w->qthr0, *thb = w->qthr1, *aca = w->qacc0, *acb = w->qacc1;   // path state of qa, qb
             uint4 *mia = w->qmisc0, *mib = w->qmisc1;
             A.q_in = qa;
-            A.count_in = ca;
             A.ray_o = rao;
             A.ray_d = rad;
             A.qthr = tha;
@@ -2613,8 +2556,7 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
             for (uint32_t depth = 0; depth < pl->opts.max_depth; ++depth) {
                 A.q_in = qa;
                 A.q_out = qb;
-                A.count_in = ca;
-                A.count_out = cb;
+                set_depth(A, w, depth);
                 A.ray_o = rao;
                 A.ray_d = rad;
                 A.ray_o_out = rbo;
@@ -2625,16 +2567,11 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
                 A.qthr_out = thb;
                 A.qacc_out = acb;
                 A.qmisc_out = mib;
-                A.work = w->ctr + 2;
-                cudaMemsetAsync(w->ctr + 2, 0, sizeof(uint32_t), st);
-                cudaMemsetAsync(cb, 0, sizeof(uint32_t), st);
                 if (all_opaque) extend_batch_kernel<false><<<grid_e, blk, 0, st>>>(A);
                 else extend_batch_kernel<true><<<grid_e, blk, 0, st>>>(A);
                 if (sorted) {
-                    shade_keys_kernel<true><<<grid_sort, blk, 0, st>>>(A);
-                    shade_scan_kernel<<<1, SORT_BLOCKS_MAX, 0, st>>>(A, (uint32_t)grid_sort);
-                    shade_scatter_kernel<<<grid_sort, blk, 0, st>>>(A);
-                    launches += 3;
+                    shade_order_kernel<true><<<grid_sort, blk, 0, st>>>(A);
+                    ++launches;
                 }
                 switch (pl->quality) {
                     case LAM_QUALITY_LOW: shade_kernel<LAM_QUALITY_LOW, false, false, true><<<grid_s, blk, 0, st>>>(A); break;
@@ -2643,8 +2580,7 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
                 }
                 launches += 2;
                 std::swap(qa, qb);
-                std::swap(ca, cb);
-                std::swap(rao, rbo);
+                    std::swap(rao, rbo);
                 std::swap(rad, rbd);
                 std::swap(tha, thb);
                 std::swap(aca, acb);

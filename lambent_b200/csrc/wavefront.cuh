@@ -13,7 +13,23 @@ constexpr uint32_t NO_REC = 0xFFFFFFFFu;
 // classes of material-ordered shading: what a bounce runs differs between sky lanes, diffuse,
 // metallic and transparent vertices
 enum : uint32_t { SHADE_SKY = 0u, SHADE_DIFFUSE = 1u, SHADE_METALLIC = 2u, SHADE_TRANSPARENT = 3u, SHADE_CLASSES = 4u };
-constexpr int SORT_BLOCKS_MAX = 1024;  // blocks of the class-count and scatter kernels (one scan block)
+// Smallest wave (paths) that the automatic order sorts: below it the sort's launches cost more than the
+// uniform warps save.  Queue against material order, 8 bounces: Cornell box 65,536 paths 293 / 323 us,
+// 262,144 504 / 488, 524,288 861 / 790; icosphere field 262,144 1880 / 1890, 524,288 2693 / 2675.
+constexpr uint64_t SORT_MIN_PATHS = 1u << 18;
+
+// Device counters of a wave (WaveBuffers::ctr), in words.  [0, CTR_WAVE) belong to a render or batch;
+// the rest hold one entry per bounce and are cleared by the wave's generate kernel, so that no bounce
+// needs a memset of its own.
+constexpr uint32_t MAX_BOUNCES = 255;
+enum : uint32_t {
+    CTR_ERR = 4, CTR_SEGMENTS = 8, CTR_TOTAL = 10, CTR_RECORDS = 13, CTR_WAVE = 64,
+    CTR_COUNT = CTR_WAVE,                      // paths queued at each depth (one more than bounces)
+    CTR_WORK = CTR_COUNT + MAX_BOUNCES + 1,    // extend's work counter
+    CTR_DEFERRED = CTR_WORK + MAX_BOUNCES,     // vertices deferred to the learned guide
+    CTR_CLASS = CTR_DEFERRED + MAX_BOUNCES,    // hits of each shading class
+    CTR_WORDS = CTR_CLASS + 4 * MAX_BOUNCES
+};
 
 // ---------------------------------------------------------------- batched renders
 // A request of lam_batch_render: its scene, camera, image and samples.
@@ -53,11 +69,11 @@ struct Args {
     float4 *qthr_out, *qacc_out;
     uint4* qmisc_out;
     uint2* hit;  // (triangle slot, instance) of the closest hit, by position in the current queue
-    // material-ordered shading (lam_pipeline_set_shade_order): the class of each queued hit, the queue
-    // positions in class order (null: the shade kernel takes them in queue order), and per-block class
-    // counts, which the scan turns into the blocks' first output slots
-    uint8_t* shade_key;
-    uint32_t *shade_order, *shade_bc;
+    // material-ordered shading (lam_pipeline_set_shade_order): the queue positions by class, one list
+    // from each end of order_a (sky, diffuse) and order_b (metallic, transparent), and the bounce's four
+    // class counts; order_a null: the shade kernel takes the positions in queue order
+    uint32_t *order_a, *order_b, *class_count;
+    uint32_t* ctr;  // all counters of the wave, which the generate kernel clears
     uint32_t *q_in, *q_out;
     uint32_t *count_in, *count_out, *work;
     uint32_t* err;
