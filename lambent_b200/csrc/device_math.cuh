@@ -141,7 +141,11 @@ LAM_DEV uint32_t pack_snorm16(float e) {
     int32_t v = (int32_t)floorf(0.5f + 32767.0f * c);
     return (uint32_t)(uint16_t)(int16_t)v;
 }
-LAM_DEV float unpack_snorm16(uint32_t h) { return fmaxf((float)(int16_t)(uint16_t)h / 32767.0f, -1.0f); }
+LAM_DEV float unpack_snorm16(uint32_t h) {
+    const float x = (float)(int16_t)(uint16_t)h, rc = 1.0f / 32767.0f;
+    const float q = __fmul_rn(x, rc);  // x / 32767 with one correction, exact for all 65,536 values (byte_over_255)
+    return fmaxf(__fmaf_rn(__fmaf_rn(-q, 32767.0f, x), rc, q), -1.0f);
+}
 LAM_DEV uint32_t normalised_to_u32(v3 n) {
     v3 v = n / fmaxf(fabsf(n.x) + fabsf(n.y) + fabsf(n.z), 0.01f);
     if (v.y >= 0.0f) return pack_snorm16(v.x) | (pack_snorm16(v.z) << 16);

@@ -16,6 +16,7 @@
 #include "guide.cuh"
 #include "guide_net.cuh"
 #include "materials.cuh"
+#include "reservoir.cuh"
 #include "scene.h"
 #include "tracer.h"
 #include "traverse.cuh"
@@ -317,7 +318,7 @@ __global__ void __launch_bounds__(WAVE_BLOCK) generate_kernel(Args A) {
             mc_store(A.tent_live + p, t);
             mc_store(A.tent_snap + p, t);
         }
-        if (A.reservoirs && A.restir == LAM_RESTIR_PER_SAMPLE) A.reservoirs[p] = lam_reservoir{};
+        if (A.reservoirs && A.restir == LAM_RESTIR_PER_SAMPLE) res_store(A.reservoirs + p, lam_reservoir{});
     } else {
         st = A.pixel_seed[p];
         if (A.tent_live) mc_store(A.tent_live + p, mc_load(A.tent_snap + p));
@@ -1425,6 +1426,21 @@ LAM_DEV float res_p_hat(const lam_reservoir& R) {
 template <int Q>
 __global__ void __launch_bounds__(WAVE_BLOCK) accumulate_kernel(Args A, uint32_t is_last_wave) {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (is_last_wave && A.restir != LAM_RESTIR_DISABLED && A.info) {
+        // the block's 36-byte surface records through shared memory, so that they leave in whole lines
+        __shared__ float rec[WAVE_BLOCK * 9];
+        if (p < A.npix) {
+            const float4 e = A.pix_emission[p], al = A.pix_albedo[p];
+            const float v[9] = {A.camera_pos.x, A.camera_pos.y, A.camera_pos.z, e.x, e.y, e.z, al.x, al.y, al.z};
+#pragma unroll
+            for (int q = 0; q < 9; ++q) rec[threadIdx.x * 9u + q] = v[q];
+        }
+        __syncthreads();
+        const uint32_t first = blockIdx.x * WAVE_BLOCK;
+        const uint32_t words = min((uint32_t)WAVE_BLOCK, A.npix - first) * 9u;
+        float* out = reinterpret_cast<float*>(A.info) + (size_t)first * 9u;
+        for (uint32_t q = threadIdx.x; q < words; q += WAVE_BLOCK) out[q] = rec[q];
+    }
     if (p >= A.npix) return;
     float4 pc = A.pix_color[p];
     v3 col = mk(pc.x, pc.y, pc.z);
@@ -1444,7 +1460,7 @@ __global__ void __launch_bounds__(WAVE_BLOCK) accumulate_kernel(Args A, uint32_t
         if (A.restir == LAM_RESTIR_PER_SAMPLE && A.reservoirs) {
             float4 pp = A.ppoint[path], pn = A.pnormal[path], vp = A.vpoint[path], vn = A.vnormal[path], o = A.orad[path];
             uint32_t ty = __float_as_uint(pp.w);
-            lam_reservoir R = A.reservoirs[p];
+            lam_reservoir R = res_load(A.reservoirs + p);
             if (ty != TY_SKY) {
                 v3 orr = mk(o.x, o.y, o.z);
                 float w = fmaxf(len(orr), 0.00001f);
@@ -1457,7 +1473,7 @@ __global__ void __launch_bounds__(WAVE_BLOCK) accumulate_kernel(Args A, uint32_t
             } else {
                 R.ty = TY_SKY;
             }
-            A.reservoirs[p] = R;
+            res_store(A.reservoirs + p, R);
         }
     }
     A.pix_color[p] = make_float4(col.x, col.y, col.z, 0.0f);
@@ -1469,15 +1485,12 @@ __global__ void __launch_bounds__(WAVE_BLOCK) accumulate_kernel(Args A, uint32_t
         A.out_color[p] = make_float4(fmaxf(c.x, 0.0f), fmaxf(c.y, 0.0f), fmaxf(c.z, 0.0f), 1.0f);
     }
     const uint32_t last_path = (A.wave_count - 1u) * A.npix + p;
-    if (A.restir != LAM_RESTIR_DISABLED && A.info) {
-        float4 e = A.pix_emission[p], al = A.pix_albedo[p];
-        lam_info inf;
-        inf.arr[0] = A.camera_pos.x; inf.arr[1] = A.camera_pos.y; inf.arr[2] = A.camera_pos.z;
-        inf.arr[3] = e.x; inf.arr[4] = e.y; inf.arr[5] = e.z;
-        inf.arr[6] = al.x; inf.arr[7] = al.y; inf.arr[8] = al.z;
-        A.info[p] = inf;
+    if (A.tent_snap && A.chains && p < A.chains_len) {
+        const float4* from = reinterpret_cast<const float4*>(A.tent_snap + p);
+        float4* to = reinterpret_cast<float4*>(A.chains + p);
+        to[0] = from[0];
+        to[1] = from[1];
     }
-    if (A.tent_snap && A.chains && p < A.chains_len) A.chains[p] = A.tent_snap[p];
     if (A.reservoirs) {
         if (A.restir == LAM_RESTIR_PER_PIXEL) {
             float4 pp = A.ppoint[last_path], pn = A.pnormal[last_path], vp = A.vpoint[last_path], vn = A.vnormal[last_path];
@@ -1494,9 +1507,9 @@ __global__ void __launch_bounds__(WAVE_BLOCK) accumulate_kernel(Args A, uint32_t
             } else {
                 R.ty = TY_SKY;
             }
-            A.reservoirs[p] = R;
+            res_store(A.reservoirs + p, R);
         } else if (A.restir == LAM_RESTIR_DISABLED) {
-            A.reservoirs[p] = lam_reservoir{};
+            res_store(A.reservoirs + p, lam_reservoir{});
         }
     }
 }
