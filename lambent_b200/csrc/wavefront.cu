@@ -1094,8 +1094,30 @@ __global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(cons
 // One-sample MIS of the cosine lobe (probability 1 - f) and the network's vMF mixture (probability f):
 // pdf(w) = (1 - f) cos/pi + f q(w).  With NET false (untrained network, f = 0) this is the plain cosine
 // branch of the shade kernel, with the same seeds and the same arithmetic.
-constexpr uint32_t GUIDE_SMEM = net::LAYERS * net::LAYER_BYTES + 2u * net::X_BYTES + 64u + 128u;
-constexpr uint32_t GUIDE_TMEM_COLS = 128;  // accumulators of tiles A (columns 0..63) and B (64..127)
+// Two warpgroups per CTA share the weights in shared memory (32 KB) and nothing else: each runs its own
+// pairs of tiles, with its own two tiles, barriers and 128 TMEM columns.  Two such CTAs fit an SM, 16
+// warps; with one warpgroup per CTA the weights' copies left room for 12.  With the finished vertices
+// handed on in registers: 1,028 -> 839 us for the eight bounces of 2.1M paths (960x540, 4 spp); bound by
+// issue and the latency of the rows' scalar work (encoding, lobes, sampling).
+constexpr int GUIDE_GROUPS = 2, GUIDE_BLOCK = GUIDE_GROUPS * WAVE_BLOCK;
+constexpr uint32_t GUIDE_SMEM = net::LAYERS * net::LAYER_BYTES + GUIDE_GROUPS * 2u * net::X_BYTES + 64u + 128u;
+constexpr uint32_t GUIDE_TMEM_GROUP = 128;  // accumulators of tiles A (columns 0..63) and B (64..127)
+constexpr uint32_t GUIDE_TMEM_COLS = GUIDE_GROUPS * GUIDE_TMEM_GROUP;
+
+// Barrier of warpgroup g's 128 threads; the OR of their flags.
+LAM_DEV bool group_or(uint32_t g, bool flag) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "barrier.cta.red.or.pred q, %2, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t"
+        "}\n"
+        : "=r"(r)
+        : "r"(flag ? 1u : 0u), "r"(g + 1u)
+        : "memory");
+    return r != 0u;
+}
 
 // The Markov sampler's mixture pdf at w from the lobes the shade kernel kept for the path:
 // c0 cos/pi + sum_k w_k vMF_k(w), where w_k already includes the vMF branch's probability.
@@ -1143,13 +1165,22 @@ LAM_DEV void record_vertex(const Args& A, uint32_t path, uint32_t seed0, v3 ro, 
 // (the reference's weight of this bounce is 1 once the albedo is in the throughput, i.e. the BSDF
 // times the cosine equals the albedo times p_metal).  Untrained (NET false) it is the reference's
 // bounce, unchanged.
+// What a finished vertex hands to the next queue (registers from here to the append: through memory it
+// was 52 bytes written by slot and read back).
+struct GuideOut {
+    float4 thr, acc;
+    v3 dir;
+    float brdf;
+    uint32_t seed, flags;
+};
+
 template <bool NET, bool MARKOV>
-LAM_DEV void guide_finish_metal(const Args& A, uint32_t q, uint32_t path, const net::Lobes* L) {
+LAM_DEV void guide_finish_metal(const Args& A, uint32_t q, uint32_t path, const net::Lobes* L, GuideOut& out) {
     const uint32_t v = MARKOV ? path : q;  // where the shade kernel left the vertex's records
     const float4 d4 = A.def_d[q], dn = A.def_n[v], dt = A.def_t[v], dr = A.def_r[v];
     v3 dir = mk(dr.x, dr.y, dr.z);
     if (NET) {
-        const float4 th = A.thr[q];
+        const float4 th = out.thr;
         const v3 rd = mk(d4.x, d4.y, d4.z), n = mk(dn.x, dn.y, dn.z), t = mk(dt.x, dt.y, dt.z);
         const uint32_t seed0 = __float_as_uint(dt.w);
         const float f = A.guide_frac;
@@ -1166,13 +1197,13 @@ LAM_DEV void guide_finish_metal(const Args& A, uint32_t q, uint32_t path, const 
         const float pm = metal_pdf(rd, n, t, dn.w, dr.w, dir);
         const float mix = (1.0f - f) * pm + f * net::mixture_pdf(*L, dir);
         const float wgt = mix > 0.0f ? pm / mix : 0.0f;
-        A.thr[q] = make_float4(th.x * wgt, th.y * wgt, th.z * wgt, th.w);
+        out.thr = make_float4(th.x * wgt, th.y * wgt, th.z * wgt, th.w);
         if (MARKOV) {
             const float4 oc = A.ort[path];
             A.ort[path] = make_float4(oc.x * wgt, oc.y * wgt, oc.z * wgt, oc.w);
         }
     }
-    A.def_d[q] = make_float4(dir.x, dir.y, dir.z, 0.0f);
+    out.dir = dir;
 }
 
 // The vertex at guide queue slot q of path `path`: its live state (origin, direction, throughput,
@@ -1181,15 +1212,20 @@ LAM_DEV void guide_finish_metal(const Args& A, uint32_t q, uint32_t path, const 
 // shade kernel (MARKOV), which keeps it and the Markov draw and lobes by path.  Training records are
 // kept by path.
 template <int Q, bool NET, bool MARKOV>
-LAM_DEV void guide_finish(const Args& A, uint32_t q, uint32_t path, const net::Lobes* L, bool& out) {
+LAM_DEV GuideOut guide_finish(const Args& A, uint32_t q, uint32_t path, const net::Lobes* L) {
     const uint32_t v = MARKOV ? path : q;
+    GuideOut out;
+    out.thr = A.thr[q];
+    out.acc = A.def_a[q];
+    out.brdf = A.brdf[q];
+    out.seed = A.seed[q];
+    out.flags = A.flags[q];
     if (A.def_kind[v] == DEF_METAL) {
-        guide_finish_metal<NET, MARKOV>(A, q, path, L);
-        out = true;
-        return;
+        guide_finish_metal<NET, MARKOV>(A, q, path, L, out);
+        return out;
     }
     const float4 o4 = A.def_o[q], d4 = A.def_d[q], dn = A.def_n[v], dt = A.def_t[v], dc = A.def_c[v];
-    const float4 th = A.thr[q], ac = A.def_a[q];
+    const float4 th = out.thr, ac = out.acc;
     const v3 ro = mk(o4.x, o4.y, o4.z), rd = mk(d4.x, d4.y, d4.z), n = mk(dn.x, dn.y, dn.z), t = mk(dt.x, dt.y, dt.z);
     const uint32_t seed0 = __float_as_uint(dt.w);
     v3 color = mk(th.x, th.y, th.z);
@@ -1212,7 +1248,7 @@ LAM_DEV void guide_finish(const Args& A, uint32_t q, uint32_t path, const net::L
                 const float u2 = rand_f32(h);
                 dir = net::mixture_sample(*L, u0, u1, u2);
                 pdf = markov_mixture_pdf(A, path, dc.w, n, dir);
-                A.flags[q] |= 0x100u;  // not drawn from a chain's vMF lobe (general.wesl:469-472)
+                out.flags |= 0x100u;  // not drawn from a chain's vMF lobe (general.wesl:469-472)
             }
             pdf = (1.0f - f) * pdf + f * net::mixture_pdf(*L, dir);
         }
@@ -1247,40 +1283,46 @@ LAM_DEV void guide_finish(const Args& A, uint32_t q, uint32_t path, const net::L
         const v3 orc = (mk(oc.x, oc.y, oc.z) * nf) * diffuse;
         A.ort[path] = make_float4(orc.x, orc.y, orc.z, oc.w);
     }
-    A.thr[q] = make_float4(color.x, color.y, color.z, th.w);
-    A.brdf[q] = cached_brdf;
-    A.def_a[q] = make_float4(ac.x, ac.y, ac.z, pdf);
-    A.def_d[q] = make_float4(dir.x, dir.y, dir.z, 0.0f);
+    out.thr = make_float4(color.x, color.y, color.z, th.w);
+    out.brdf = cached_brdf;
+    out.acc = make_float4(ac.x, ac.y, ac.z, pdf);
+    out.dir = dir;
     record_vertex(A, path, seed0, ro, n, rd, dir, color_pre, ac);
-    out = true;
+    return out;
+}
+
+// Appends the warp's finished vertices to the next queue.
+LAM_DEV void guide_append(const Args& A, bool go, uint32_t q, uint32_t path, const GuideOut& out) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t mask = __ballot_sync(0xFFFFFFFFu, go);
+    uint32_t slot = 0;
+    if (lane == 0 && mask) slot = atomicAdd(A.count_out, __popc(mask));
+    slot = __shfl_sync(0xFFFFFFFFu, slot, 0);
+    if (go) {
+        const uint32_t s = slot + __popc(mask & ((1u << lane) - 1u));
+        A.q_out[s] = path;
+        A.ray_o_out[s] = A.def_o[q];
+        A.ray_d_out[s] = make_float4(out.dir.x, out.dir.y, out.dir.z, 0.0f);
+        A.qthr_out[s] = out.thr;
+        A.qacc_out[s] = out.acc;
+        A.qmisc_out[s] = make_uint4(__float_as_uint(out.brdf), out.seed, out.flags, 0u);
+    }
 }
 
 template <int Q, bool NET, bool MARKOV>
-__global__ void __launch_bounds__(WAVE_BLOCK) guide_sample_kernel(Args A) {
+__global__ void __launch_bounds__(NET ? GUIDE_BLOCK : WAVE_BLOCK) guide_sample_kernel(const __grid_constant__ Args A) {
     const uint32_t n = *A.dq_count;
     const uint32_t lane = threadIdx.x & 31u;
     if (!NET) {
         for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; base < n; base += gridDim.x * blockDim.x) {
             const uint32_t i = base + lane;
-            bool go = false;
             uint32_t path = 0;
+            GuideOut out;
             if (i < n) {
                 path = A.dq[i];
-                guide_finish<Q, false, MARKOV>(A, i, path, nullptr, go);
+                out = guide_finish<Q, false, MARKOV>(A, i, path, nullptr);
             }
-            const uint32_t mask = __ballot_sync(0xFFFFFFFFu, go);
-            uint32_t slot = 0;
-            if (lane == 0 && mask) slot = atomicAdd(A.count_out, __popc(mask));
-            slot = __shfl_sync(0xFFFFFFFFu, slot, 0);
-            if (go) {
-                const uint32_t s = slot + __popc(mask & ((1u << lane) - 1u));
-                A.q_out[s] = path;
-                A.ray_o_out[s] = A.def_o[i];
-                A.ray_d_out[s] = A.def_d[i];
-                A.qthr_out[s] = A.thr[i];
-                A.qacc_out[s] = A.def_a[i];
-                A.qmisc_out[s] = make_uint4(__float_as_uint(A.brdf[i]), A.seed[i], A.flags[i], 0u);
-            }
+            guide_append(A, i < n, i, path, out);
         }
         return;
     }
@@ -1289,16 +1331,18 @@ __global__ void __launch_bounds__(WAVE_BLOCK) guide_sample_kernel(Args A) {
     extern __shared__ uint8_t smraw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smraw) + 127u) & ~uintptr_t(127));
     uint8_t* W = sm;
-    uint8_t* XA = sm + net::LAYERS * net::LAYER_BYTES;
+    const uint32_t group = threadIdx.x >> 7, row = threadIdx.x & 127u;
+    uint8_t* XA = sm + net::LAYERS * net::LAYER_BYTES + group * 2u * net::X_BYTES;
     uint8_t* XB = XA + net::X_BYTES;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(XB + net::X_BYTES);
-    uint32_t* slot_t = reinterpret_cast<uint32_t*>(bars + 2);
+    uint64_t* all_bars = reinterpret_cast<uint64_t*>(sm + net::LAYERS * net::LAYER_BYTES + GUIDE_GROUPS * 2u * net::X_BYTES);
+    uint64_t* bars = all_bars + 2u * group;
+    uint32_t* slot_t = reinterpret_cast<uint32_t*>(all_bars + 2u * GUIDE_GROUPS);
     {
         const uint4* src = reinterpret_cast<const uint4*>(A.guide_w);
         uint4* dst = reinterpret_cast<uint4*>(W);
         for (uint32_t i = threadIdx.x; i < net::LAYERS * net::LAYER_BYTES / 16u; i += blockDim.x) dst[i] = src[i];
     }
-    if (threadIdx.x == 0) {
+    if (row == 0) {
         net::mbar_init(bars);
         net::mbar_init(bars + 1);
     }
@@ -1306,15 +1350,15 @@ __global__ void __launch_bounds__(WAVE_BLOCK) guide_sample_kernel(Args A) {
     net::fence_before();
     __syncthreads();
     net::fence_after();
-    const uint32_t tmem = *slot_t;
+    const uint32_t tmem_all = *slot_t, tmem = tmem_all + group * GUIDE_TMEM_GROUP;
     const uint32_t bar_a = net::smem_u32(bars), bar_b = net::smem_u32(bars + 1);
     const uint32_t w_addr = net::smem_u32(W), xa = net::smem_u32(XA), xb = net::smem_u32(XB);
-    const uint32_t t_row = tmem + ((threadIdx.x & ~31u) << 16);
+    const uint32_t t_row = tmem + ((row & ~31u) << 16);
     uint32_t phase = 0;
     bool failed = false;
     const uint32_t pairs = (n + 2u * net::TILE - 1) / (2u * net::TILE);
-    for (uint32_t pair = blockIdx.x; pair < pairs; pair += gridDim.x) {
-        const uint32_t ia = pair * 2u * net::TILE + threadIdx.x, ib = ia + net::TILE;
+    for (uint32_t pair = blockIdx.x * GUIDE_GROUPS + group; pair < pairs; pair += gridDim.x * GUIDE_GROUPS) {
+        const uint32_t ia = pair * 2u * net::TILE + row, ib = ia + net::TILE;
         const bool va = ia < n, vb = ib < n;
         const uint32_t pa = va ? A.dq[ia] : 0u, pb = vb ? A.dq[ib] : 0u;
         // origin and direction are stored by slot (rows ia and ib are read in order); the normal too,
@@ -1333,7 +1377,7 @@ __global__ void __launch_bounds__(WAVE_BLOCK) guide_sample_kernel(Args A) {
             }
             float f[net::WIDTH];
             net::encode_features(q, A.box, f);
-            net::store_row(X, net::X_RG, threadIdx.x, f);
+            net::store_row(X, net::X_RG, row, f);
         };
         query(va, ia, pa, XA);
         query(vb, ib, pb, XB);
@@ -1341,12 +1385,12 @@ __global__ void __launch_bounds__(WAVE_BLOCK) guide_sample_kernel(Args A) {
         for (uint32_t l = 0; l < (uint32_t)net::LAYERS; ++l) {
             net::fence_async_smem();
             net::fence_before();
-            if (__syncthreads_or(failed ? 1 : 0)) {
+            if (group_or(group, failed)) {
                 failed = true;
                 ok = false;
                 break;
             }
-            if (threadIdx.x == 0) {
+            if (row == 0) {
                 net::fence_after();
                 net::issue_fwd(tmem, xa, w_addr + l * net::LAYER_BYTES);
                 net::mma_commit(bar_a);
@@ -1355,10 +1399,10 @@ __global__ void __launch_bounds__(WAVE_BLOCK) guide_sample_kernel(Args A) {
             }
             if (!net::mbar_wait(bar_a, phase)) failed = true;
             net::fence_after();
-            if (l < 3u) net::epilogue_relu(t_row, XA, threadIdx.x);
+            if (l < 3u) net::epilogue_relu(t_row, XA, row);
             if (!net::mbar_wait(bar_b, phase)) failed = true;
             net::fence_after();
-            if (l < 3u) net::epilogue_relu(t_row + 64u, XB, threadIdx.x);
+            if (l < 3u) net::epilogue_relu(t_row + 64u, XB, row);
             phase ^= 1u;
         }
         if (!ok) break;
@@ -1367,25 +1411,13 @@ __global__ void __launch_bounds__(WAVE_BLOCK) guide_sample_kernel(Args A) {
             const uint32_t path = h == 0u ? pa : pb, q = h == 0u ? ia : ib;
             float raw[net::OUT];
             net::head_read(t_row + 64u * h, raw);
-            bool go = false;
+            GuideOut out;
             if (v) {
                 net::Lobes L;
                 net::lobes_from_raw(raw, L);
-                guide_finish<Q, true, MARKOV>(A, q, path, &L, go);
+                out = guide_finish<Q, true, MARKOV>(A, q, path, &L);
             }
-            const uint32_t mask = __ballot_sync(0xFFFFFFFFu, go);
-            uint32_t slot = 0;
-            if (lane == 0 && mask) slot = atomicAdd(A.count_out, __popc(mask));
-            slot = __shfl_sync(0xFFFFFFFFu, slot, 0);
-            if (go) {
-                const uint32_t s = slot + __popc(mask & ((1u << lane) - 1u));
-                A.q_out[s] = path;
-                A.ray_o_out[s] = A.def_o[q];
-                A.ray_d_out[s] = A.def_d[q];
-                A.qthr_out[s] = A.thr[q];
-                A.qacc_out[s] = A.def_a[q];
-                A.qmisc_out[s] = make_uint4(__float_as_uint(A.brdf[q]), A.seed[q], A.flags[q], 0u);
-            }
+            guide_append(A, v, q, path, out);
         }
     }
     if (failed) {
@@ -1398,7 +1430,7 @@ __global__ void __launch_bounds__(WAVE_BLOCK) guide_sample_kernel(Args A) {
     if (failed && threadIdx.x == 0) atomicOr(A.err, 1u << 8);
     if (threadIdx.x < 32) {
         net::fence_after();
-        net::tmem_free(tmem, GUIDE_TMEM_COLS);
+        net::tmem_free(tmem_all, GUIDE_TMEM_COLS);
     }
 }
 
@@ -1675,7 +1707,7 @@ static int ensure_wave(lam_pipeline* pl, uint32_t width, uint32_t height, bool f
         attrs((const void*)guide_sample_kernel<LAM_QUALITY_MEDIUM, true, true>);
         attrs((const void*)guide_sample_kernel<LAM_QUALITY_HIGH, true, true>);
         // resident CTAs per SM from the kernel's registers and shared memory (the occupancy query
-        // under-reports this kernel); at most 4 keep the 128-column TMEM allocations within 512 columns
+        // under-reports this kernel); at most 2 keep the 256-column TMEM allocations within 512 columns
         cudaFuncAttributes fa{};
         int regs_sm = 0, smem_sm = 0, smem_reserved = 0;
         const void* sized = guide ? (const void*)guide_sample_kernel<LAM_QUALITY_MEDIUM, true, true>
@@ -1688,10 +1720,10 @@ static int ensure_wave(lam_pipeline* pl, uint32_t width, uint32_t height, bool f
             free_wave(w);
             return cuda_error(e, "guide kernel attributes");
         }
-        const int regs_block = ((fa.numRegs + 7) / 8) * 8 * WAVE_BLOCK;
+        const int regs_block = ((fa.numRegs + 7) / 8) * 8 * GUIDE_BLOCK;
         const int by_regs = regs_block > 0 ? regs_sm / regs_block : 1;
         const int by_smem = smem_sm / (int)(GUIDE_SMEM + fa.sharedSizeBytes + smem_reserved);
-        w->grid_guide = w->sms * std::min(4, std::max(1, std::min(by_regs, by_smem)));
+        w->grid_guide = w->sms * std::min(512 / (int)GUIDE_TMEM_COLS, std::max(1, std::min(by_regs, by_smem)));
     }
     pl->wave = w;
     return LAM_OK;
@@ -1728,10 +1760,10 @@ int ensure_handler(lam_pipeline* pl) {
 template <int Q>
 static void launch_guide(bool net, bool markov, int grid, cudaStream_t st, const Args& A) {
     if (markov) {
-        if (net) guide_sample_kernel<Q, true, true><<<grid, WAVE_BLOCK, GUIDE_SMEM, st>>>(A);
+        if (net) guide_sample_kernel<Q, true, true><<<grid, GUIDE_BLOCK, GUIDE_SMEM, st>>>(A);
         else guide_sample_kernel<Q, false, true><<<grid, WAVE_BLOCK, 0, st>>>(A);
     } else {
-        if (net) guide_sample_kernel<Q, true, false><<<grid, WAVE_BLOCK, GUIDE_SMEM, st>>>(A);
+        if (net) guide_sample_kernel<Q, true, false><<<grid, GUIDE_BLOCK, GUIDE_SMEM, st>>>(A);
         else guide_sample_kernel<Q, false, false><<<grid, WAVE_BLOCK, 0, st>>>(A);
     }
 }
