@@ -5,7 +5,8 @@
 //   guide_eval_kernel    128-row tiles: features -> 4 tcgen05 layers -> 40 head outputs per query
 //   guide_grad_kernel    forward + backward of 128-row tiles; weight gradients accumulate in TMEM
 //                        across the tiles of a CTA and leave as one f32 partial per CTA
-//   guide_update_kernel  sums the partials in a fixed order (deterministic) and applies Adam
+//   guide_sum_kernel     sums the partials in a fixed order (deterministic)
+//   guide_train_kernel   a run of Adam steps in one cooperative launch: gradients, sums, updates
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -19,12 +20,13 @@ namespace lam {
 namespace net {
 
 constexpr uint32_t ERR_MMA_TIMEOUT = 1u << 8;
-constexpr uint32_t EVAL_SMEM = LAYERS * LAYER_BYTES + X_BYTES + 64u + 128u;
-// The last 32 KB are slack: every MMA operand extent stays inside its own tile, and the slack keeps
-// even a misread of the MN-major gradient operand's strides inside this CTA's shared memory.
-constexpr uint32_t GRAD_SMEM = LAYERS * LAYER_BYTES + 4u * X_BYTES + G_BYTES + 64u + 128u + 32768u;
+// Evaluation: two warpgroups per CTA share the weights; each runs pairs of tiles, tile B's MMAs under tile
+// A's epilogue, with its own tiles, barriers and 128 TMEM columns (as the render's sampling kernel does).
+constexpr uint32_t EVAL_GROUPS = 2u, EVAL_THREADS = EVAL_GROUPS * TILE;
+constexpr uint32_t EVAL_SMEM = LAYERS * LAYER_BYTES + EVAL_GROUPS * 2u * X_BYTES + 64u + 128u;
+constexpr uint32_t GRAD_SMEM = LAYERS * LAYER_BYTES + 4u * X_BYTES + G_BYTES + 64u + TILE * LOBES * 4u + 128u;
 constexpr uint32_t GRAD_TMEM_COLS = 512;  // acc 0..63, dW[l] at 64 (l + 1)
-constexpr uint32_t EVAL_TMEM_COLS = 64;
+constexpr uint32_t EVAL_TMEM_COLS = EVAL_GROUPS * 128u;
 
 LAM_DEV uint8_t* align128(uint8_t* p) {
     return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 127u) & ~uintptr_t(127));
@@ -53,48 +55,102 @@ struct EvalArgs {
     float* out;            // n x 40
     uint32_t* err;
     uint32_t wait_tries;   // polls of each completion wait before it gives up
+    uint32_t out_aligned;  // out is a multiple of 16
 };
 
-__global__ void __launch_bounds__(128) guide_eval_kernel(EvalArgs A) {
+// 100,003 queries: 41 us with one warpgroup and one tile at a time per CTA and 40 separate 4-byte stores per
+// row, 22 us here.
+__global__ void __launch_bounds__(EVAL_THREADS, 2) guide_eval_kernel(const __grid_constant__ EvalArgs A) {
     extern __shared__ uint8_t smraw[];
-    uint8_t* sm = align128(smraw);
-    uint8_t* W = sm;
-    uint8_t* X = sm + LAYERS * LAYER_BYTES;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(X + X_BYTES);
-    uint32_t* slot = reinterpret_cast<uint32_t*>(X + X_BYTES + 8);
+    const uint32_t group = threadIdx.x / TILE, row = threadIdx.x & (TILE - 1u);
+    uint8_t* W = align128(smraw);
+    uint8_t* X[2];
+    X[0] = W + LAYERS * LAYER_BYTES + group * 2u * X_BYTES;
+    X[1] = X[0] + X_BYTES;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(W + LAYERS * LAYER_BYTES + EVAL_GROUPS * 2u * X_BYTES);
+    uint32_t* slot = reinterpret_cast<uint32_t*>(bars + 2u * EVAL_GROUPS);
+    bars += 2u * group;
     stage_weights(W, A.packed);
-    if (threadIdx.x == 0) mbar_init(bar);
+    if (row == 0) {
+        mbar_init(bars);
+        mbar_init(bars + 1);
+    }
     if (threadIdx.x < 32) tmem_alloc(slot, EVAL_TMEM_COLS);
     fence_before();
     __syncthreads();
     fence_after();
-    TileCtx c{*slot, smem_u32(bar), 0u, false, A.wait_tries};
-    const uint32_t w_addr = smem_u32(W);
-    const uint32_t tiles = (A.n + TILE - 1) / TILE;
-    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const uint32_t idx = tile * TILE + threadIdx.x;
-        Query q{mk(0.0f, 0.0f, 0.0f), mk(0.0f, 1.0f, 0.0f), mk(0.0f, 1.0f, 0.0f)};
-        if (idx < A.n) {
-            const float* r = A.queries + (size_t)idx * 9u;
-            q.pos = mk(r[0], r[1], r[2]);
-            q.n = mk(r[3], r[4], r[5]);
-            q.wo = mk(r[6], r[7], r[8]);
+    const uint32_t tmem = *slot + group * 128u, t_row = tmem + ((row & ~31u) << 16);
+    const uint32_t w_addr = smem_u32(W), bar = smem_u32(bars);
+    uint32_t phase = 0;
+    bool failed = false;
+    const uint32_t pairs = (A.n + 2u * TILE - 1u) / (2u * TILE);
+    for (uint32_t pair = blockIdx.x * EVAL_GROUPS + group; pair < pairs; pair += gridDim.x * EVAL_GROUPS) {
+#pragma unroll
+        for (uint32_t h = 0; h < 2u; ++h) {
+            const uint32_t idx = (2u * pair + h) * TILE + row;
+            Query q{mk(0.0f, 0.0f, 0.0f), mk(0.0f, 1.0f, 0.0f), mk(0.0f, 1.0f, 0.0f)};
+            if (idx < A.n) {
+                const float* r = A.queries + (size_t)idx * 9u;
+                q.pos = mk(r[0], r[1], r[2]);
+                q.n = mk(r[3], r[4], r[5]);
+                q.wo = mk(r[6], r[7], r[8]);
+            }
+            float f[WIDTH];
+            encode_features(q, A.box, f);
+            store_row(X[h], X_RG, row, f);
         }
-        float f[WIDTH];
-        encode_features(q, A.box, f);
-        store_row(X, X_RG, threadIdx.x, f);
-        float raw[OUT];
-        if (!forward_infer(c, X, w_addr, raw)) break;
-        if (idx < A.n)
-            for (int k = 0; k < OUT; ++k) A.out[(size_t)idx * OUT + k] = raw[k];
+        bool ok = true;
+        for (uint32_t l = 0; l < (uint32_t)LAYERS; ++l) {
+            fence_async_smem();
+            fence_before();
+            if (group_or(group, failed)) {
+                failed = true;
+                ok = false;
+                break;
+            }
+            if (row == 0) {
+                fence_after();
+                for (uint32_t h = 0; h < 2u; ++h) {
+                    issue_fwd(tmem + 64u * h, smem_u32(X[h]), w_addr + l * LAYER_BYTES);
+                    mma_commit(bar + 8u * h);
+                }
+            }
+#pragma unroll
+            for (uint32_t h = 0; h < 2u; ++h) {
+                if (!mbar_wait(bar + 8u * h, phase, A.wait_tries)) failed = true;
+                fence_after();
+                if (l < 3u) epilogue_relu(t_row + 64u * h, X[h], row);
+            }
+            phase ^= 1u;
+        }
+        if (!ok) break;
+#pragma unroll
+        for (uint32_t h = 0; h < 2u; ++h) {
+            const uint32_t idx = (2u * pair + h) * TILE + row;
+            float raw[OUT];
+            head_read(t_row + 64u * h, raw);
+            if (idx < A.n) {  // rows of 160 bytes; the caller's buffer may be aligned to 4 only
+                float* out = A.out + (size_t)idx * OUT;
+                if (A.out_aligned) {
+#pragma unroll
+                    for (int k = 0; k < OUT / 4; ++k)
+                        reinterpret_cast<float4*>(out)[k] = make_float4(raw[4 * k], raw[4 * k + 1], raw[4 * k + 2], raw[4 * k + 3]);
+                } else {
+                    for (int k = 0; k < OUT; ++k) out[k] = raw[k];
+                }
+            }
+        }
     }
-    if (c.failed) mbar_wait(c.bar, c.phase ^ 1u, DRAIN_TRIES);  // let an MMA in flight finish before TMEM is freed
+    if (failed) {  // let MMAs in flight finish before TMEM is freed
+        mbar_wait(bar, phase ^ 1u, DRAIN_TRIES);
+        mbar_wait(bar + 8u, phase ^ 1u, DRAIN_TRIES);
+    }
     fence_before();
-    c.failed = __syncthreads_or(c.failed ? 1 : 0) != 0;
-    if (c.failed && threadIdx.x == 0) atomicOr(A.err, ERR_MMA_TIMEOUT);
+    failed = __syncthreads_or(failed ? 1 : 0) != 0;
+    if (failed && threadIdx.x == 0) atomicOr(A.err, ERR_MMA_TIMEOUT);
     if (threadIdx.x < 32) {
         fence_after();
-        tmem_free(c.tmem, EVAL_TMEM_COLS);
+        tmem_free(*slot, EVAL_TMEM_COLS);
     }
 }
 
@@ -115,139 +171,61 @@ struct GradArgs {
     uint32_t wait_tries;    // polls of each completion wait before it gives up
 };
 
-__global__ void __launch_bounds__(128, 1) guide_grad_kernel(GradArgs A) {
-    extern __shared__ uint8_t smraw[];
-    uint8_t* sm = align128(smraw);
-    uint8_t* W = sm;
-    uint8_t* Xs[4];
-    for (int l = 0; l < 4; ++l) Xs[l] = sm + LAYERS * LAYER_BYTES + l * X_BYTES;
-    uint8_t* G = sm + LAYERS * LAYER_BYTES + 4 * X_BYTES;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(G + G_BYTES);
-    uint32_t* slot = reinterpret_cast<uint32_t*>(G + G_BYTES + 8);
-    float* sloss = reinterpret_cast<float*>(G + G_BYTES + 12);
-    stage_weights(W, A.packed);
-    {
-        uint4* g4 = reinterpret_cast<uint4*>(G);
-        for (uint32_t i = threadIdx.x; i < G_BYTES / 16u; i += blockDim.x) g4[i] = make_uint4(0u, 0u, 0u, 0u);
+// The gradient kernels run two threads per row of a tile, one per half of its 64 columns (warps w and
+// w + 4 reach the same TMEM lanes): with one CTA per SM, encoding, epilogues and stores are chains of
+// scalar work with one warp per scheduler to hide them.  The head, whose lobes share their sums, is the
+// first half's.
+constexpr uint32_t GRAD_THREADS = 2u * TILE;
+LAM_DEV uint32_t grad_row() { return threadIdx.x & (TILE - 1u); }
+LAM_DEV uint32_t grad_half() { return threadIdx.x / TILE; }
+
+// A CTA's shared memory of the gradient kernels: weights, the inputs of the four layers, the gradient tile.
+struct GradSmem {
+    uint8_t *W, *X, *G;
+    uint64_t* bar;   // [0]: the round that the next epilogue reads; [1]: weight gradients
+    uint32_t* slot;
+    float* loss;
+    float* terms;    // LOBES log terms per row
+    LAM_DEV explicit GradSmem(uint8_t* raw) {
+        W = align128(raw);
+        X = W + LAYERS * LAYER_BYTES;
+        G = X + 4 * X_BYTES;
+        bar = reinterpret_cast<uint64_t*>(G + G_BYTES);
+        slot = reinterpret_cast<uint32_t*>(G + G_BYTES + 16);
+        loss = reinterpret_cast<float*>(G + G_BYTES + 20);
+        terms = reinterpret_cast<float*>(G + G_BYTES + 64);
     }
+    LAM_DEV uint8_t* x(uint32_t l) const { return X + l * X_BYTES; }
+};
+
+struct GradCtx : TileCtx {
+    uint32_t dw_phase;  // of the weight gradients' barrier
+};
+// MMAs still in flight after a wait gave up finish before TMEM is read or freed.
+LAM_DEV void grad_drain(const GradCtx& c) {
+    mbar_wait(c.bar, c.phase ^ 1u, DRAIN_TRIES);
+    mbar_wait(c.bar + 8u, c.dw_phase ^ 1u, DRAIN_TRIES);
+}
+
+// Clears the gradient tile (its columns 64..127 stay zero), the barrier and the loss; allocates TMEM.
+LAM_DEV GradCtx grad_begin(const GradSmem& S, uint32_t wait_tries) {
+    uint4* g4 = reinterpret_cast<uint4*>(S.G);
+    for (uint32_t i = threadIdx.x; i < G_BYTES / 16u; i += blockDim.x) g4[i] = make_uint4(0u, 0u, 0u, 0u);
     if (threadIdx.x == 0) {
-        mbar_init(bar);
-        *sloss = 0.0f;
+        mbar_init(S.bar);
+        mbar_init(S.bar + 1);
+        *S.loss = 0.0f;
     }
-    if (threadIdx.x < 32) tmem_alloc(slot, GRAD_TMEM_COLS);
+    if (threadIdx.x < 32) tmem_alloc(S.slot, GRAD_TMEM_COLS);
     fence_before();
     __syncthreads();
     fence_after();
-    TileCtx c{*slot, smem_u32(bar), 0u, false, A.wait_tries};
-    const uint32_t row = threadIdx.x;
-    const uint32_t t_row = c.tmem + ((threadIdx.x & ~31u) << 16);
-    const uint32_t w_addr = smem_u32(W), g_addr = smem_u32(G);
-    uint32_t n = A.n;
-    if (A.n_dev) n = min(n, *A.n_dev);
-    const uint32_t tiles = A.batch / TILE;
-    bool any = false, stop = false;  // both uniform across the CTA
-    float loss = 0.0f;
-    for (uint32_t tile = blockIdx.x; tile < tiles && !stop; tile += gridDim.x) {
-        const uint32_t b = tile * TILE + row;
-        bool valid;
-        uint32_t idx;
-        if (A.sequential) {
-            valid = b < n;
-            idx = b;
-        } else {
-            valid = n > 0u;
-            idx = valid ? rand_u32(A.seed ^ rand_u32(A.step * 0x9E3779B9u + b)) % n : 0u;
-        }
-        Query q{mk(0.0f, 0.0f, 0.0f), mk(0.0f, 1.0f, 0.0f), mk(0.0f, 1.0f, 0.0f)};
-        v3 wi = mk(0.0f, 1.0f, 0.0f);
-        float weight = 0.0f;
-        if (valid) {
-            const float* r = A.recs + (size_t)idx * A.stride;
-            q.pos = mk(r[0], r[1], r[2]);
-            q.n = mk(r[3], r[4], r[5]);
-            q.wo = mk(r[6], r[7], r[8]);
-            wi = mk(r[9], r[10], r[11]);
-            weight = r[12];
-            if (!(weight >= 0.0f) || !(weight < 3.0e38f)) weight = 0.0f;
-        }
-        float f[WIDTH];
-        encode_features(q, A.box, f);
-        store_row(Xs[0], X_RG, row, f);
-        // forward, keeping every layer's input for the backward pass
-        bool ok = true;
-        for (uint32_t l = 0; l < 4u && ok; ++l) {
-            ok = mma_round(c, [&] { issue_fwd(c.tmem, smem_u32(Xs[l]), w_addr + l * LAYER_BYTES); });
-            if (!ok) {
-                stop = true;
-                break;
-            }
-            if (l < 3u) {
-                epilogue_relu(t_row, Xs[l + 1], row);
-            } else {
-                float raw[OUT], g[WIDTH];
-                head_read(t_row, raw);
-                loss += head_grad(raw, wi, weight, A.scale, g);
-                for (int k = OUT; k < WIDTH; ++k) g[k] = 0.0f;
-                store_row(G, G_RG, row, g);
-            }
-        }
-        // backward: dW[l] += G^T X[l]; G <- (G W[l]) * relu'(X[l])
-        for (int l = 3; l >= 0 && ok; --l) {
-            const bool acc_dw = any;
-            ok = mma_round(c, [&] {
-                issue_dw(c.tmem + 64u * (uint32_t)(l + 1), g_addr, smem_u32(Xs[l]), acc_dw);
-                if (l > 0) issue_dx(c.tmem, g_addr, w_addr + (uint32_t)l * LAYER_BYTES);
-            });
-            if (!ok) {
-                stop = true;
-                break;
-            }
-            if (l > 0) {
-                float v[64];
-                tmem_ld64(t_row, v);
-#pragma unroll
-                for (uint32_t ch = 0; ch < 8; ++ch) {
-                    const uint4 x = load_chunk(Xs[l], X_RG, row, ch);
-                    const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        if (!(bf16_lo(xw[k]) > 0.0f)) v[8 * ch + 2 * k] = 0.0f;
-                        if (!(bf16_hi(xw[k]) > 0.0f)) v[8 * ch + 2 * k + 1] = 0.0f;
-                    }
-                }
-                v[63] = 0.0f;
-#pragma unroll
-                for (uint32_t ch = 0; ch < 8; ++ch) store_chunk(G, G_RG, row, ch, v + 8 * ch);
-            }
-        }
-        any = true;
-    }
-    // loss: warp sums, then one shared-memory add per warp
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) loss += __shfl_down_sync(0xFFFFFFFFu, loss, o);
-    if ((threadIdx.x & 31u) == 0u) atomicAdd(sloss, loss);
-    if (c.failed) mbar_wait(c.bar, c.phase ^ 1u, DRAIN_TRIES);  // an MMA in flight finishes before TMEM is read or freed
-    fence_before();
-    c.failed = __syncthreads_or(c.failed ? 1 : 0) != 0;
-    fence_after();
-    // weight-gradient partials: rows 0..63 of each dW accumulator live in the lanes of warps 0 and 1
-    float* part = A.partial + (size_t)blockIdx.x * PARAMS;
-    if (threadIdx.x < 64) {
-        const uint32_t o = threadIdx.x;
-        for (uint32_t l = 0; l < 4u; ++l) {
-            float v[64];
-            tmem_ld64(t_row + 64u * (l + 1u), v);
-            const bool use = any && !c.failed && trainable(l, o);
-            float4* dst = reinterpret_cast<float4*>(part + l * 4096u + o * 64u);
-#pragma unroll
-            for (int k = 0; k < 16; ++k)
-                dst[k] = use ? make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-    }
-    if (threadIdx.x == 0) {
-        A.partial_loss[blockIdx.x] = *sloss;
-        if (c.failed) atomicOr(A.err, ERR_MMA_TIMEOUT);
-    }
+    return GradCtx{{*S.slot, smem_u32(S.bar), 0u, false, wait_tries}, 0u};
+}
+
+// Frees TMEM once the CTA's MMAs have finished; reports a wait that gave up.
+LAM_DEV void grad_end(const GradCtx& c, uint32_t* err) {
+    if (threadIdx.x == 0 && c.failed) atomicOr(err, ERR_MMA_TIMEOUT);
     fence_before();
     __syncthreads();
     if (threadIdx.x < 32) {
@@ -256,45 +234,346 @@ __global__ void __launch_bounds__(128, 1) guide_grad_kernel(GradArgs A) {
     }
 }
 
+struct GradRecord {
+    Query q;
+    v3 wi;
+    float weight;
+};
+// The record of this thread's row of a tile.
+LAM_DEV GradRecord grad_record(const GradArgs& A, uint32_t n, uint32_t step, uint32_t tile) {
+    const uint32_t b = tile * TILE + grad_row();
+    bool valid;
+    uint32_t idx;
+    if (A.sequential) {
+        valid = b < n;
+        idx = b;
+    } else {
+        valid = n > 0u;
+        idx = valid ? rand_u32(A.seed ^ rand_u32(step * 0x9E3779B9u + b)) % n : 0u;
+    }
+    GradRecord R{{mk(0.0f, 0.0f, 0.0f), mk(0.0f, 1.0f, 0.0f), mk(0.0f, 1.0f, 0.0f)}, mk(0.0f, 1.0f, 0.0f), 0.0f};
+    if (valid) {
+        const float* r = A.recs + (size_t)idx * A.stride;
+        R.q.pos = mk(r[0], r[1], r[2]);
+        R.q.n = mk(r[3], r[4], r[5]);
+        R.q.wo = mk(r[6], r[7], r[8]);
+        R.wi = mk(r[9], r[10], r[11]);
+        R.weight = r[12];
+        if (!(R.weight >= 0.0f) || !(R.weight < 3.0e38f)) R.weight = 0.0f;
+    }
+    return R;
+}
+LAM_DEV void grad_encode(const GradSmem& S, const GradRecord& R, const float* box) {
+    float f[WIDTH];
+    // each half computes only the features that it stores
+    if (grad_half() == 0u) {
+        encode_features(R.q, box, f);
+#pragma unroll
+        for (uint32_t c = 0; c < 4; ++c) store_chunk(S.x(0), X_RG, grad_row(), c, f + 8 * c);
+    } else {
+        encode_features(R.q, box, f);
+#pragma unroll
+        for (uint32_t c = 4; c < 8; ++c) store_chunk(S.x(0), X_RG, grad_row(), c, f + 8 * c);
+    }
+}
+
+// Forward and backward pass of a tile whose features are in x(0); the weight gradients are added to
+// (`add`) or start the TMEM accumulators.  False once a wait has given up.
+LAM_DEV bool grad_tile(GradCtx& c, const GradSmem& S, const GradRecord& R, float scale, bool add, float& loss) {
+    const uint32_t row = grad_row(), half = grad_half();
+    const uint32_t t_row = c.tmem + ((row & ~31u) << 16);
+    const uint32_t w_addr = smem_u32(S.W), g_addr = smem_u32(S.G);
+    // forward, keeping every layer's input for the backward pass
+    for (uint32_t l = 0; l < 4u; ++l) {
+        if (!mma_round(c, [&] { issue_fwd(c.tmem, smem_u32(S.x(l)), w_addr + l * LAYER_BYTES); })) return false;
+        if (l < 3u) {
+            float v[32];
+            tmem_ld32(t_row + 32u * half, v);
+#pragma unroll
+            for (int k = 0; k < 32; ++k) v[k] = fmaxf(v[k], 0.0f);
+            if (half) v[31] = 1.0f;  // column 63
+#pragma unroll
+            for (uint32_t ch = 0; ch < 4; ++ch) store_chunk(S.x(l + 1), X_RG, row, 4u * half + ch, v + 8 * ch);
+        } else {
+            float raw[OUT], g[OUT / 2];
+            head_read(t_row, raw);
+            float* terms = S.terms + row * LOBES;
+            if (half == 0u) loss += head_grad<0>(raw, R.wi, R.weight, scale, terms, g);
+            else head_grad<1>(raw, R.wi, R.weight, scale, terms, g);
+#pragma unroll
+            for (uint32_t k = 0; k < 8u; ++k)  // outputs 40..63 have no gradient
+                *reinterpret_cast<uint2*>(S.G + core_off(row, 8u * k + 4u * half, G_RG)) =
+                    k < 5u ? make_uint2(pack_bf16(g[4 * k], g[4 * k + 1]), pack_bf16(g[4 * k + 2], g[4 * k + 3]))
+                           : make_uint2(0u, 0u);
+        }
+    }
+    // backward: dW[l] += G^T X[l]; G <- (G W[l]) * relu'(X[l])
+    // The input gradients are issued first, with a barrier of their own: their epilogue runs under the
+    // weight gradients' MMAs, up to the store into G, which those read.
+    for (int l = 3; l >= 0; --l) {
+        fence_async_smem();
+        fence_before();
+        if (__syncthreads_or(c.failed ? 1 : 0)) {
+            c.failed = true;
+            return false;
+        }
+        if (threadIdx.x == 0) {
+            fence_after();
+            if (l > 0) {
+                issue_dx(c.tmem, g_addr, w_addr + (uint32_t)l * LAYER_BYTES);
+                mma_commit(c.bar);
+            }
+            issue_dw(c.tmem + 64u * (uint32_t)(l + 1), g_addr, smem_u32(S.x(l)), add);
+            mma_commit(c.bar + 8u);
+        }
+        float v[32];
+        if (l > 0) {
+            if (!mbar_wait(c.bar, c.phase, c.tries)) c.failed = true;
+            c.phase ^= 1u;
+            fence_after();
+            tmem_ld32(t_row + 32u * half, v);
+#pragma unroll
+            for (uint32_t ch = 0; ch < 4; ++ch) {
+                const uint4 x = load_chunk(S.x(l), X_RG, row, 4u * half + ch);
+                const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (!(bf16_lo(xw[k]) > 0.0f)) v[8 * ch + 2 * k] = 0.0f;
+                    if (!(bf16_hi(xw[k]) > 0.0f)) v[8 * ch + 2 * k + 1] = 0.0f;
+                }
+            }
+            if (half) v[31] = 0.0f;  // column 63
+        }
+        if (!mbar_wait(c.bar + 8u, c.dw_phase, c.tries)) c.failed = true;
+        c.dw_phase ^= 1u;
+        fence_after();
+        if (l > 0) {
+#pragma unroll
+            for (uint32_t ch = 0; ch < 4; ++ch) store_chunk(S.G, G_RG, row, 4u * half + ch, v + 8 * ch);
+        }
+    }
+    return true;
+}
+
+// The CTA's weight-gradient partials: rows 0..63 of each dW accumulator live in the lanes of the first
+// two warps of each half.  Partials are stored as 16-byte pieces, [layer][piece of the row][row], so that
+// a warp's stores are contiguous (row by row each of them touched 32 lines: 2.2 us of a step).
+LAM_DEV void grad_write(const GradCtx& c, float* part, bool any) {
+    if (grad_row() < 64u) {
+        const uint32_t o = grad_row(), half = grad_half(), t_row = c.tmem + ((o & ~31u) << 16) + 32u * half;
+        for (uint32_t l = 0; l < 4u; ++l) {
+            float v[32];
+            tmem_ld32(t_row + 64u * (l + 1u), v);
+            const bool use = any && !c.failed && trainable(l, o);
+            float4* dst = reinterpret_cast<float4*>(part) + l * 1024u + 8u * half * 64u + o;
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                dst[64 * k] = use ? make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+}
+// The parameter W[l][o][i] at place q of a partial.
+LAM_DEV uint32_t partial_param(uint32_t q) {
+    const uint32_t l = q / 4096u, piece = (q / 256u) % 16u, o = (q / 4u) % 64u;
+    return l * 4096u + o * 64u + 4u * piece + (q & 3u);
+}
+
+__global__ void __launch_bounds__(GRAD_THREADS, 1) guide_grad_kernel(const __grid_constant__ GradArgs A) {
+    extern __shared__ uint8_t smraw[];
+    const GradSmem S(smraw);
+    stage_weights(S.W, A.packed);
+    GradCtx c = grad_begin(S, A.wait_tries);
+    uint32_t n = A.n;
+    if (A.n_dev) n = min(n, *A.n_dev);
+    const uint32_t tiles = A.batch / TILE;
+    bool any = false;  // uniform across the CTA
+    float loss = 0.0f;
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const GradRecord R = grad_record(A, n, A.step, tile);
+        grad_encode(S, R, A.box);
+        if (!grad_tile(c, S, R, A.scale, any, loss)) break;
+        any = true;
+    }
+    // loss: warp sums, then one shared-memory add per warp
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) loss += __shfl_down_sync(0xFFFFFFFFu, loss, o);
+    if ((threadIdx.x & 31u) == 0u) atomicAdd(S.loss, loss);
+    if (c.failed) grad_drain(c);
+    fence_before();
+    c.failed = __syncthreads_or(c.failed ? 1 : 0) != 0;
+    fence_after();
+    grad_write(c, A.partial + (size_t)blockIdx.x * PARAMS, any);
+    if (threadIdx.x == 0) A.partial_loss[blockIdx.x] = *S.loss;
+    grad_end(c, A.err);
+}
+
 struct UpdateArgs {
     const float* partial;
     const float* partial_loss;
     uint32_t parts;
-    uint32_t mode;  // 0: write grad/loss, 1: Adam step
     float* grad;
     float* loss;
     float* master;
     float* m;
     float* v;
     uint16_t* packed;
-    float lr_t, b1, b2, eps;
+    float b1, b2, eps;
 };
 
-__global__ void guide_update_kernel(UpdateArgs A) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p == 0 && A.loss) {
+// The sum of the partials' place q, in order; the loads of N are in flight together.  (L2 loads: the
+// training kernel reads partials that other SMs wrote while it runs.)
+template <uint32_t N>
+LAM_DEV float partial_sum(const float* partial, uint32_t parts, uint32_t q) {
+    float g = 0.0f;
+    uint32_t c = 0;
+    for (; c < parts; c += N) {
+        float v[N];
+#pragma unroll
+        for (uint32_t k = 0; k < N; ++k) v[k] = c + k < parts ? __ldcg(partial + (size_t)(c + k) * PARAMS + q) : 0.0f;
+#pragma unroll
+        for (uint32_t k = 0; k < N; ++k)
+            if (c + k < parts) g += v[k];
+    }
+    return g;
+}
+
+// A parameter with its Adam state.
+struct AdamState {
+    float w, m, v;
+};
+LAM_DEV AdamState adam_load(const UpdateArgs& A, uint32_t p) { return AdamState{A.master[p], A.m[p], A.v[p]}; }
+LAM_DEV void adam_step(const UpdateArgs& A, uint32_t p, AdamState x, float g, float lr_t) {
+    const uint32_t l = p / 4096u, o = (p / 64u) % 64u, i = p % 64u;
+    if (!trainable(l, o)) return;
+    // the contractions are spelled out: left to the compiler they depend on the code around them
+    const float m = __fmaf_rn(1.0f - A.b1, g, __fmul_rn(A.b1, x.m));
+    const float v = __fmaf_rn(__fmul_rn(1.0f - A.b2, g), g, __fmul_rn(A.b2, x.v));
+    A.m[p] = m;
+    A.v[p] = v;
+    const float w = x.w - lr_t * m / (sqrtf(v) + A.eps);
+    A.master[p] = w;
+    __nv_bfloat16 b = __float2bfloat16_rn(w);
+    A.packed[packed_index(l, o, i)] = *reinterpret_cast<uint16_t*>(&b);
+}
+
+// Loss and gradient of a lam_guide_loss_grad: the partials summed in order.
+__global__ void guide_sum_kernel(UpdateArgs A) {
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q == 0) {
         float s = 0.0f;
         for (uint32_t c = 0; c < A.parts; ++c) s += A.partial_loss[c];
         *A.loss = s;
     }
-    if (p >= (uint32_t)PARAMS) return;
-    float g = 0.0f;
-    for (uint32_t c = 0; c < A.parts; ++c) g += A.partial[(size_t)c * PARAMS + p];
-    const uint32_t l = p / 4096u, o = (p / 64u) % 64u, i = p % 64u;
-    if (!trainable(l, o)) g = 0.0f;
-    if (A.mode == 0u) {
-        A.grad[p] = g;
-        return;
+    if (q >= (uint32_t)PARAMS) return;
+    const uint32_t p = partial_param(q), l = p / 4096u, o = (p / 64u) % 64u;
+    const float g = partial_sum<16>(A.partial, A.parts, q);
+    A.grad[p] = trainable(l, o) ? g : 0.0f;
+}
+
+// All CTAs of the (cooperatively launched) grid meet: the k-th call waits for (k + 1) * gridDim arrivals.
+// Bounded: false, on every thread of the CTA, once the wait has given up.
+constexpr uint32_t GRID_TRIES = 1u << 22;
+LAM_DEV void grid_arrive(uint32_t* count) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(count, 1u);
     }
-    if (!trainable(l, o)) return;
-    const float m = A.b1 * A.m[p] + (1.0f - A.b1) * g;
-    const float v = A.b2 * A.v[p] + (1.0f - A.b2) * g * g;
-    A.m[p] = m;
-    A.v[p] = v;
-    const float w = A.master[p] - A.lr_t * m / (sqrtf(v) + A.eps);
-    A.master[p] = w;
-    __nv_bfloat16 b = __float2bfloat16_rn(w);
-    A.packed[packed_index(l, o, i)] = *reinterpret_cast<uint16_t*>(&b);
+}
+LAM_DEV bool grid_wait(const uint32_t* count, uint32_t k) {
+    uint32_t ok = 1u;
+    if (threadIdx.x == 0) {
+        const uint32_t target = (k + 1u) * gridDim.x;
+        ok = 0u;
+        for (uint32_t t = 0; t < GRID_TRIES && !ok; ++t) {
+            uint32_t v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+            ok = v >= target;
+        }
+        __threadfence();
+    }
+    return __syncthreads_and(ok != 0u) != 0;
+}
+
+// Adam steps A.step .. A.step + steps - 1 in one launch.  Per step a CTA runs its tiles and writes its
+// partials; the grid meets; the parameters, spread over all threads, are summed in the partials' order
+// (deterministic) and updated; the grid meets again.  Kept between steps: TMEM, the cleared gradient
+// tile and the launch; the next step's first records are fetched and encoded while the other CTAs finish
+// their partials.  A step of 16,384 records: 18.8 us; as two launches per step,
+// 22.5 us of gradients, 5.7 of update and 5 of gaps.  What is left is a chain: weights 2 us, eight MMA rounds
+// with their epilogues 7, the head 2.7, partials 1.2, two meetings and the sums 6.
+constexpr uint32_t TRAIN_STEPS = 64;  // most steps of a launch
+struct TrainArgs {
+    GradArgs g;
+    UpdateArgs u;
+    uint32_t steps;
+    uint32_t* count;  // arrivals, zero at launch
+    float lr[TRAIN_STEPS];
+};
+__global__ void __launch_bounds__(GRAD_THREADS, 1) guide_train_kernel(const __grid_constant__ TrainArgs T) {
+    extern __shared__ uint8_t smraw[];
+    const GradSmem S(smraw);
+    const GradArgs& A = T.g;
+    GradCtx c = grad_begin(S, A.wait_tries);
+    uint32_t n = A.n;
+    if (A.n_dev) n = min(n, *A.n_dev);
+    const uint32_t tiles = A.batch / TILE;
+    GradRecord R = grad_record(A, n, A.step, blockIdx.x);
+    grad_encode(S, R, A.box);
+    for (uint32_t s = 0; s < T.steps; ++s) {
+        {
+            const uint4* src = reinterpret_cast<const uint4*>(A.packed);
+            uint4* dst = reinterpret_cast<uint4*>(S.W);
+#pragma unroll
+            for (uint32_t k = 0; k < (uint32_t)(LAYERS * LAYER_BYTES / 16) / GRAD_THREADS; ++k)
+                dst[k * GRAD_THREADS + threadIdx.x] = __ldcg(src + k * GRAD_THREADS + threadIdx.x);
+        }
+        float loss = 0.0f;
+        bool any = false;
+        for (uint32_t tile = blockIdx.x; tile < tiles && !c.failed; tile += gridDim.x) {
+            if (any) {
+                R = grad_record(A, n, A.step + s, tile);
+                grad_encode(S, R, A.box);
+            }
+            if (!grad_tile(c, S, R, A.scale, any, loss)) break;
+            any = true;
+        }
+        if (c.failed) grad_drain(c);
+        fence_before();
+        c.failed = __syncthreads_or(c.failed ? 1 : 0) != 0;
+        fence_after();
+        grad_write(c, A.partial + (size_t)blockIdx.x * PARAMS, any);
+        fence_before();
+        // a CTA whose waits gave up keeps meeting the others, with partials of zero
+        grid_arrive(T.count);
+        const bool more = s + 1u < T.steps;
+        // under the others' tails: the next step's records, and the state of this thread's first parameter
+        if (more && !c.failed) {
+            R = grad_record(A, n, A.step + s + 1u, blockIdx.x);
+            grad_encode(S, R, A.box);
+        }
+        const uint32_t q0 = blockIdx.x * TILE + threadIdx.x;
+        const bool mine = threadIdx.x < TILE && q0 < (uint32_t)PARAMS;
+        AdamState x{0.0f, 0.0f, 0.0f};
+        if (mine) x = adam_load(T.u, partial_param(q0));
+        if (!grid_wait(T.count, 2u * s)) {
+            c.failed = true;
+            break;
+        }
+        // 128 parameters per CTA at the grid of a 16,384-record batch
+        for (uint32_t q = q0; threadIdx.x < TILE && q < (uint32_t)PARAMS; q += gridDim.x * TILE) {
+            const uint32_t p = partial_param(q);
+            const float g = partial_sum<64>(A.partial, gridDim.x, q);
+            adam_step(T.u, p, q == q0 ? x : adam_load(T.u, p), g, T.lr[s]);
+        }
+        if (!more) break;
+        grid_arrive(T.count);
+        if (!grid_wait(T.count, 2u * s + 1u)) {
+            c.failed = true;
+            break;
+        }
+    }
+    grad_end(c, A.err);
 }
 
 }  // namespace net
@@ -343,9 +622,16 @@ static int upload_params(lam_guide* g, const float* host) {
     return LAM_OK;
 }
 
+// CTAs of the gradient kernels: one per tile, at most one per SM.
+static uint32_t grad_grid(const lam_guide* g, uint32_t batch) {
+    return std::max(1u, std::min<uint32_t>(batch / net::TILE, g->parts));
+}
+
 static int setup_kernels(lam_guide* g) {
     if (g->kernels_ready) return LAM_OK;
     cudaError_t e = cudaFuncSetAttribute(net::guide_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, net::GRAD_SMEM);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(net::guide_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, net::GRAD_SMEM);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(net::guide_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, net::EVAL_SMEM);
     if (e != cudaSuccess) return cuda_error(e, "guide kernel attributes");
@@ -353,15 +639,8 @@ static int setup_kernels(lam_guide* g) {
     return LAM_OK;
 }
 
-// Gradient partials of `batch` rows (one launch) and their reduction (mode 0: grad/loss, 1: Adam).
-int guide_grad_and_update(lam_guide* g, const float* recs, uint32_t stride, uint32_t n, const uint32_t* n_dev,
-                          uint32_t batch, bool sequential, float scale, const float box[6], uint32_t mode, float* grad,
-                          float* loss, cudaStream_t st) {
-    int rc = setup_kernels(g);
-    if (rc) return rc;
-    const uint32_t tiles = batch / net::TILE;
-    const uint32_t grid = std::max(1u, std::min<uint32_t>(tiles, g->parts));
-    net::GradArgs A;
+static void fill_args(lam_guide* g, const float* recs, uint32_t stride, uint32_t n, const uint32_t* n_dev, uint32_t batch,
+                      bool sequential, float scale, const float box[6], net::GradArgs& A, net::UpdateArgs& U) {
     A.recs = recs;
     A.stride = stride;
     A.n = n;
@@ -377,14 +656,10 @@ int guide_grad_and_update(lam_guide* g, const float* recs, uint32_t stride, uint
     A.partial_loss = g->partial_loss;
     A.err = g->err;
     A.wait_tries = g->wait_tries;
-    net::guide_grad_kernel<<<grid, 128, net::GRAD_SMEM, st>>>(A);
-    net::UpdateArgs U;
     U.partial = g->partial;
     U.partial_loss = g->partial_loss;
-    U.parts = grid;
-    U.mode = mode;
-    U.grad = grad;
-    U.loss = loss;
+    U.parts = grad_grid(g, batch);
+    U.grad = U.loss = nullptr;
     U.master = g->master;
     U.m = g->adam_m;
     U.v = g->adam_v;
@@ -392,16 +667,50 @@ int guide_grad_and_update(lam_guide* g, const float* recs, uint32_t stride, uint
     U.b1 = 0.9f;
     U.b2 = 0.99f;
     U.eps = 1e-8f;
-    U.lr_t = 0.0f;
-    if (mode == 1u) {
-        g->steps++;
-        const double t = (double)g->steps;
-        U.lr_t = (float)(g->opts.learning_rate * std::sqrt(1.0 - std::pow((double)U.b2, t)) /
-                         (1.0 - std::pow((double)U.b1, t)));
-    }
-    net::guide_update_kernel<<<net::PARAMS / 256, 256, 0, st>>>(U);
+}
+
+// Loss and gradient over n records (two launches).
+static int guide_loss_grad(lam_guide* g, const float* recs, uint32_t n, const float box[6], float* grad, float* loss,
+                           cudaStream_t st) {
+    int rc = setup_kernels(g);
+    if (rc) return rc;
+    const uint32_t batch = (n + net::TILE - 1) / net::TILE * net::TILE;
+    net::GradArgs A;
+    net::UpdateArgs U;
+    fill_args(g, recs, 13u, n, nullptr, batch, true, 1.0f / (float)n, box, A, U);
+    U.grad = grad;
+    U.loss = loss;
+    net::guide_grad_kernel<<<U.parts, net::GRAD_THREADS, net::GRAD_SMEM, st>>>(A);
+    net::guide_sum_kernel<<<net::PARAMS / 256, 256, 0, st>>>(U);
     cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_error(e, "guide training launch");
+    if (e != cudaSuccess) return cuda_error(e, "guide gradient launch");
+    return LAM_OK;
+}
+
+// `steps` Adam steps on minibatches of options.batch records drawn from n (or *n_dev, if fewer).
+int guide_train(lam_guide* g, const float* recs, uint32_t stride, uint32_t n, const uint32_t* n_dev, uint32_t steps,
+                const float box[6], cudaStream_t st) {
+    int rc = setup_kernels(g);
+    if (rc) return rc;
+    net::TrainArgs T;
+    T.count = g->err + 8;
+    while (steps) {
+        T.steps = std::min(steps, net::TRAIN_STEPS);
+        fill_args(g, recs, stride, n, n_dev, g->opts.batch, false, 1.0f / (float)g->opts.batch, box, T.g, T.u);
+        for (uint32_t k = 0; k < T.steps; ++k) {
+            const double t = (double)(g->steps + k + 1);
+            T.lr[k] = (float)(g->opts.learning_rate * std::sqrt(1.0 - std::pow((double)T.u.b2, t)) /
+                              (1.0 - std::pow((double)T.u.b1, t)));
+        }
+        cudaError_t e = cudaMemsetAsync(T.count, 0, sizeof(uint32_t), st);
+        if (e != cudaSuccess) return cuda_error(e, "guide training");
+        void* args[] = {&T};
+        // cooperative: the CTAs wait for one another (at most one per SM)
+        e = cudaLaunchCooperativeKernel((const void*)net::guide_train_kernel, dim3(T.u.parts), dim3(net::GRAD_THREADS), args, net::GRAD_SMEM, st);
+        if (e != cudaSuccess) return cuda_error(e, "guide training launch");
+        g->steps += T.steps;
+        steps -= T.steps;
+    }
     return LAM_OK;
 }
 
@@ -418,9 +727,10 @@ int guide_eval_launch(const lam_guide* g, const float* queries, uint32_t n, cons
     A.out = out;
     A.err = g->err;
     A.wait_tries = g->wait_tries;
-    const uint32_t tiles = (n + net::TILE - 1) / net::TILE;
-    const uint32_t grid = std::max(1u, std::min<uint32_t>(tiles, (uint32_t)g->sms * 4u));
-    net::guide_eval_kernel<<<grid, 128, net::EVAL_SMEM, st>>>(A);
+    A.out_aligned = ((uintptr_t)out & 15u) == 0u ? 1u : 0u;
+    const uint32_t per_cta = 2u * net::TILE * net::EVAL_GROUPS;
+    const uint32_t grid = std::min<uint32_t>((n + per_cta - 1u) / per_cta, (uint32_t)g->sms * 2u);
+    net::guide_eval_kernel<<<grid, net::EVAL_THREADS, net::EVAL_SMEM, st>>>(A);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(e, "lam_guide_eval launch");
     return LAM_OK;
@@ -525,20 +835,14 @@ extern "C" int lam_guide_loss_grad(lam_guide* g, const lam_guide_record* records
                                    float* grad, float* loss, void* stream) {
     if (!g || !box || !grad || !loss || (n && !records)) return set_error(LAM_ERR_INVALID_ARGUMENT, "lam_guide_loss_grad: null argument");
     if (n == 0) return set_error(LAM_ERR_INVALID_ARGUMENT, "lam_guide_loss_grad: no records");
-    const uint32_t batch = (n + net::TILE - 1) / net::TILE * net::TILE;
-    return guide_grad_and_update(g, reinterpret_cast<const float*>(records), 13u, n, nullptr, batch, true, 1.0f / (float)n,
-                                 box, 0u, grad, loss, (cudaStream_t)stream);
+    return guide_loss_grad(g, reinterpret_cast<const float*>(records), n, box, grad, loss, (cudaStream_t)stream);
 }
 
 extern "C" int lam_guide_train(lam_guide* g, const lam_guide_record* records, uint32_t n, uint32_t steps,
                                const float box[6], void* stream) {
     if (!g || !box || (n && !records)) return set_error(LAM_ERR_INVALID_ARGUMENT, "lam_guide_train: null argument");
-    for (uint32_t s = 0; s < steps && n; ++s) {
-        int rc = guide_grad_and_update(g, reinterpret_cast<const float*>(records), 13u, n, nullptr, g->opts.batch, false,
-                                       1.0f / (float)g->opts.batch, box, 1u, nullptr, nullptr, (cudaStream_t)stream);
-        if (rc) return rc;
-    }
-    return LAM_OK;
+    if (!n) return LAM_OK;
+    return guide_train(g, reinterpret_cast<const float*>(records), 13u, n, nullptr, steps, box, (cudaStream_t)stream);
 }
 
 extern "C" int lam_guide_set_wait_limit(lam_guide* g, uint32_t tries) {

@@ -118,6 +118,21 @@ LAM_DEV bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t tries = WAIT_TRIE
     return false;
 }
 
+// Barrier of warpgroup g's 128 threads; the OR of their flags.
+LAM_DEV bool group_or(uint32_t g, bool flag) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "barrier.cta.red.or.pred q, %2, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t"
+        "}\n"
+        : "=r"(r)
+        : "r"(flag ? 1u : 0u), "r"(g + 1u)
+        : "memory");
+    return r != 0u;
+}
+
 // 32 lanes x 16 consecutive f32 columns: this thread's row, columns [col, col + 16).  The wait is in
 // the same statement so that no use of the registers can be scheduled before the load completes.
 LAM_DEV void tmem_ld16(uint32_t taddr, float* v) {
@@ -152,6 +167,21 @@ LAM_DEV void tmem_ld64(uint32_t taddr, float* v) {
         : "r"(taddr));
 #pragma unroll
     for (int k = 0; k < 64; ++k) v[k] = __uint_as_float(r[k]);
+}
+// 32 consecutive columns in one load and one wait.
+LAM_DEV void tmem_ld32(uint32_t taddr, float* v) {
+    uint32_t r[32];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+#pragma unroll
+    for (int k = 0; k < 32; ++k) v[k] = __uint_as_float(r[k]);
 }
 // 32 + 8 columns (the head) in one statement and one wait.
 LAM_DEV void tmem_ld40(uint32_t taddr, float* v) {
@@ -313,13 +343,24 @@ LAM_DEV v3 mixture_sample(const Lobes& L, float u0, float u1, float u2) {
 }
 
 // Gradient of  scale * (-weight * log q(w))  with respect to the 40 head outputs; returns the loss term.
-LAM_DEV float head_grad(const float* raw, v3 w, float weight, float scale, float* g) {
+// Two threads share a row, HALF = 0 or 1 of its lobes each (1,500 instructions of one warp per scheduler
+// otherwise): the lobes' log terms meet in `terms` (LOBES floats of the row) at a barrier of the block,
+// the mixture sums are formed by both, in lobe order.  g: outputs 8 k + 4 HALF + 0..3 as g[4 k + 0..3].
+template <int HALF>
+LAM_DEV float head_grad(const float* raw, v3 w, float weight, float scale, float* terms, float* g) {
+    constexpr int H = LOBES / 2, J = HALF * H;
     Lobes L;
     lobes_from_raw(raw, L);
     float lf[LOBES], mx = -3.0e38f;
 #pragma unroll
-    for (int j = 0; j < LOBES; ++j) {
+    for (int j = J; j < J + H; ++j) {
         lf[j] = __logf(fmaxf(L.pi[j], 1e-30f)) + vmf_log_pdf(L.kappa[j], dot(L.mu[j], w));
+        terms[j] = lf[j];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < LOBES; ++j) {
+        lf[j] = terms[j];
         mx = fmaxf(mx, lf[j]);
     }
     float s = 0.0f;
@@ -328,20 +369,21 @@ LAM_DEV float head_grad(const float* raw, v3 w, float weight, float scale, float
     const float logq = mx + __logf(s);
     const float c = -weight * scale;
 #pragma unroll
-    for (int j = 0; j < LOBES; ++j) {
+    for (int q = 0; q < H; ++q) {
+        const int j = J + q;
         const float r = __expf(lf[j] - logq);
         const float k = L.kappa[j];
         const float cm = dot(L.mu[j], w);
-        g[j] = c * (r - L.pi[j]);
+        g[q] = c * (r - L.pi[j]);
         const float in_range = (raw[8 + j] > KAPPA_LOG_MIN && raw[8 + j] < KAPPA_LOG_MAX) ? 1.0f : 0.0f;
         const float dlogf_dk = 1.0f / k - 2.0f / expm1f(2.0f * k) + (cm - 1.0f);
-        g[8 + j] = c * r * k * dlogf_dk * in_range;
+        g[H + q] = c * r * k * dlogf_dk * in_range;
         v3 m = mk(raw[16 + j], raw[24 + j], raw[32 + j]);
         const float ml = fmaxf(len(m), 1e-12f);
         v3 dm = (w - L.mu[j] * cm) * (c * r * k / ml);
-        g[16 + j] = dm.x;
-        g[24 + j] = dm.y;
-        g[32 + j] = dm.z;
+        g[2 * H + q] = dm.x;
+        g[3 * H + q] = dm.y;
+        g[4 * H + q] = dm.z;
     }
     return -weight * scale * logq;
 }
@@ -419,19 +461,6 @@ LAM_DEV void epilogue_relu(uint32_t t_row, uint8_t* dst, uint32_t row) {
     for (uint32_t c = 0; c < 8; ++c) store_chunk(dst, X_RG, row, c, v + 8 * c);
 }
 LAM_DEV void head_read(uint32_t t_row, float* raw) { tmem_ld40(t_row, raw); }
-
-// Forward pass of a tile whose features are in X (overwritten layer by layer); raw = head outputs.
-LAM_DEV bool forward_infer(TileCtx& c, uint8_t* X, uint32_t w_addr, float* raw) {
-    const uint32_t x_addr = smem_u32(X);
-    const uint32_t row = threadIdx.x;
-    const uint32_t t_row = c.tmem + ((threadIdx.x & ~31u) << 16);
-    for (uint32_t l = 0; l < (uint32_t)LAYERS; ++l) {
-        if (!mma_round(c, [&] { issue_fwd(c.tmem, x_addr, w_addr + l * LAYER_BYTES); })) return false;
-        if (l < 3u) epilogue_relu(t_row, X, row);
-        else head_read(t_row, raw);
-    }
-    return true;
-}
 
 }  // namespace net
 }  // namespace lam

@@ -99,9 +99,8 @@ namespace lam {
 // Render-side training record: pos, normal, wo, wi, weight (the public lam_guide_record), then the
 // path throughput and accumulated colour at the vertex, and the previous record of the same path.
 constexpr uint32_t GUIDE_RECORD_STRIDE = 20;
-int guide_grad_and_update(lam_guide* g, const float* recs, uint32_t stride, uint32_t n, const uint32_t* n_dev,
-                          uint32_t batch, bool sequential, float scale, const float box[6], uint32_t mode, float* grad,
-                          float* loss, cudaStream_t st);
+int guide_train(lam_guide* g, const float* recs, uint32_t stride, uint32_t n, const uint32_t* n_dev, uint32_t steps,
+                const float box[6], cudaStream_t st);
 int guide_check_error(const lam_guide* g);
 
 int set_intersection_handler(lam_tracer* t, const char* src);

@@ -1104,21 +1104,6 @@ constexpr uint32_t GUIDE_SMEM = net::LAYERS * net::LAYER_BYTES + GUIDE_GROUPS * 
 constexpr uint32_t GUIDE_TMEM_GROUP = 128;  // accumulators of tiles A (columns 0..63) and B (64..127)
 constexpr uint32_t GUIDE_TMEM_COLS = GUIDE_GROUPS * GUIDE_TMEM_GROUP;
 
-// Barrier of warpgroup g's 128 threads; the OR of their flags.
-LAM_DEV bool group_or(uint32_t g, bool flag) {
-    uint32_t r;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.u32 p, %1, 0;\n\t"
-        "barrier.cta.red.or.pred q, %2, 128, p;\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t"
-        "}\n"
-        : "=r"(r)
-        : "r"(flag ? 1u : 0u), "r"(g + 1u)
-        : "memory");
-    return r != 0u;
-}
-
 // The Markov sampler's mixture pdf at w from the lobes the shade kernel kept for the path:
 // c0 cos/pi + sum_k w_k vMF_k(w), where w_k already includes the vMF branch's probability.
 LAM_DEV float markov_mixture_pdf(const Args& A, uint32_t path, float c0, v3 n, v3 w) {
@@ -1385,7 +1370,7 @@ __global__ void __launch_bounds__(NET ? GUIDE_BLOCK : WAVE_BLOCK) guide_sample_k
         for (uint32_t l = 0; l < (uint32_t)net::LAYERS; ++l) {
             net::fence_async_smem();
             net::fence_before();
-            if (group_or(group, failed)) {
+            if (net::group_or(group, failed)) {
                 failed = true;
                 ok = false;
                 break;
@@ -2284,13 +2269,10 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
         ++launches;
         if (training) {
             h = begin(4);
-            for (uint32_t k = 0; k < gd->opts.steps_per_wave; ++k) {
-                rc = guide_grad_and_update(gd, gd->records, GUIDE_RECORD_STRIDE, gd->opts.record_capacity, w->ctr + CTR_RECORDS,
-                                           gd->opts.batch, false, 1.0f / (float)gd->opts.batch, s->bounds, 1u, nullptr,
-                                           nullptr, st);
-                if (rc) return rc;
-                launches += 2;
-            }
+            rc = guide_train(gd, gd->records, GUIDE_RECORD_STRIDE, gd->opts.record_capacity, w->ctr + CTR_RECORDS,
+                             gd->opts.steps_per_wave, s->bounds, st);
+            if (rc) return rc;
+            ++launches;
             end(h);
             gd->trained_spp += A.wave_count;
         }
