@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "guide_net.cuh"
+#include "launch.cuh"
 #include "scene.h"
 #include "tracer.h"
 
@@ -70,6 +71,7 @@ __global__ void __launch_bounds__(EVAL_THREADS, 2) guide_eval_kernel(const __gri
     uint64_t* bars = reinterpret_cast<uint64_t*>(W + LAYERS * LAYER_BYTES + EVAL_GROUPS * 2u * X_BYTES);
     uint32_t* slot = reinterpret_cast<uint32_t*>(bars + 2u * EVAL_GROUPS);
     bars += 2u * group;
+    wait_previous();
     stage_weights(W, A.packed);
     if (row == 0) {
         mbar_init(bars);
@@ -381,6 +383,7 @@ LAM_DEV uint32_t partial_param(uint32_t q) {
 __global__ void __launch_bounds__(GRAD_THREADS, 1) guide_grad_kernel(const __grid_constant__ GradArgs A) {
     extern __shared__ uint8_t smraw[];
     const GradSmem S(smraw);
+    wait_previous();
     stage_weights(S.W, A.packed);
     GradCtx c = grad_begin(S, A.wait_tries);
     uint32_t n = A.n;
@@ -458,6 +461,7 @@ LAM_DEV void adam_step(const UpdateArgs& A, uint32_t p, AdamState x, float g, fl
 
 // Loss and gradient of a lam_guide_loss_grad: the partials summed in order.
 __global__ void guide_sum_kernel(UpdateArgs A) {
+    wait_previous();
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q == 0) {
         float s = 0.0f;
@@ -680,8 +684,8 @@ static int guide_loss_grad(lam_guide* g, const float* recs, uint32_t n, const fl
     fill_args(g, recs, 13u, n, nullptr, batch, true, 1.0f / (float)n, box, A, U);
     U.grad = grad;
     U.loss = loss;
-    net::guide_grad_kernel<<<U.parts, net::GRAD_THREADS, net::GRAD_SMEM, st>>>(A);
-    net::guide_sum_kernel<<<net::PARAMS / 256, 256, 0, st>>>(U);
+    launch_next(net::guide_grad_kernel, U.parts, net::GRAD_THREADS, net::GRAD_SMEM, st, A);
+    launch_next(net::guide_sum_kernel, net::PARAMS / 256, 256, 0, st, U);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(e, "guide gradient launch");
     return LAM_OK;
@@ -730,7 +734,7 @@ int guide_eval_launch(const lam_guide* g, const float* queries, uint32_t n, cons
     A.out_aligned = ((uintptr_t)out & 15u) == 0u ? 1u : 0u;
     const uint32_t per_cta = 2u * net::TILE * net::EVAL_GROUPS;
     const uint32_t grid = std::min<uint32_t>((n + per_cta - 1u) / per_cta, (uint32_t)g->sms * 2u);
-    net::guide_eval_kernel<<<grid, net::EVAL_THREADS, net::EVAL_SMEM, st>>>(A);
+    launch_next(net::guide_eval_kernel, grid, net::EVAL_THREADS, net::EVAL_SMEM, st, A);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(e, "lam_guide_eval launch");
     return LAM_OK;

@@ -1,0 +1,35 @@
+// launch.cuh - programmatic dependent launch of kernels that follow one another in a stream.
+//
+// A kernel launched with launch_next may be set up, and its blocks started, as the previous kernel's last
+// blocks exit; its wait_previous() holds it until that kernel's results are complete and visible.  Every
+// kernel launched so calls it before it touches memory that another kernel writes or reads.  Without the
+// launch attribute, and after a kernel that was launched otherwise, it does nothing.
+//
+// It trims the 2-3 us between dependent kernels: 128x128, 1 spp, 5 bounces 158 -> 133 us; 256x256, 16 spp, 8
+// bounces 1,417 -> 1,366.  Letting the next kernel start earlier, when all blocks of the previous one have
+// (griddepcontrol.launch_dependents at their beginning), made every larger render slower (1,434 us; 1080p
+// icosphere field 78.2 -> 79.2 ms): blocks that start while another kernel holds an SM keep that kernel's
+// split of shared memory and L1.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace lam {
+
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... T>
+inline cudaError_t launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const T&... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &attr;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
+}  // namespace lam

@@ -11,6 +11,7 @@
 
 #include "device_math.cuh"
 #include "guide.cuh"
+#include "launch.cuh"
 #include "reservoir.cuh"
 #include "scene.h"
 #include "tracer.h"
@@ -67,6 +68,7 @@ LAM_DEV bool merge(lam_reservoir& res, const lam_reservoir& r, float p, uint32_t
 
 __global__ void __launch_bounds__(PASS_BLOCK) temporal_kernel(lam_reservoir* cur, const lam_reservoir* old, uint32_t width, uint32_t height,
                                 uint32_t seed_offset) {
+    wait_previous();
     const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= width * height) return;
     const uint32_t x = idx % width, y = idx / width;
@@ -105,6 +107,7 @@ __global__ void __launch_bounds__(PASS_BLOCK) spatial_kernel(const lam_reservoir
                                                              uint32_t height, uint32_t is_samples, uint32_t is_space,
                                                              uint64_t space_m, uint64_t max_m, uint32_t seed_offset,
                                                              float4* __restrict__ out) {
+    wait_previous();
     const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= width * height) return;
     const uint32_t x = idx % width, y = idx / width;
@@ -153,6 +156,7 @@ __global__ void __launch_bounds__(PASS_BLOCK) spatial_kernel(const lam_reservoir
 template <bool GI>
 __global__ void __launch_bounds__(PASS_BLOCK) eof_move_kernel(uint4* __restrict__ cur, uint4* __restrict__ old, uint64_t n,
                                                               uint32_t cap) {
+    wait_previous();
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     uint4 v = cur[i];
@@ -174,6 +178,7 @@ __global__ void __launch_bounds__(PASS_BLOCK) eof_move_kernel(uint4* __restrict_
 constexpr uint32_t EOF_CELLS = 64, CELL_WORDS = W_STRIDE / 2;
 __global__ void __launch_bounds__(EOF_CELLS* CELL_WORDS) eof_world_kernel(uint2* __restrict__ world, uint2* __restrict__ old,
                                                                           uint64_t cells) {
+    wait_previous();
     __shared__ uint2 w[EOF_CELLS * CELL_WORDS];
     const uint64_t i = (uint64_t)blockIdx.x * (EOF_CELLS * CELL_WORDS) + threadIdx.x;
     const bool in = i < cells * CELL_WORDS;
@@ -207,6 +212,7 @@ struct FramePtrs {
 
 __global__ void average_kernel(FramePtrs fp, uint32_t n, uint32_t first, uint32_t count, uint64_t pixels, float* out,
                                uint32_t total) {
+    wait_previous();
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= pixels) return;
     float4 a = first == 0u ? make_float4(0.0f, 0.0f, 0.0f, 0.0f)
@@ -303,24 +309,24 @@ extern "C" int lam_data_buffers_advance_frame(lam_data_buffers* b, uint32_t adv,
     const size_t world_bytes = b->world_len * sizeof(lam_world_markov_chain);
     if (adv & LAM_BUFFER_SPATIAL_RESAMPLING) {
         const uint64_t n = res_bytes / sizeof(uint4);
-        eof_move_kernel<true><<<(unsigned)((n + PASS_BLOCK - 1) / PASS_BLOCK), PASS_BLOCK, 0, st>>>(
-            (uint4*)b->reservoirs, (uint4*)b->old_reservoirs, n, cap);
+        launch_next(eof_move_kernel<true>, (unsigned)((n + PASS_BLOCK - 1) / PASS_BLOCK), PASS_BLOCK, 0, st,
+                    (uint4*)b->reservoirs, (uint4*)b->old_reservoirs, n, cap);
     } else {
         cudaMemsetAsync(b->reservoirs, 0, res_bytes, st);
         cudaMemsetAsync(b->old_reservoirs, 0, res_bytes, st);
     }
     if (adv & LAM_BUFFER_MARKOV_CHAIN_SCREEN_SPACE) {
         const uint64_t n = chain_bytes / sizeof(uint4);
-        eof_move_kernel<false><<<(unsigned)((n + PASS_BLOCK - 1) / PASS_BLOCK), PASS_BLOCK, 0, st>>>(
-            (uint4*)b->chains, (uint4*)b->old_chains, n, 0u);
+        launch_next(eof_move_kernel<false>, (unsigned)((n + PASS_BLOCK - 1) / PASS_BLOCK), PASS_BLOCK, 0, st,
+                    (uint4*)b->chains, (uint4*)b->old_chains, n, 0u);
     } else {
         cudaMemsetAsync(b->chains, 0, chain_bytes, st);
         cudaMemsetAsync(b->old_chains, 0, chain_bytes, st);
     }
     if (adv & LAM_BUFFER_MARKOV_CHAIN_WORLD_SPACE) {
         const uint64_t n = b->world_len;
-        eof_world_kernel<<<(unsigned)((n + EOF_CELLS - 1) / EOF_CELLS), EOF_CELLS * CELL_WORDS, 0, st>>>(
-            (uint2*)b->world, (uint2*)b->old_world, n);
+        launch_next(eof_world_kernel, (unsigned)((n + EOF_CELLS - 1) / EOF_CELLS), EOF_CELLS * CELL_WORDS, 0, st,
+                    (uint2*)b->world, (uint2*)b->old_world, n);
     } else {
         cudaMemsetAsync(b->world, 0, world_bytes, st);
         cudaMemsetAsync(b->old_world, 0, world_bytes, st);
@@ -359,8 +365,8 @@ extern "C" int lam_temporal_resampling(lam_data_buffers* b, uint32_t width, uint
     if (!b) return set_error(LAM_ERR_INVALID_ARGUMENT, "null buffers");
     if (width != b->width || height != b->height) return set_error(LAM_ERR_INVALID_ARGUMENT, "size differs from the buffers");
     uint32_t n = width * height;
-    temporal_kernel<<<(n + PASS_BLOCK - 1) / PASS_BLOCK, PASS_BLOCK, 0, (cudaStream_t)stream>>>(
-        (lam_reservoir*)b->reservoirs, (const lam_reservoir*)b->old_reservoirs, width, height, seed_offset);
+    launch_next(temporal_kernel, (n + PASS_BLOCK - 1) / PASS_BLOCK, PASS_BLOCK, 0, (cudaStream_t)stream,
+                (lam_reservoir*)b->reservoirs, (const lam_reservoir*)b->old_reservoirs, width, height, seed_offset);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? LAM_OK : cuda_error(e, "lam_temporal_resampling");
 }
@@ -374,9 +380,9 @@ extern "C" int lam_spatial_resampling(lam_data_buffers* b, const lam_frame_targe
     uint32_t n = b->width * b->height;
     const uint32_t max_val = is_space * is_space - 1u;
     const uint64_t max_m = ~0ull / std::max(1u, max_val) + 1ull, space_m = ~0ull / is_space + 1ull;
-    spatial_kernel<<<(n + PASS_BLOCK - 1) / PASS_BLOCK, PASS_BLOCK, 0, (cudaStream_t)stream>>>(
-        (const lam_reservoir*)b->reservoirs, (const lam_info*)b->info, b->width, b->height, is_samples, is_space, space_m,
-        max_m, seed_offset, (float4*)tg->color);
+    launch_next(spatial_kernel, (n + PASS_BLOCK - 1) / PASS_BLOCK, PASS_BLOCK, 0, (cudaStream_t)stream,
+                (const lam_reservoir*)b->reservoirs, (const lam_info*)b->info, b->width, b->height, is_samples, is_space,
+                space_m, max_m, seed_offset, (float4*)tg->color);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? LAM_OK : cuda_error(e, "lam_spatial_resampling");
 }
@@ -394,8 +400,8 @@ extern "C" int lam_average_frames(const float* const* frames, uint32_t n, uint32
             if (!frames[first + k]) return set_error(LAM_ERR_INVALID_ARGUMENT, "null frame pointer");
             fp.f[k] = (const float4*)frames[first + k];
         }
-        average_kernel<<<(unsigned)((pixels + PASS_BLOCK - 1) / PASS_BLOCK), PASS_BLOCK, 0, (cudaStream_t)stream>>>(
-            fp, n, first, cnt, pixels, out, n);
+        launch_next(average_kernel, (unsigned)((pixels + PASS_BLOCK - 1) / PASS_BLOCK), PASS_BLOCK, 0, (cudaStream_t)stream,
+                    fp, n, first, cnt, pixels, out, n);
     }
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? LAM_OK : cuda_error(e, "lam_average_frames");

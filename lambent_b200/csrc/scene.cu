@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "bvh8.h"
+#include "launch.cuh"
 #include "materials.cuh"
 #include "scene.h"
 #include "traverse.cuh"
@@ -410,7 +411,8 @@ __global__ void __launch_bounds__(TRACE_BLOCK) trace_rays_kernel(const __grid_co
     __shared__ TraceSmem sm;
     const uint4* tl;
     const DevInstance* in;
-    stage_tlas(S, sm, tl, in);
+    stage_tlas(S, sm, tl, in);  // the scene is no kernel's output
+    wait_previous();
     uint32_t err = 0u;
     auto load = [&](uint32_t i, float3& o, float3& d, float& t0, float& t1) {
         const float4 r0 = __ldg(reinterpret_cast<const float4*>(rays + i));
@@ -435,6 +437,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK) trace_rays_kernel(const __grid_co
 __global__ void __launch_bounds__(TRACE_BLOCK) finish_hits_kernel(const __grid_constant__ DevScene S,
                                                                   const lam_ray* __restrict__ rays, uint32_t n,
                                                                   lam_hit* hits) {
+    wait_previous();
     const uint32_t i = blockIdx.x * TRACE_BLOCK + threadIdx.x;
     if (i >= n) return;
     const uint32_t tri = hits[i].primitive_index, inst = hits[i].instance_index;
@@ -467,13 +470,13 @@ static cudaError_t launch_trace(const lam_scene* s, const lam_ray* rays, uint32_
     const dim3 grid(s->sms * 8), block(TRACE_BLOCK);
     const bool alpha = !s->dev.all_opaque;
     if (mode == LAM_TRACE_ANY) {
-        if (alpha) trace_rays_kernel<true, true><<<grid, block, 0, st>>>(s->dev, rays, n, hits, words, flags);
-        else trace_rays_kernel<true, false><<<grid, block, 0, st>>>(s->dev, rays, n, hits, words, flags);
+        if (alpha) launch_next(trace_rays_kernel<true, true>, grid, block, 0, st, s->dev, rays, n, hits, words, flags);
+        else launch_next(trace_rays_kernel<true, false>, grid, block, 0, st, s->dev, rays, n, hits, words, flags);
     } else {
-        if (alpha) trace_rays_kernel<false, true><<<grid, block, 0, st>>>(s->dev, rays, n, hits, words, flags);
-        else trace_rays_kernel<false, false><<<grid, block, 0, st>>>(s->dev, rays, n, hits, words, flags);
+        if (alpha) launch_next(trace_rays_kernel<false, true>, grid, block, 0, st, s->dev, rays, n, hits, words, flags);
+        else launch_next(trace_rays_kernel<false, false>, grid, block, 0, st, s->dev, rays, n, hits, words, flags);
     }
-    finish_hits_kernel<<<(n + TRACE_BLOCK - 1) / TRACE_BLOCK, block, 0, st>>>(s->dev, rays, n, hits);
+    launch_next(finish_hits_kernel, (n + TRACE_BLOCK - 1) / TRACE_BLOCK, block, 0, st, s->dev, rays, n, hits);
     return cudaGetLastError();
 }
 

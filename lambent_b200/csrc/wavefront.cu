@@ -15,6 +15,7 @@
 
 #include "guide.cuh"
 #include "guide_net.cuh"
+#include "launch.cuh"
 #include "materials.cuh"
 #include "reservoir.cuh"
 #include "scene.h"
@@ -298,7 +299,8 @@ LAM_DEV void start_wave(const Args& A, uint32_t paths) {
     for (uint32_t k = CTR_WAVE + threadIdx.x; k < CTR_WORDS; k += blockDim.x) A.ctr[k] = k == CTR_COUNT ? paths : 0u;
 }
 
-__global__ void __launch_bounds__(WAVE_BLOCK) generate_kernel(Args A) {
+__global__ void __launch_bounds__(WAVE_BLOCK) generate_kernel(const __grid_constant__ Args A) {
+    wait_previous();
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (blockIdx.x == 0u) {
         start_wave(A, A.npix * A.wave_count);
@@ -359,15 +361,14 @@ __global__ void __launch_bounds__(WAVE_BLOCK) extend_kernel(const __grid_constan
     __shared__ TraceSmem sm;
     const uint4* tl;
     const DevInstance* in;
-    stage_tlas(A.S, sm, tl, in);
+    stage_tlas(A.S, sm, tl, in);  // the scene is no kernel's output
+    wait_previous();
     const uint32_t n = *A.count_in;
-    const uint32_t lane = threadIdx.x & 31u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         atomicAdd(A.segments, (unsigned long long)n);      // this render
         atomicAdd(A.segments + 1, (unsigned long long)n);  // since the pipeline's buffers were created
     }
     uint32_t err = 0u;
-    (void)lane;
     trace_persistent<false, ALPHA>(
         A.S, tl, in, n, A.work, err,
         [&](uint32_t i, float3& o, float3& d, float& t0, float& t1) {
@@ -505,6 +506,7 @@ LAM_DEV void finalize_records(const Args& A, uint32_t path, v3 scol) {
 // BATCH: each path's scene is its request's (lam_batch_render).
 template <bool BATCH>
 __global__ void __launch_bounds__(WAVE_BLOCK) shade_order_kernel(const __grid_constant__ Args A) {
+    wait_previous();
     // U positions per thread, each stage's loads issued for all of them before the next stage's: a class
     // is a chain of four dependent loads (hit; triangle word and instance; material index; material)
     constexpr uint32_t NW = WAVE_BLOCK / 32, U = 4;
@@ -593,6 +595,7 @@ template <int Q, bool GUIDE, bool LEARN, bool BATCH, bool REC = GUIDE>
 // that spill (measured: 79 ms against 87 ms per 16-spp step at 1080p).  The Markov-guided forms keep
 // their registers (160; three CTAs per SM, which their shared-memory candidates also allow).
 __global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(const __grid_constant__ Args A) {
+    wait_previous();
     const uint32_t n = *A.count_in;
     const uint32_t lane = threadIdx.x & 31u;
     Grid G;
@@ -1296,6 +1299,7 @@ LAM_DEV void guide_append(const Args& A, bool go, uint32_t q, uint32_t path, con
 
 template <int Q, bool NET, bool MARKOV>
 __global__ void __launch_bounds__(NET ? GUIDE_BLOCK : WAVE_BLOCK) guide_sample_kernel(const __grid_constant__ Args A) {
+    wait_previous();
     const uint32_t n = *A.dq_count;
     const uint32_t lane = threadIdx.x & 31u;
     if (!NET) {
@@ -1441,7 +1445,8 @@ LAM_DEV float res_p_hat(const lam_reservoir& R) {
 }
 
 template <int Q>
-__global__ void __launch_bounds__(WAVE_BLOCK) accumulate_kernel(Args A, uint32_t is_last_wave) {
+__global__ void __launch_bounds__(WAVE_BLOCK) accumulate_kernel(const __grid_constant__ Args A, uint32_t is_last_wave) {
+    wait_previous();
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (is_last_wave && A.restir != LAM_RESTIR_DISABLED && A.info) {
         // the block's 36-byte surface records through shared memory, so that they leave in whole lines
@@ -1532,7 +1537,8 @@ __global__ void __launch_bounds__(WAVE_BLOCK) accumulate_kernel(Args A, uint32_t
 }
 
 // subgroupShuffle(tentative, (lane + 1) % 32) after each sample (general.wesl:349-361, 582)
-__global__ void shuffle_kernel(Args A) {
+__global__ void shuffle_kernel(const __grid_constant__ Args A) {
+    wait_previous();
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= A.npix) return;
     const uint32_t x = p % A.width, y = p / A.width;
@@ -1745,21 +1751,21 @@ int ensure_handler(lam_pipeline* pl) {
 template <int Q>
 static void launch_guide(bool net, bool markov, int grid, cudaStream_t st, const Args& A) {
     if (markov) {
-        if (net) guide_sample_kernel<Q, true, true><<<grid, GUIDE_BLOCK, GUIDE_SMEM, st>>>(A);
-        else guide_sample_kernel<Q, false, true><<<grid, WAVE_BLOCK, 0, st>>>(A);
+        if (net) launch_next(guide_sample_kernel<Q, true, true>, grid, GUIDE_BLOCK, GUIDE_SMEM, st, A);
+        else launch_next(guide_sample_kernel<Q, false, true>, grid, WAVE_BLOCK, 0, st, A);
     } else {
-        if (net) guide_sample_kernel<Q, true, false><<<grid, GUIDE_BLOCK, GUIDE_SMEM, st>>>(A);
-        else guide_sample_kernel<Q, false, false><<<grid, WAVE_BLOCK, 0, st>>>(A);
+        if (net) launch_next(guide_sample_kernel<Q, true, false>, grid, GUIDE_BLOCK, GUIDE_SMEM, st, A);
+        else launch_next(guide_sample_kernel<Q, false, false>, grid, WAVE_BLOCK, 0, st, A);
     }
 }
 
 template <int Q>
 static void launch_shade(bool guide, bool learned, dim3 g, dim3 b, cudaStream_t st, const Args& A) {
-    if (guide && learned) shade_kernel<Q, true, true, false><<<g, b, GUIDE_SHADE_SMEM, st>>>(A);
-    else if (guide) shade_kernel<Q, true, false, false><<<g, b, GUIDE_SHADE_SMEM, st>>>(A);
-    else if (learned) shade_kernel<Q, false, true, false><<<g, b, 0, st>>>(A);
-    else if (A.ort) shade_kernel<Q, false, false, false, true><<<g, b, 0, st>>>(A);
-    else shade_kernel<Q, false, false, false><<<g, b, 0, st>>>(A);
+    if (guide && learned) launch_next(shade_kernel<Q, true, true, false>, g, b, GUIDE_SHADE_SMEM, st, A);
+    else if (guide) launch_next(shade_kernel<Q, true, false, false>, g, b, GUIDE_SHADE_SMEM, st, A);
+    else if (learned) launch_next(shade_kernel<Q, false, true, false>, g, b, 0, st, A);
+    else if (A.ort) launch_next(shade_kernel<Q, false, false, false, true>, g, b, 0, st, A);
+    else launch_next(shade_kernel<Q, false, false, false>, g, b, 0, st, A);
 }
 
 
@@ -1802,6 +1808,7 @@ LAM_DEV void create_ray_req(const BatchReq& R, uint32_t x, uint32_t y, v3* o, v3
 // Zeroes the batch's error flags, its segment count and the per-request completion counters, and
 // stamps the batch start.
 __global__ void batch_start_kernel(uint32_t* ctr, uint32_t* done, unsigned long long* times, uint32_t n) {
+    wait_previous();
     if (threadIdx.x < CTR_TOTAL) ctr[threadIdx.x] = 0u;
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) done[i] = 0u;
     __syncthreads();
@@ -1811,6 +1818,7 @@ __global__ void batch_start_kernel(uint32_t* ctr, uint32_t* done, unsigned long 
 // One thread per (segment, pixel): the request's seed chain and camera ray for each of the
 // segment's samples (as generate_kernel does for a single render).
 __global__ void __launch_bounds__(WAVE_BLOCK) batch_generate_kernel(const __grid_constant__ Args A) {
+    wait_previous();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (blockIdx.x == 0u) start_wave(A, A.npix);  // npix: paths of this wave
     if (t >= A.pix_threads) return;
@@ -1844,6 +1852,7 @@ __global__ void __launch_bounds__(WAVE_BLOCK) batch_generate_kernel(const __grid
 
 template <bool ALPHA>
 __global__ void __launch_bounds__(WAVE_BLOCK) extend_batch_kernel(const __grid_constant__ Args A) {
+    wait_previous();
     const uint32_t n = *A.count_in;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         atomicAdd(A.segments, (unsigned long long)n);
@@ -1867,6 +1876,7 @@ __global__ void __launch_bounds__(WAVE_BLOCK) extend_batch_kernel(const __grid_c
 // One thread per (segment, pixel): sums the segment's samples in sample order; after a request's
 // last sample writes its mean colour and, for the last pixel to finish, its completion time.
 __global__ void __launch_bounds__(WAVE_BLOCK) batch_accumulate_kernel(const __grid_constant__ Args A) {
+    wait_previous();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= A.pix_threads) return;
     const BatchSeg sg = A.segs[find_seg(A.segs, A.nsegs, t)];
@@ -2203,7 +2213,7 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
         A.rec_head = training ? w->rec_head : nullptr;
         A.guide_frac = use_net ? gd->opts.guide_fraction : 0.0f;
         int h = begin(0);
-        generate_kernel<<<gpix, blk, 0, st>>>(A);
+        launch_next(generate_kernel, gpix, blk, 0, st, A);
         end(h);
         ++launches;
         for (uint32_t depth = 0; depth < pl->opts.max_depth; ++depth) {
@@ -2225,14 +2235,14 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
                 void* kargs[] = {&A};
                 cudaLaunchKernel((const void*)pl->handler->extend, dim3(w->grid_extend), blk, kargs, 0, st);
             } else if (alpha) {
-                extend_kernel<true><<<w->grid_extend, blk, 0, st>>>(A);
+                launch_next(extend_kernel<true>, w->grid_extend, blk, 0, st, A);
             } else {
-                extend_kernel<false><<<w->grid_extend, blk, 0, st>>>(A);
+                launch_next(extend_kernel<false>, w->grid_extend, blk, 0, st, A);
             }
             end(h);
             h = begin(2);
             if (sorted) {
-                shade_order_kernel<false><<<w->grid_sort, blk, 0, st>>>(A);
+                launch_next(shade_order_kernel<false>, w->grid_sort, blk, 0, st, A);
                 ++launches;
             }
             switch (pl->quality) {
@@ -2260,11 +2270,11 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
         }
         h = begin(3);
         if (guide) {
-            shuffle_kernel<<<gpix, blk, 0, st>>>(A);
+            launch_next(shuffle_kernel, gpix, blk, 0, st, A);
             ++launches;
         }
         const uint32_t last = first + A.wave_count >= pl->opts.samples ? 1u : 0u;
-        accumulate_kernel<0><<<gpix, blk, 0, st>>>(A, last);
+        launch_next(accumulate_kernel<0>, gpix, blk, 0, st, A, last);
         end(h);
         ++launches;
         if (training) {
@@ -2567,7 +2577,7 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
     const dim3 blk(WAVE_BLOCK);
     uint32_t launches = 0;
     auto record = [&]() {
-        batch_start_kernel<<<1, 256, 0, st>>>(w->ctr, b->done, b->times, n);
+        launch_next(batch_start_kernel, 1, 256, 0, st, w->ctr, b->done, b->times, n);
         for (size_t wv = 0; wv < P.wave_begin.size(); ++wv) {
             A.segs = b->segs + P.wave_begin[wv];
             A.nsegs = P.wave_nsegs[wv];
@@ -2585,7 +2595,7 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
             A.qacc = aca;
             A.qmisc = mia;
             const dim3 gp((A.pix_threads + WAVE_BLOCK - 1) / WAVE_BLOCK);
-            batch_generate_kernel<<<gp, blk, 0, st>>>(A);
+            launch_next(batch_generate_kernel, gp, blk, 0, st, A);
             for (uint32_t depth = 0; depth < pl->opts.max_depth; ++depth) {
                 A.q_in = qa;
                 A.q_out = qb;
@@ -2600,16 +2610,16 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
                 A.qthr_out = thb;
                 A.qacc_out = acb;
                 A.qmisc_out = mib;
-                if (all_opaque) extend_batch_kernel<false><<<grid_e, blk, 0, st>>>(A);
-                else extend_batch_kernel<true><<<grid_e, blk, 0, st>>>(A);
+                if (all_opaque) launch_next(extend_batch_kernel<false>, grid_e, blk, 0, st, A);
+                else launch_next(extend_batch_kernel<true>, grid_e, blk, 0, st, A);
                 if (sorted) {
-                    shade_order_kernel<true><<<grid_sort, blk, 0, st>>>(A);
+                    launch_next(shade_order_kernel<true>, grid_sort, blk, 0, st, A);
                     ++launches;
                 }
                 switch (pl->quality) {
-                    case LAM_QUALITY_LOW: shade_kernel<LAM_QUALITY_LOW, false, false, true><<<grid_s, blk, 0, st>>>(A); break;
-                    case LAM_QUALITY_HIGH: shade_kernel<LAM_QUALITY_HIGH, false, false, true><<<grid_s, blk, 0, st>>>(A); break;
-                    default: shade_kernel<LAM_QUALITY_MEDIUM, false, false, true><<<grid_s, blk, 0, st>>>(A); break;
+                    case LAM_QUALITY_LOW: launch_next(shade_kernel<LAM_QUALITY_LOW, false, false, true>, grid_s, blk, 0, st, A); break;
+                    case LAM_QUALITY_HIGH: launch_next(shade_kernel<LAM_QUALITY_HIGH, false, false, true>, grid_s, blk, 0, st, A); break;
+                    default: launch_next(shade_kernel<LAM_QUALITY_MEDIUM, false, false, true>, grid_s, blk, 0, st, A); break;
                 }
                 launches += 2;
                 std::swap(qa, qb);
@@ -2619,7 +2629,7 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
                 std::swap(aca, acb);
                 std::swap(mia, mib);
             }
-            batch_accumulate_kernel<<<gp, blk, 0, st>>>(A);
+            launch_next(batch_accumulate_kernel, gp, blk, 0, st, A);
             launches += 2;
         }
     };
