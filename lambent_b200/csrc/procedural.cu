@@ -26,7 +26,8 @@ extern "C" __global__ void __launch_bounds__(WAVE_BLOCK) lam_proc_extend(const _
     trace_persistent<false, true>(
         A.S, tl, in, n, A.work, err,
         [&](uint32_t i, float3& o, float3& d, float& t0, float& t1) {
-            const float4 o4 = A.ray_o[i], d4 = A.ray_d[i];
+            float4 o4, d4;
+            load_ray(A, i, &o4, &d4);
             o = make_float3(o4.x, o4.y, o4.z);
             d = make_float3(d4.x, d4.y, d4.z);
             t0 = A.tmin;
@@ -35,7 +36,7 @@ extern "C" __global__ void __launch_bounds__(WAVE_BLOCK) lam_proc_extend(const _
         [&](uint32_t i, const TraceResult& tr) {
             A.hit[i] = make_uint2(tr.tri, tr.inst);
             if (tr.tri != NO_HIT && (in[tr.inst].flags & INST_PROCEDURAL)) {
-                const uint32_t path = A.q_in[i];
+                const uint32_t path = A.first ? i : A.q_in[i];
                 A.phit_a[path] = make_float4(tr.pn.x, tr.pn.y, tr.pn.z, tr.t);
                 A.phit_b[path] = make_float4(tr.ptg.x, tr.ptg.y, tr.ptg.z, 0.0f);
             }

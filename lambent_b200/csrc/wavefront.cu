@@ -327,29 +327,30 @@ __global__ void __launch_bounds__(WAVE_BLOCK) generate_kernel(const __grid_const
     }
     v3 o, d;
     create_ray(A, x, y, &o, &d);
+    if (A.first) A.ray_d[p] = make_float4(d.x, d.y, d.z, 0.0f);
     for (uint32_t j = 0; j < A.wave_count; ++j) {
         const uint32_t path = j * A.npix + p;
         const uint32_t fill_seed = st;
         st = advance_fill_seed(st);
-        A.ray_o[path] = make_float4(o.x, o.y, o.z, 0.0f);
-        A.ray_d[path] = make_float4(d.x, d.y, d.z, 0.0f);
-        A.qthr[path] = make_float4(1.0f, 1.0f, 1.0f, -1.0f);
-        A.qacc[path] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        A.qmisc[path] = make_uint4(0u, st, 0u, 0u);
-        if (A.ort) {
+        if (A.first) {
+            A.q_in[path] = st;
+        } else {  // Markov guiding: the whole state
+            A.ray_o[path] = make_float4(o.x, o.y, o.z, 0.0f);
+            A.ray_d[path] = make_float4(d.x, d.y, d.z, 0.0f);
+            A.qthr[path] = make_float4(1.0f, 1.0f, 1.0f, -1.0f);
+            A.qacc[path] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            A.qmisc[path] = make_uint4(0u, st, 0u, 0u);
+            A.q_in[path] = path;
             A.ort[path] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
             A.orad[path] = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
             A.ppoint[path] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(TY_SKY));
             A.pnormal[path] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(fill_seed));
             A.vpoint[path] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             A.vnormal[path] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
-        if (A.lnormal) {
             A.lnormal[path] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             A.ldir[path] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
         if (A.rec_head) A.rec_head[path] = NO_REC;
-        A.q_in[path] = path;
         st = rand_u32(st);
     }
     A.pixel_seed[p] = st;
@@ -372,7 +373,8 @@ __global__ void __launch_bounds__(WAVE_BLOCK) extend_kernel(const __grid_constan
     trace_persistent<false, ALPHA>(
         A.S, tl, in, n, A.work, err,
         [&](uint32_t i, float3& o, float3& d, float& t0, float& t1) {
-            const float4 o4 = ld_stream(A.ray_o + i), d4 = ld_stream(A.ray_d + i);
+            float4 o4, d4;
+            load_ray(A, i, &o4, &d4);
             o = make_float3(o4.x, o4.y, o4.z);
             d = make_float3(d4.x, d4.y, d4.z);
             t0 = A.tmin;
@@ -646,8 +648,12 @@ __global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(cons
         float4 o_thr = make_float4(0.0f, 0.0f, 0.0f, 0.0f), o_acc = o_thr;  // the outgoing state
         uint4 o_misc = make_uint4(0u, 0u, 0u, 0u);
         if (i < n) {
+            // depth 0 (load_ray): the queue is the identity, and every state but the seed is its start value
+            const bool first = !BATCH && !GUIDE && A.first;
             path = A.q_in[i];
-            const uint4 misc = ld_stream(A.qmisc + i);
+            uint4 misc = make_uint4(0u, path, 0u, 0u);
+            if (first) path = i;
+            else misc = ld_stream(A.qmisc + i);
             uint32_t fl = misc.z;
             // per-render fields; a batched render takes them from the path's request
             const DevScene* Sp = &A.S;
@@ -664,28 +670,32 @@ __global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(cons
                 out_normal = R.out_normal;
                 out_albedo = R.out_albedo;
             } else {
-                pixel = path % A.npix;
-                sample_index = A.wave_first + path / A.npix;
+                pixel = pixel_of(A, path);
+                sample_index = A.wave_first + plane_of(A, path);
             }
             const DevScene& S = *Sp;
             const bool last_sample = sample_index + 1u == samples;
             const uint32_t depth = fl & 0xFFu;
             bool last_not_vmf = (fl >> 8) & 1u;
-            const float4 o4 = ld_stream(A.ray_o + i), d4 = ld_stream(A.ray_d + i);
+            float4 o4, d4;
+            load_ray(A, i, &o4, &d4);
             ro = mk(o4.x, o4.y, o4.z);
             rd = mk(d4.x, d4.y, d4.z);
             seg_w = o4.w;
-            float4 th = ld_stream(A.qthr + i);
+            float4 th = make_float4(1.0f, 1.0f, 1.0f, -1.0f), ac = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (!first) {
+                th = ld_stream(A.qthr + i);
+                ac = ld_stream(A.qacc + i);
+            }
             v3 color = mk(th.x, th.y, th.z);
             float picked = th.w;
-            float4 ac = ld_stream(A.qacc + i);
             v3 scol = mk(ac.x, ac.y, ac.z);
             float cached_pdf = ac.w, cached_brdf = __uint_as_float(misc.x);
             uint32_t seed = misc.y;
             v3 orc = splat(1.0f), orad = splat(0.0f);
             float sum_mc = 0.0f;
-            float4 pp = make_float4(0, 0, 0, 0), pn = make_float4(0, 0, 0, 0);
-            if (REC) {
+            float4 pp = make_float4(0, 0, 0, __uint_as_float(TY_SKY)), pn = make_float4(0, 0, 0, 0);
+            if (REC && !first) {
                 float4 t0 = A.ort[path], t1 = A.orad[path];
                 orc = mk(t0.x, t0.y, t0.z);
                 sum_mc = t0.w;
@@ -1033,6 +1043,10 @@ __global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(cons
             // live state at its slot in the guide kernel's queue, and a continuing one its state at its
             // slot in the next queue (both below)
             if (!cont) A.acc[path] = o_acc;
+            if (REC && first && !cont) {  // a path without a visible vertex (depth 1 writes it otherwise)
+                A.vpoint[path] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                A.vnormal[path] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
             if (REC) {
                 A.ort[path] = make_float4(orc.x, orc.y, orc.z, sum_mc);
                 A.orad[path] = make_float4(orad.x, orad.y, orad.z, 0.0f);
@@ -2068,6 +2082,7 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
     A.width = tg->width;
     A.height = tg->height;
     A.npix = w->npix;
+    A.npix_m = ~0ull / w->npix + 1ull;
     A.samples = pl->opts.samples;
     A.max_depth = pl->opts.max_depth;
     A.restir = restir;
@@ -2212,6 +2227,7 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
         }
         A.rec_head = training ? w->rec_head : nullptr;
         A.guide_frac = use_net ? gd->opts.guide_fraction : 0.0f;
+        A.first = guide ? 0u : 1u;
         int h = begin(0);
         launch_next(generate_kernel, gpix, blk, 0, st, A);
         end(h);
@@ -2220,6 +2236,7 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
             A.q_in = qa;
             A.q_out = qb;
             set_depth(A, w, depth);
+            A.first = !guide && depth == 0u ? 1u : 0u;
             A.ray_o = rao;
             A.ray_d = rad;
             A.ray_o_out = rbo;

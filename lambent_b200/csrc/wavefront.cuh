@@ -55,6 +55,8 @@ struct Args {
     uint32_t width, height, npix, samples, max_depth, restir, seed_offset;
     float tmin, tmax;
     uint32_t wave_first, wave_count;
+    uint64_t npix_m;         // ~0 / npix + 1: multiplier of pixel_of's division
+    uint32_t first;          // depth 0 of a wave whose generate kernel left only seeds and directions (first_ray)
     uint32_t pdf_at_sample;  // LAM_GUIDE_PDF_AT_SAMPLE: Markov mixture pdf with its cosine term at the chosen direction
     uint32_t guide_metal;    // LAM_GUIDE_METAL: the learned guide is mixed in at rough metallic vertices too
     // wave buffers
@@ -127,5 +129,26 @@ struct Args {
     uint32_t* req_done;      // per request: pixels finished
     unsigned long long* req_time;  // per request: global timer at completion; [n] = batch start
 };
+
+// Sample plane and pixel of a path: path / npix and path % npix by a multiplication (exact for 32-bit paths;
+// Lemire, Kaser and Kurz, "Faster remainder by direct computation", 2019).
+LAM_DEV uint32_t plane_of(const Args& A, uint32_t path) {
+    return A.npix > 1u ? (uint32_t)__umul64hi(A.npix_m, (uint64_t)path) : path;
+}
+LAM_DEV uint32_t pixel_of(const Args& A, uint32_t path) { return path - plane_of(A, path) * A.npix; }
+
+// The ray at position i of the queue.  At depth 0 (A.first) the queue is the identity, all rays start at
+// the camera and the samples of a pixel share their direction: the generate kernel then writes 16 bytes per
+// pixel and a seed per path instead of 84 bytes per path, which extend and shade read back (icosphere
+// field at 1080p, 16 spp: 33M paths; FIRST_T).
+LAM_DEV void load_ray(const Args& A, uint32_t i, float4* o, float4* d) {
+    if (A.first) {
+        *o = make_float4(A.camera_pos.x, A.camera_pos.y, A.camera_pos.z, 0.0f);
+        *d = A.ray_d[pixel_of(A, i)];
+    } else {
+        *o = ld_stream(A.ray_o + i);
+        *d = ld_stream(A.ray_d + i);
+    }
+}
 
 }  // namespace lam
