@@ -22,10 +22,7 @@ struct DebugArgs {
 
 template <bool ALPHA>
 __global__ void __launch_bounds__(128) debug_kernel(DebugArgs A) {
-    __shared__ TraceSmem sm;
-    const uint4* tl;
-    const DevInstance* in;
-    stage_tlas(A.S, sm, tl, in);
+    const DevInstance* in = stage_instances(A.S);
     __shared__ CoopScratch<false> scratch[4];  // one per warp of a 128-thread block
     CoopScratch<false>& ws = scratch[threadIdx.x >> 5];
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -49,7 +46,7 @@ __global__ void __launch_bounds__(128) debug_kernel(DebugArgs A) {
     uint32_t err = 0;
     T.transparent_passes = false;
     T.init(A.S, ws, o, d, A.tmin, A.tmax);
-    while (T.step(A.S, tl, in, stack, ws, err)) {
+    while (T.step(A.S, in, stack, ws, err)) {
     }
     float3 c = make_float3(0.0f, 0.0f, 0.0f);
     const TraceResult& r = T.res;
@@ -108,8 +105,8 @@ int render_debug(lam_pipeline* pl, const lam_scene* s, const lam_camera* cam, co
     A.albedo = (float4*)tg->albedo;
     const uint32_t n = tg->width * tg->height;
     dim3 grid((n + 127) / 128), block(128);
-    if (s->dev.all_opaque) debug_kernel<false><<<grid, block, 0, st>>>(A);
-    else debug_kernel<true><<<grid, block, 0, st>>>(A);
+    if (s->dev.all_opaque) debug_kernel<false><<<grid, block, instance_smem(A.S), st>>>(A);
+    else debug_kernel<true><<<grid, block, instance_smem(A.S), st>>>(A);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(e, "debug render launch");
     pl->stats.samples = n;

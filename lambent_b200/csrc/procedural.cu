@@ -13,10 +13,7 @@ using namespace lam;
 // The wavefront extend step (extend_kernel) with the handler: also records the handler's normal,
 // tangent and t for procedural hits, which the shade kernel reads.
 extern "C" __global__ void __launch_bounds__(WAVE_BLOCK) lam_proc_extend(const __grid_constant__ Args A) {
-    __shared__ TraceSmem sm;
-    const uint4* tl;
-    const DevInstance* in;
-    stage_tlas(A.S, sm, tl, in);
+    const DevInstance* in = stage_instances(A.S);
     const uint32_t n = *A.count_in;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         atomicAdd(A.segments, (unsigned long long)n);
@@ -24,7 +21,7 @@ extern "C" __global__ void __launch_bounds__(WAVE_BLOCK) lam_proc_extend(const _
     }
     uint32_t err = 0u;
     trace_persistent<false, true>(
-        A.S, tl, in, n, A.work, err,
+        A.S, in, n, A.work, err,
         [&](uint32_t i, float3& o, float3& d, float& t0, float& t1) {
             float4 o4, d4;
             load_ray(A, i, &o4, &d4);
@@ -48,10 +45,7 @@ extern "C" __global__ void __launch_bounds__(WAVE_BLOCK) lam_proc_extend(const _
 template <bool ANY>
 LAM_DEV void proc_trace(const DevScene& S, const lam_ray* __restrict__ rays, uint32_t n, lam_hit* __restrict__ hits,
                         uint32_t* __restrict__ counter, uint32_t* __restrict__ err_out) {
-    __shared__ TraceSmem sm;
-    const uint4* tl;
-    const DevInstance* in;
-    stage_tlas(S, sm, tl, in);
+    const DevInstance* in = stage_instances(S);
     uint32_t err = 0u;
     auto load = [&](uint32_t i, float3& o, float3& d, float& t0, float& t1) {
         const float4 r0 = __ldg(reinterpret_cast<const float4*>(rays + i));
@@ -91,7 +85,7 @@ LAM_DEV void proc_trace(const DevScene& S, const lam_ray* __restrict__ rays, uin
         }
         hits[i] = h;
     };
-    trace_persistent<ANY, true>(S, tl, in, n, counter, err, load, store);
+    trace_persistent<ANY, true>(S, in, n, counter, err, load, store);
     if (err) *err_out = err;  // mapped host memory; one flag only, so a plain store
     trace_done(counter);
 }

@@ -313,8 +313,11 @@ extern "C" int lam_scene_create(const lam_scene_desc* d, void* stream, lam_scene
         return code;
     };
     if ((rc = alloc_trace_slots(s, st))) return fail(rc);
-    if ((rc = upload(s, reinterpret_cast<const uint4*>(blas_nodes.data()), blas_nodes.size() * 5, &D.blas_nodes, st))) return fail(rc);
-    if ((rc = upload(s, reinterpret_cast<const uint4*>(tlas.nodes.data()), tlas.nodes.size() * 5, &D.tlas_nodes, st))) return fail(rc);
+    for (Bvh8Node nd : tlas.nodes) {  // after the BLASes' nodes, in one array
+        nd.child_base += (uint32_t)total_nodes;
+        blas_nodes.push_back(nd);
+    }
+    if ((rc = upload(s, reinterpret_cast<const uint4*>(blas_nodes.data()), blas_nodes.size() * 5, &D.nodes, st))) return fail(rc);
     if ((rc = upload(s, tris.data(), tris.size(), &D.tris, st))) return fail(rc);
     if ((rc = upload(s, tlas.leaf_items.data(), tlas.leaf_items.size(), &D.tlas_items, st))) return fail(rc);
     if ((rc = upload(s, inst.data(), inst.size(), &D.inst, st))) return fail(rc);
@@ -338,6 +341,7 @@ extern "C" int lam_scene_create(const lam_scene_desc* d, void* stream, lam_scene
     D.attr_first = d->diffuse_count + d->emission_count;
     D.attr_count = d->attribute_count;
     D.recolour_layer = D.attr_first + d->attribute_count;
+    D.tlas_root = (uint32_t)total_nodes;
     D.tlas_node_count = (uint32_t)tlas.nodes.size();
     D.instance_count = ni;
     D.all_opaque = all_opaque ? 1u : 0u;
@@ -403,15 +407,12 @@ extern "C" int lam_scene_destroy(lam_scene* s) {
 namespace lam {
 
 template <bool ANY, bool ALPHA>
-__global__ void __launch_bounds__(TRACE_BLOCK) trace_rays_kernel(const __grid_constant__ DevScene S,
+__global__ void __launch_bounds__(TRACE_BLOCK, ALPHA ? 6 : 7) trace_rays_kernel(const __grid_constant__ DevScene S,
                                                                  const lam_ray* __restrict__ rays, uint32_t n,
                                                                  lam_hit* __restrict__ hits,
                                                                  uint32_t* __restrict__ counter,
                                                                  uint32_t* __restrict__ err_out) {
-    __shared__ TraceSmem sm;
-    const uint4* tl;
-    const DevInstance* in;
-    stage_tlas(S, sm, tl, in);  // the scene is no kernel's output
+    const DevInstance* in = stage_instances(S);  // the scene is no kernel's output
     wait_previous();
     uint32_t err = 0u;
     auto load = [&](uint32_t i, float3& o, float3& d, float& t0, float& t1) {
@@ -426,7 +427,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK) trace_rays_kernel(const __grid_co
         hits[i].primitive_index = tr.tri;
         hits[i].instance_index = tr.inst;
     };
-    trace_persistent<ANY, ALPHA>(S, tl, in, n, counter, err, load, store);
+    trace_persistent<ANY, ALPHA>(S, in, n, counter, err, load, store);
     if (err) *err_out = err;  // possibly mapped host memory; one flag only, so a plain store
     trace_done(counter);
 }
@@ -470,11 +471,11 @@ static cudaError_t launch_trace(const lam_scene* s, const lam_ray* rays, uint32_
     const dim3 grid(s->sms * 8), block(TRACE_BLOCK);
     const bool alpha = !s->dev.all_opaque;
     if (mode == LAM_TRACE_ANY) {
-        if (alpha) launch_next(trace_rays_kernel<true, true>, grid, block, 0, st, s->dev, rays, n, hits, words, flags);
-        else launch_next(trace_rays_kernel<true, false>, grid, block, 0, st, s->dev, rays, n, hits, words, flags);
+        if (alpha) launch_next(trace_rays_kernel<true, true>, grid, block, instance_smem(s->dev), st, s->dev, rays, n, hits, words, flags);
+        else launch_next(trace_rays_kernel<true, false>, grid, block, instance_smem(s->dev), st, s->dev, rays, n, hits, words, flags);
     } else {
-        if (alpha) launch_next(trace_rays_kernel<false, true>, grid, block, 0, st, s->dev, rays, n, hits, words, flags);
-        else launch_next(trace_rays_kernel<false, false>, grid, block, 0, st, s->dev, rays, n, hits, words, flags);
+        if (alpha) launch_next(trace_rays_kernel<false, true>, grid, block, instance_smem(s->dev), st, s->dev, rays, n, hits, words, flags);
+        else launch_next(trace_rays_kernel<false, false>, grid, block, instance_smem(s->dev), st, s->dev, rays, n, hits, words, flags);
     }
     launch_next(finish_hits_kernel, (n + TRACE_BLOCK - 1) / TRACE_BLOCK, block, 0, st, s->dev, rays, n, hits);
     return cudaGetLastError();

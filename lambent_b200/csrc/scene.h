@@ -29,8 +29,7 @@ struct DevTexLayer {
 };
 
 struct DevScene {
-    const uint4* blas_nodes;      // 5 uint4 per node, all BLASes concatenated
-    const uint4* tlas_nodes;
+    const uint4* nodes;           // 5 uint4 per node, all BLASes concatenated, then the TLAS
     const float4* tris;           // 3 float4 per triangle slot: (v0, prim bits), (v1, 0), (v2, 0)
     const uint32_t* tlas_items;   // instance ids in TLAS leaf order
     const DevInstance* inst;
@@ -45,7 +44,7 @@ struct DevScene {
     uint32_t attr_first, attr_count;
     uint32_t recolour_layer;
     uint32_t sky_size;
-    uint32_t tlas_node_count;
+    uint32_t tlas_root, tlas_node_count;
     uint32_t instance_count;
     uint32_t all_opaque;
     uint32_t has_procedural;      // some instance holds AABB geometry

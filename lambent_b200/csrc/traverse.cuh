@@ -159,6 +159,23 @@ LAM_DEV float qone(uint32_t w, uint32_t k) {
     return __uint_as_float(__byte_perm(w, 0x3F800000u, 0x7604u + (k << 4)));
 }
 
+// Pairs of floats for the packed FMA.
+LAM_DEV uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+LAM_DEV uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+LAM_DEV float half2f(uint64_t v, uint32_t e) {
+    float a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    return e ? b : a;
+}
+
 // Intersects the 8 children of one node.  Outputs the node group (child_base, internal hits in
 // bits 24..31 in octant order | imask) and the leaf group (leaf_base, item hits in bits 0..23).
 LAM_DEV void intersect_node(const uint4* __restrict__ np, float3 o, float3 inv, uint32_t oct, float tmin, float tmax,
@@ -195,19 +212,25 @@ LAM_DEV void intersect_node(const uint4* __restrict__ np, float3 o, float3 inv, 
     const float Ax = 32768.0f * adx, Ay = 32768.0f * ady, Az = 32768.0f * adz;
     const float Bx = __fmaf_rn(-32768.0f, adx, aox), By = __fmaf_rn(-32768.0f, ady, aoy),
                 Bz = __fmaf_rn(-32768.0f, adz, aoz);
+    // two children per packed FMA: the loop is bound by issue (icosphere field 78.0 -> 74.9 ms a frame)
+    const uint64_t A2x = pack2(Ax, Ax), A2y = pack2(Ay, Ay), A2z = pack2(Az, Az);
+    const uint64_t B2x = pack2(Bx, Bx), B2y = pack2(By, By), B2z = pack2(Bz, Bz);
 #pragma unroll
-    for (uint32_t i = 0; i < 8; ++i) {
+    for (uint32_t i = 0; i < 8; i += 2) {
         const uint32_t k = i & 3u;
-        const float tnx = __fmaf_rn(qone(i < 4 ? nx0 : nx1, k), Ax, Bx);
-        const float tny = __fmaf_rn(qone(i < 4 ? ny0 : ny1, k), Ay, By);
-        const float tnz = __fmaf_rn(qone(i < 4 ? nz0 : nz1, k), Az, Bz);
-        const float tfx = __fmaf_rn(qone(i < 4 ? fx0 : fx1, k), Ax, Bx);
-        const float tfy = __fmaf_rn(qone(i < 4 ? fy0 : fy1, k), Ay, By);
-        const float tfz = __fmaf_rn(qone(i < 4 ? fz0 : fz1, k), Az, Bz);
-        const float tn = fmaxf(fmaxf(tnx, tny), fmaxf(tnz, tmin));
-        const float tf = fminf(fminf(tfx, tfy), fminf(tfz, tmax));
-        if (tn <= tf * 1.00000095367431640625f)
-            hits |= __byte_perm(i < 4 ? bits_a : bits_b, 0u, 0x4440u + k) << __byte_perm(i < 4 ? at_a : at_b, 0u, 0x4440u + k);
+        const uint64_t nx2 = fma2(pack2(qone(i < 4 ? nx0 : nx1, k), qone(i < 4 ? nx0 : nx1, k + 1)), A2x, B2x);
+        const uint64_t ny2 = fma2(pack2(qone(i < 4 ? ny0 : ny1, k), qone(i < 4 ? ny0 : ny1, k + 1)), A2y, B2y);
+        const uint64_t nz2 = fma2(pack2(qone(i < 4 ? nz0 : nz1, k), qone(i < 4 ? nz0 : nz1, k + 1)), A2z, B2z);
+        const uint64_t fx2 = fma2(pack2(qone(i < 4 ? fx0 : fx1, k), qone(i < 4 ? fx0 : fx1, k + 1)), A2x, B2x);
+        const uint64_t fy2 = fma2(pack2(qone(i < 4 ? fy0 : fy1, k), qone(i < 4 ? fy0 : fy1, k + 1)), A2y, B2y);
+        const uint64_t fz2 = fma2(pack2(qone(i < 4 ? fz0 : fz1, k), qone(i < 4 ? fz0 : fz1, k + 1)), A2z, B2z);
+#pragma unroll
+        for (uint32_t e = 0; e < 2; ++e) {
+            const float tn = fmaxf(fmaxf(half2f(nx2, e), half2f(ny2, e)), fmaxf(half2f(nz2, e), tmin));
+            const float tf = fminf(fminf(half2f(fx2, e), half2f(fy2, e)), fminf(half2f(fz2, e), tmax));
+            if (tn <= tf * 1.00000095367431640625f)
+                hits |= __byte_perm(i < 4 ? bits_a : bits_b, 0u, 0x4440u + k + e) << __byte_perm(i < 4 ? at_a : at_b, 0u, 0x4440u + k + e);
+        }
     }
     ng = make_uint2(n1.x, (hits & 0xFF000000u) | imask);
     tg = make_uint2(n1.y, hits & 0x00FFFFFFu);
@@ -307,7 +330,7 @@ struct Traverser {
         cur_inst = 0u;
         cur_flags = 0u;
         set_ray(org, d);
-        ng = S.tlas_node_count ? make_uint2(0u, (1u << (24u + oct)) | 1u) : make_uint2(0u, 0u);
+        ng = S.tlas_node_count ? make_uint2(S.tlas_root, (1u << (24u + oct)) | 1u) : make_uint2(0u, 0u);
         tg = make_uint2(0u, 0u);
     }
 
@@ -330,8 +353,8 @@ struct Traverser {
     // the step.  `stack` holds TRAVERSAL_STACK entries owned by this lane (kept outside the struct so
     // that the struct itself stays in registers).
     template <bool COOP>
-    LAM_DEV int step_impl(const DevScene& S, const uint4* __restrict__ tlas_nodes, const DevInstance* __restrict__ insts,
-                          uint2* stack, Scratch& ws, uint32_t& err) {
+    LAM_DEV int step_impl(const DevScene& S, const DevInstance* __restrict__ insts, uint2* stack, Scratch& ws,
+                          uint32_t& err) {
         const uint32_t lane = threadIdx.x & 31u;
         if (ng.y > 0x00FFFFFFu) {
             const uint32_t k = __ffs(ng.y >> 24) - 1u;
@@ -339,9 +362,9 @@ struct Traverser {
             const uint32_t slot = k ^ oct;
             const uint32_t child = ng.x + __popc(ng.y & ((1u << slot) - 1u) & 0xFFu);
             if (ng.y > 0x00FFFFFFu) push(stack, ng, err);
-            // one call site for TLAS and BLAS nodes: lanes of a warp on either level share one test
-            // (two call sites run the 8-wide test twice whenever a warp straddles the levels)
-            intersect_node((blas_base < 0 ? tlas_nodes : S.blas_nodes) + 5u * child, o, inv, oct, tmin, best_t, ng, tg);
+            // one call site and one array for TLAS and BLAS nodes: lanes of a warp on either level share
+            // one test (two call sites run the 8-wide test twice whenever a warp straddles the levels)
+            intersect_node(S.nodes + 5u * child, o, inv, oct, tmin, best_t, ng, tg);
         } else {
             tg = ng;
             ng = make_uint2(0u, 0u);
@@ -448,9 +471,8 @@ struct Traverser {
     }
 
     // Returns false once the traversal has finished (res is final).
-    LAM_DEV bool step(const DevScene& S, const uint4* __restrict__ tlas_nodes, const DevInstance* __restrict__ insts,
-                      uint2* stack, Scratch& ws, uint32_t& err) {
-        return step_impl<false>(S, tlas_nodes, insts, stack, ws, err) == STEP_MORE;
+    LAM_DEV bool step(const DevScene& S, const DevInstance* __restrict__ insts, uint2* stack, Scratch& ws, uint32_t& err) {
+        return step_impl<false>(S, insts, stack, ws, err) == STEP_MORE;
     }
 
     // End of a step: leave a finished instance, pop the next group; false when the ray is done.
@@ -611,13 +633,8 @@ struct Traverser {
 };
 
 // Lanes below this many active rays trigger a refill of the idle lanes from the work queue.
-#ifndef LAM_REFILL_THRESHOLD
-#define LAM_REFILL_THRESHOLD 28
-#endif
-constexpr int REFILL_THRESHOLD = LAM_REFILL_THRESHOLD;
-// Fewest rays a warp takes from a queue that cannot fill the grid: 1,000 random rays of the icosphere
-// field take 102 / 80 / 75 us with 32 / 8 / 4, a 128x128 render of the Cornell box 246 / 232 / 245.
-constexpr int MIN_WARP_RAYS = 8;
+constexpr int REFILL_THRESHOLD = 26;  // 24..30 within 2%: 26 / 28 / 30 take 1,773 / 1,801 / 1,868 us for 4.2M rays
+constexpr uint32_t SMALL_WARPS = 8;  // per SM, see trace_persistent
 
 // Persistent warp loop over work items [0, n) claimed with a global counter.  `load(i, o, d, t0, t1)`
 // fetches item i; `store(i, res)` consumes a finished traversal.  Every lane of the warp must call it,
@@ -627,18 +644,22 @@ constexpr int MIN_WARP_RAYS = 8;
 // With MULTI the items belong to different scenes: `load(i, o, d, t0, t1, sp)` also returns the item's
 // scene, whose TLAS and instances are read from global memory.
 template <bool ANY, bool ALPHA, bool MULTI = false, class Load, class Store>
-LAM_DEV void trace_persistent(const DevScene& S0, const uint4* __restrict__ tl, const DevInstance* __restrict__ in,
-                              uint32_t n, uint32_t* __restrict__ work, uint32_t& err, Load load, Store store) {
+LAM_DEV void trace_persistent(const DevScene& S0, const DevInstance* __restrict__ in, uint32_t n,
+                              uint32_t* __restrict__ work, uint32_t& err, Load load, Store store) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt_mask = (1u << lane) - 1u;
     __shared__ CoopScratch<MULTI> coop_ws[4];  // one per warp of a 128-thread block
     CoopScratch<MULTI>& ws = coop_ws[(threadIdx.x >> 5) & 3u];
     if (lane == 0u) ws.total = 0u;
     __syncwarp();
-    // A queue smaller than the grid's lanes is spread over its warps: a warp runs as long as its
-    // longest ray, and fewer rays a warp diverge less
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    const uint32_t cap = min(32u, max((uint32_t)MIN_WARP_RAYS, (n + warps - 1u) / warps));
+    // A queue that cannot fill the chip is spread over SMALL_WARPS warps per SM: a warp runs as long as its
+    // longest ray, and fewer rays a warp diverge less.  (More warps with fewer rays each issue more in total:
+    // 1,000 rays of the icosphere field take 102 us with 32 a warp, 80 with 8, 72 with 1; a 128x128 render of
+    // the Cornell box 246 us with 32, 245 with 4, 232 with 8, 229.5 with 14.)
+    uint32_t sms;
+    asm("mov.u32 %0, %%nsmid;" : "=r"(sms));
+    const uint32_t warps = min(gridDim.x * (blockDim.x >> 5), sms * SMALL_WARPS);
+    const uint32_t cap = min(32u, (n + warps - 1u) / warps);
     Traverser<ANY, ALPHA, MULTI> T;
     uint2 stack[TRAVERSAL_STACK];
     const DevScene* sp = nullptr;
@@ -675,8 +696,8 @@ LAM_DEV void trace_persistent(const DevScene& S0, const uint4* __restrict__ tl, 
         if (!__any_sync(0xFFFFFFFFu, active)) break;
         int code = STEP_MORE;
         if (active) {
-            if constexpr (MULTI) code = T.template step_impl<true>(*sp, sp->tlas_nodes, sp->inst, stack, ws, err);
-            else code = T.template step_impl<true>(S0, tl, in, stack, ws, err);
+            if constexpr (MULTI) code = T.template step_impl<true>(*sp, sp->inst, stack, ws, err);
+            else code = T.template step_impl<true>(S0, in, stack, ws, err);
         }
         const bool want = active && code == STEP_COOP;
         if (__any_sync(0xFFFFFFFFu, want)) {  // warp-uniform: triangle tests dealt out over all lanes
@@ -703,25 +724,24 @@ LAM_DEV void trace_done(uint32_t* words) {
 constexpr int TRACE_BLOCK = 128;
 constexpr uint32_t SMEM_INSTANCES = 128;
 
-struct TraceSmem {
-    DevInstance inst[SMEM_INSTANCES];
-};
+// Bytes of dynamic shared memory that a traversal kernel of this scene is launched with: its instance
+// records, if they are few enough (every instance entry reads one).  Sized by the scene, so that a small
+// one leaves the rest to L1 (64 instances: 17 instead of 21 KB a CTA, icosphere field 74.9 -> 74.6 ms).
+inline uint32_t instance_smem(const DevScene& S) {
+    return S.instance_count <= SMEM_INSTANCES ? S.instance_count * (uint32_t)sizeof(DevInstance) : 0u;
+}
 
-// Copies the instance records into shared memory when they fit (every instance entry reads one);
-// returns the pointers the traversal should use.  The TLAS nodes stay in global memory, where
-// they are L1-resident: one node-test call site then loads TLAS and BLAS nodes alike through the
-// read-only path (staging them in shared memory made those loads generic: 1104 against 1118
-// Mrays/s).
-LAM_DEV void stage_tlas(const DevScene& S, TraceSmem& sm, const uint4*& tl, const DevInstance*& in) {
-    tl = S.tlas_nodes;
-    in = S.inst;
-    if (S.instance_count <= SMEM_INSTANCES) {
-        const uint4* src = reinterpret_cast<const uint4*>(S.inst);
-        uint4* dst = reinterpret_cast<uint4*>(sm.inst);
-        for (uint32_t i = threadIdx.x; i < S.instance_count * 4u; i += blockDim.x) dst[i] = src[i];
-        in = sm.inst;
-    }
+// Copies the instance records into shared memory when they fit; returns where the traversal finds them.
+// The nodes stay in global memory, where the TLAS is L1-resident: one node-test call site then loads TLAS
+// and BLAS nodes alike through the read-only path (staging the TLAS in shared memory made those loads
+// generic: 1104 against 1118 Mrays/s).
+LAM_DEV const DevInstance* stage_instances(const DevScene& S) {
+    extern __shared__ uint4 staged_instances[];
+    if (S.instance_count > SMEM_INSTANCES) return S.inst;
+    const uint4* src = reinterpret_cast<const uint4*>(S.inst);
+    for (uint32_t i = threadIdx.x; i < S.instance_count * 4u; i += blockDim.x) staged_instances[i] = src[i];
     __syncthreads();
+    return reinterpret_cast<const DevInstance*>(staged_instances);
 }
 
 }  // namespace lam

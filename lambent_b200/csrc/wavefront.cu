@@ -359,10 +359,7 @@ __global__ void __launch_bounds__(WAVE_BLOCK) generate_kernel(const __grid_const
 // ---------------------------------------------------------------- extend
 template <bool ALPHA>
 __global__ void __launch_bounds__(WAVE_BLOCK) extend_kernel(const __grid_constant__ Args A) {
-    __shared__ TraceSmem sm;
-    const uint4* tl;
-    const DevInstance* in;
-    stage_tlas(A.S, sm, tl, in);  // the scene is no kernel's output
+    const DevInstance* in = stage_instances(A.S);  // the scene is no kernel's output
     wait_previous();
     const uint32_t n = *A.count_in;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -371,7 +368,7 @@ __global__ void __launch_bounds__(WAVE_BLOCK) extend_kernel(const __grid_constan
     }
     uint32_t err = 0u;
     trace_persistent<false, ALPHA>(
-        A.S, tl, in, n, A.work, err,
+        A.S, in, n, A.work, err,
         [&](uint32_t i, float3& o, float3& d, float& t0, float& t1) {
             float4 o4, d4;
             load_ray(A, i, &o4, &d4);
@@ -882,7 +879,7 @@ __global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(cons
                     for (int k = 16; k < 20; ++k) {
                         seed = rand_u32(rand_u32(seed)) + 1u;
                     }
-#pragma unroll 7
+#pragma unroll 3
                     for (int k = 0; k < NUM_RESAMPLES; ++k) seed = rand_u32(rand_u32(seed));
                 }
                 const bool reflecting = should_reflect || is.ty == TY_METALLIC;
@@ -1677,7 +1674,7 @@ static int ensure_wave(lam_pipeline* pl, uint32_t width, uint32_t height, bool f
     pl->prof_segments_base = 0;
     cudaDeviceGetAttribute(&w->sms, cudaDevAttrMultiProcessorCount, pl->device);
     int occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, extend_kernel<false>, WAVE_BLOCK, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, extend_kernel<false>, WAVE_BLOCK, SMEM_INSTANCES * sizeof(DevInstance));
     w->grid_extend = w->sms * std::max(1, occ);
     occ = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, shade_kernel<LAM_QUALITY_MEDIUM, false, false, false>, WAVE_BLOCK, 0);
@@ -1874,7 +1871,7 @@ __global__ void __launch_bounds__(WAVE_BLOCK) extend_batch_kernel(const __grid_c
     }
     uint32_t err = 0u;
     trace_persistent<false, ALPHA, true>(
-        A.S, nullptr, nullptr, n, A.work, err,
+        A.S, nullptr, n, A.work, err,
         [&](uint32_t i, float3& o, float3& d, float& t0, float& t1, const DevScene*& sp) {
             const float4 o4 = A.ray_o[i], d4 = A.ray_d[i];
             o = make_float3(o4.x, o4.y, o4.z);
@@ -2250,11 +2247,11 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
             h = begin(1);
             if (proc) {
                 void* kargs[] = {&A};
-                cudaLaunchKernel((const void*)pl->handler->extend, dim3(w->grid_extend), blk, kargs, 0, st);
+                cudaLaunchKernel((const void*)pl->handler->extend, dim3(w->grid_extend), blk, kargs, instance_smem(A.S), st);
             } else if (alpha) {
-                launch_next(extend_kernel<true>, w->grid_extend, blk, 0, st, A);
+                launch_next(extend_kernel<true>, w->grid_extend, blk, instance_smem(A.S), st, A);
             } else {
-                launch_next(extend_kernel<false>, w->grid_extend, blk, 0, st, A);
+                launch_next(extend_kernel<false>, w->grid_extend, blk, instance_smem(A.S), st, A);
             }
             end(h);
             h = begin(2);
@@ -2785,6 +2782,6 @@ extern "C" int lam_pipeline_trace_rays(lam_pipeline* pl, const lam_scene* s, con
     return run_trace(s, c.st, "lam_pipeline_trace_rays", [](uint32_t* words, uint32_t* flags, const void* arg) {
         Call a = *static_cast<const Call*>(arg);
         void* kargs[] = {&a.S, &a.rays, &a.n, &a.hits, &words, &flags};
-        return cudaLaunchKernel((const void*)a.kernel, a.grid, dim3(TRACE_BLOCK), kargs, 0, a.st);
+        return cudaLaunchKernel((const void*)a.kernel, a.grid, dim3(TRACE_BLOCK), kargs, instance_smem(a.S), a.st);
     }, &c);
 }

@@ -140,7 +140,8 @@ LAM_DEV uint32_t pixel_of(const Args& A, uint32_t path) { return path - plane_of
 // The ray at position i of the queue.  At depth 0 (A.first) the queue is the identity, all rays start at
 // the camera and the samples of a pixel share their direction: the generate kernel then writes 16 bytes per
 // pixel and a seed per path instead of 84 bytes per path, which extend and shade read back (icosphere
-// field at 1080p, 16 spp: 33M paths; FIRST_T).
+// field at 1080p, 16 spp: 33M paths, 0.2 ms; a ReSTIR frame at 1080p, whose start state was 180 bytes, 2,767
+// -> 2,626 us).
 LAM_DEV void load_ray(const Args& A, uint32_t i, float4* o, float4* d) {
     if (A.first) {
         *o = make_float4(A.camera_pos.x, A.camera_pos.y, A.camera_pos.z, 0.0f);
