@@ -479,7 +479,7 @@ int lam_pipeline_set_profiling(lam_pipeline* pipeline, int enabled);
 int lam_render_profile_get(lam_pipeline* pipeline, lam_stage_times* out);
 /* Wave size (no counterpart in the reference, whose rt_main holds one pixel's samples in a thread):
  * lam_render runs a frame's samples in waves of at most max(pixels, max_paths) paths; each path in
- * flight keeps about 220 bytes of device state.  0 restores the default of about 32M paths (one
+ * flight keeps about 200 bytes of device state.  0 restores the default of about 32M paths (one
  * 16-spp wave at 1080p, about 7 GB).  Markov guiding and per-sample ReSTIR always run one sample per
  * wave.  The image does not depend on the wave size; smaller waves trade speed for memory.  Takes
  * effect at the next lam_render.  lam_render itself caps a new wave at half the free device memory

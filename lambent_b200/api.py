@@ -431,7 +431,7 @@ class Pipeline:
         check(lib().lam_pipeline_set_profiling(self._h, 1 if enabled else 0))
 
     def set_wave_paths(self, max_paths=0):
-        """Bounds the paths of one wave (device memory ~220 B per path); 0 restores the default."""
+        """Bounds the paths of one wave (device memory ~200 B per path); 0 restores the default."""
         check(lib().lam_pipeline_set_wave_paths(self._h, int(max_paths)))
 
     def set_shade_order(self, order=_abi.SHADE_ORDER_AUTO):

@@ -230,18 +230,38 @@ __global__ void average_kernel(FramePtrs fp, uint32_t n, uint32_t first, uint32_
     (void)n;
 }
 
-static int dalloc(void** p, size_t bytes) {
-    *p = nullptr;
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e != cudaSuccess) return cuda_error(e, "cudaMalloc (data buffers)");
-    e = cudaMemset(*p, 0, bytes);
-    if (e != cudaSuccess) return cuda_error(e, "cudaMemset (data buffers)");
+static void free_blocks(std::vector<void*>& blocks) {
+    for (void* p : blocks) cudaFree(p);
+    blocks.clear();
+}
+
+// Cleared device memory for the buffers of `sizes`: one block, or an allocation each if none is over 1 MB
+// (the driver serves those from memory that it has mapped already).
+static int alloc_blocks(std::vector<void*>& blocks, void** const* buffers, const size_t* sizes, int n) {
+    size_t total = 0, largest = 0;
+    for (int k = 0; k < n; ++k) {
+        total += (sizes[k] + 255u) / 256u * 256u;
+        largest = std::max(largest, sizes[k]);
+    }
+    const bool single = largest <= (1u << 20);
+    char* at = nullptr;
+    for (int k = 0; k < n; ++k) {
+        if (single || k == 0) {
+            const size_t bytes = single ? sizes[k] : total;
+            cudaError_t e = cudaMalloc((void**)&at, bytes);
+            if (e != cudaSuccess) return cuda_error(e, "cudaMalloc (data buffers)");
+            blocks.push_back(at);
+            e = cudaMemset(at, 0, bytes);
+            if (e != cudaSuccess) return cuda_error(e, "cudaMemset (data buffers)");
+        }
+        *buffers[k] = at;
+        at += (sizes[k] + 255u) / 256u * 256u;
+    }
     return LAM_OK;
 }
 
 static void free_window(lam_data_buffers* b) {
-    void* ps[] = {b->reservoirs, b->old_reservoirs, b->info, b->chains, b->old_chains, b->pixel_seed};
-    for (void* p : ps) cudaFree(p);
+    free_blocks(b->window);
     b->reservoirs = b->old_reservoirs = b->info = b->chains = b->old_chains = b->pixel_seed = nullptr;
 }
 
@@ -253,14 +273,10 @@ static int alloc_window(lam_data_buffers* b, uint32_t w, uint32_t h) {
     // reservoirs are always per pixel: rt_main writes gi_reservoirs[idx] in every ReSTIR mode
     b->reservoir_len = pix;
     b->chain_len = (b->types & LAM_BUFFER_MARKOV_CHAIN_SCREEN_SPACE) ? pix : 1;
-    int rc = 0;
-    rc |= dalloc(&b->reservoirs, b->reservoir_len * sizeof(lam_reservoir));
-    rc |= dalloc(&b->old_reservoirs, b->reservoir_len * sizeof(lam_reservoir));
-    rc |= dalloc(&b->info, pix * sizeof(lam_info));
-    rc |= dalloc(&b->chains, b->chain_len * sizeof(lam_markov_chain));
-    rc |= dalloc(&b->old_chains, b->chain_len * sizeof(lam_markov_chain));
-    rc |= dalloc(&b->pixel_seed, pix * sizeof(uint32_t));
-    return rc ? LAM_ERR_CUDA : LAM_OK;
+    void** const buffers[] = {&b->reservoirs, &b->old_reservoirs, &b->info, &b->chains, &b->old_chains, &b->pixel_seed};
+    const size_t res = b->reservoir_len * sizeof(lam_reservoir), chain = b->chain_len * sizeof(lam_markov_chain);
+    const size_t sizes[] = {res, res, pix * sizeof(lam_info), chain, chain, pix * sizeof(uint32_t)};
+    return alloc_blocks(b->window, buffers, sizes, 6) ? LAM_ERR_CUDA : LAM_OK;
 }
 
 }  // namespace lam
@@ -278,12 +294,14 @@ extern "C" int lam_data_buffers_new(uint32_t width, uint32_t height, uint32_t wo
     b->world_size = std::max(1u, world_size);
     b->world_len = (types & LAM_BUFFER_MARKOV_CHAIN_WORLD_SPACE) ? b->world_size : 1;
     int rc = alloc_window(b, width, height);
-    if (!rc) rc |= dalloc(&b->world, b->world_len * sizeof(lam_world_markov_chain));
-    if (!rc) rc |= dalloc(&b->old_world, b->world_len * sizeof(lam_world_markov_chain));
+    if (!rc) {
+        void** const buffers[] = {&b->world, &b->old_world};
+        const size_t grid = b->world_len * sizeof(lam_world_markov_chain), sizes[] = {grid, grid};
+        rc = alloc_blocks(b->grids, buffers, sizes, 2);
+    }
     if (rc) {
         free_window(b);
-        cudaFree(b->world);
-        cudaFree(b->old_world);
+        free_blocks(b->grids);
         delete b;
         return rc;
     }
@@ -354,8 +372,7 @@ extern "C" int lam_data_buffers_get(const lam_data_buffers* b, uint32_t which, v
 extern "C" int lam_data_buffers_destroy(lam_data_buffers* b) {
     if (!b) return LAM_OK;
     free_window(b);
-    cudaFree(b->world);
-    cudaFree(b->old_world);
+    free_blocks(b->grids);
     delete b;
     return LAM_OK;
 }

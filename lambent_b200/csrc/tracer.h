@@ -31,6 +31,7 @@ struct lam_data_buffers {
     void* old_world = nullptr;
     void* pixel_seed = nullptr;      // u32[W*H] seed chain between waves of one render
     size_t reservoir_len = 1, chain_len = 1, world_len = 1, pixels = 1;
+    std::vector<void*> window, grids;  // allocations that hold the per-pixel buffers and the two world grids
 };
 
 namespace lam {

