@@ -625,11 +625,12 @@ __global__ void __launch_bounds__(WAVE_BLOCK) shade_order_kernel(const __grid_co
 
 // REC: out-radiance, primary and visible vertices are recorded (ReSTIR, Markov guiding).
 template <int Q, bool GUIDE, bool LEARN, bool BATCH, bool REC = GUIDE>
-// Six CTAs per SM for the unguided forms: the kernel waits on chains of dependent gathers (queue ->
-// hit -> triangle -> material -> texture), so resident warps matter more than the few registers
-// that spill (measured: 79 ms against 87 ms per 16-spp step at 1080p).  The Markov-guided forms keep
-// their registers (160; three CTAs per SM, which their shared-memory candidates also allow).
-__global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(const __grid_constant__ Args A) {
+// Seven CTAs per SM for the plain forms, six with reservoirs or deferral: the kernel waits on chains of
+// dependent gathers (queue -> hit -> triangle -> material -> texture), so resident warps matter more than
+// the few registers that spill (seven against six: 256x256, 16 spp 1,319 / 1,331 us, 64 thumbnails 4,240 /
+// 4,286; eight 1,421 against 1,416 before; a ReSTIR frame is slower at seven).  The Markov-guided forms
+// keep their registers (160; three CTAs per SM, which their shared-memory candidates also allow).
+__global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : (REC || LEARN ? 6 : 7))) shade_kernel(const __grid_constant__ Args A) {
     wait_previous();
     const uint32_t n = *A.count_in;
     const uint32_t lane = threadIdx.x & 31u;
@@ -733,8 +734,10 @@ __global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(cons
                 orc = mk(t0.x, t0.y, t0.z);
                 sum_mc = t0.w;
                 orad = mk(t1.x, t1.y, t1.z);
-                pp = A.ppoint[path];
-                pn = A.pnormal[path];
+                if (GUIDE) {  // the primary vertex trains the chains when the path ends
+                    pp = A.ppoint[path];
+                    pn = A.pnormal[path];
+                }
             }
             v3 last_normal = splat(0.0f), last_dir = splat(0.0f);
             if (GUIDE) {
@@ -1081,10 +1084,12 @@ __global__ void __launch_bounds__(WAVE_BLOCK, (GUIDE ? 1 : 6)) shade_kernel(cons
                 A.vnormal[path] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
             if (REC) {
-                A.ort[path] = make_float4(orc.x, orc.y, orc.z, sum_mc);
+                if (cont) A.ort[path] = make_float4(orc.x, orc.y, orc.z, sum_mc);
                 A.orad[path] = make_float4(orad.x, orad.y, orad.z, 0.0f);
-                A.ppoint[path] = pp;
-                A.pnormal[path] = pn;
+                if (depth == 0u) {  // the primary vertex is settled
+                    A.ppoint[path] = pp;
+                    A.pnormal[path] = pn;
+                }
             }
             if (GUIDE) {
                 A.lnormal[path] = make_float4(last_normal.x, last_normal.y, last_normal.z, 0.0f);
@@ -1729,7 +1734,12 @@ static int ensure_wave(lam_pipeline* pl, uint32_t width, uint32_t height, bool f
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, extend_kernel<false>, WAVE_BLOCK, SMEM_INSTANCES * sizeof(DevInstance));
     w->grid_extend = w->sms * std::max(1, occ);
     occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, shade_kernel<LAM_QUALITY_MEDIUM, false, false, false>, WAVE_BLOCK, 0);
+    // the blocks of the shade form that these renders run: its grid-stride loop wants one resident round
+    // (a ReSTIR frame at 1080p 2,294 us, 2,535 with the plain form's count; guided 256x256 2,492 / 2,688)
+    const void* shade = full      ? (const void*)shade_kernel<LAM_QUALITY_MEDIUM, false, false, false, true>
+                        : learned ? (const void*)shade_kernel<LAM_QUALITY_MEDIUM, false, true, false>
+                                  : (const void*)shade_kernel<LAM_QUALITY_MEDIUM, false, false, false>;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, shade, WAVE_BLOCK, 0);
     w->grid_shade = w->sms * std::max(1, occ);
     w->grid_sort = w->sms * 6;
     if (guide) {
