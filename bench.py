@@ -40,10 +40,10 @@ EXTEND_DRAM_BYTES_PER_SEGMENT = 132.4
 # What does bound the traversal kernel, from an ncu capture of two extend launches of the same
 # 960x540 case (sections SpeedOfLight, ComputeWorkloadAnalysis, MemoryWorkloadAnalysis,
 # WarpStateStats; command beside the figures in the extend-kernel profile summary): instruction issue.
-EXTEND_MEASURED_BOUND = {"kind": "instruction issue (BVH and triangles stay in L2)", "issue_slots_busy": 0.750,
-                         "alu_pipe": 0.588, "fma_pipe": 0.254, "dram_throughput": 0.010, "l2_throughput": 0.109,
-                         "l2_hit_rate": 0.797, "threads_per_instruction": 18.9, "warps_active": 0.363,
-                         "stalls_per_issue": {"wait": 1.95, "not_selected": 1.38, "long_scoreboard": 1.22},
+EXTEND_MEASURED_BOUND = {"kind": "instruction issue (BVH and triangles stay in L2)", "issue_slots_busy": 0.740,
+                         "alu_pipe": 0.545, "fma_pipe": 0.257, "dram_throughput": 0.014, "l2_throughput": 0.180,
+                         "l2_hit_rate": 0.845, "threads_per_instruction": 15.9, "warps_active": 0.422,
+                         "stalls_per_issue": {"wait": 2.05, "not_selected": 1.56, "long_scoreboard": 1.41},
                          "note": "mean of two launches of the 960x540, 4-spp case"}
 
 
