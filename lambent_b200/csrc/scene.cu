@@ -507,15 +507,14 @@ int run_trace(const lam_scene* s, cudaStream_t st, const char* who, TraceLaunch 
     }
     volatile uint32_t* flags = s->trace_flags + slot;
     cudaError_t e = launch(s->trace_words + slot * TRACE_SLOT_WORDS, s->trace_flags_dev + slot, arg);
-    if (e == cudaSuccess) {
-        e = cudaStreamSynchronize(st);
-        // a wait that failed (a stream being captured) says nothing about the kernel: the slot stays taken
-        if (e != cudaSuccess) return cuda_error(e, who);
-    }
+    // also after a launch that failed: a kernel before it may run.  A wait that failed (a stream being captured)
+    // says nothing about the kernels: the slot stays taken
+    const cudaError_t wait = cudaStreamSynchronize(st);
+    if (wait != cudaSuccess) return cuda_error(e != cudaSuccess ? e : wait, who);
     const uint32_t got = *flags;
     *flags = 0u;
     s->trace_busy.fetch_and(~(1ull << slot), std::memory_order_release);
-    if (e != cudaSuccess) return cuda_error(e, who);  // the launch failed: nothing ran
+    if (e != cudaSuccess) return cuda_error(e, who);
     return got & ERR_STACK_OVERFLOW ? set_error(LAM_ERR_STACK_OVERFLOW, "traversal stack overflow") : LAM_OK;
 }
 
