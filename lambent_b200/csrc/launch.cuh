@@ -13,6 +13,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "host_steps.h"
+
 namespace lam {
 
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -31,5 +33,21 @@ inline cudaError_t launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size
     c.numAttrs = 1;
     return cudaLaunchKernelEx(&c, kernel, P(args)...);
 }
+
+// Dependent launches of one call on a stream, each of which reads what those before it wrote.
+struct Launches {
+    cudaStream_t st;
+    Steps<cudaError_t> steps;
+    explicit Launches(cudaStream_t stream) : st(stream) {}
+    template <class... P, class... T>
+    void next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, const T&... args) {
+        steps([&] { return launch_next(kernel, grid, block, smem, st, args...); });
+    }
+    // The first failure, which is then no longer the runtime's last error either.
+    cudaError_t status() const {
+        if (steps.status != cudaSuccess) (void)cudaGetLastError();
+        return steps.status;
+    }
+};
 
 }  // namespace lam

@@ -469,16 +469,19 @@ __global__ void __launch_bounds__(TRACE_BLOCK) finish_hits_kernel(const __grid_c
 static cudaError_t launch_trace(const lam_scene* s, const lam_ray* rays, uint32_t n, uint32_t mode, lam_hit* hits,
                                 uint32_t* words, uint32_t* flags, cudaStream_t st) {
     const dim3 grid(s->sms * 8), block(TRACE_BLOCK);
+    const uint32_t smem = instance_smem(s->dev);
     const bool alpha = !s->dev.all_opaque;
+    Launches go(st);
     if (mode == LAM_TRACE_ANY) {
-        if (alpha) launch_next(trace_rays_kernel<true, true>, grid, block, instance_smem(s->dev), st, s->dev, rays, n, hits, words, flags);
-        else launch_next(trace_rays_kernel<true, false>, grid, block, instance_smem(s->dev), st, s->dev, rays, n, hits, words, flags);
+        if (alpha) go.next(trace_rays_kernel<true, true>, grid, block, smem, s->dev, rays, n, hits, words, flags);
+        else go.next(trace_rays_kernel<true, false>, grid, block, smem, s->dev, rays, n, hits, words, flags);
     } else {
-        if (alpha) launch_next(trace_rays_kernel<false, true>, grid, block, instance_smem(s->dev), st, s->dev, rays, n, hits, words, flags);
-        else launch_next(trace_rays_kernel<false, false>, grid, block, instance_smem(s->dev), st, s->dev, rays, n, hits, words, flags);
+        if (alpha) go.next(trace_rays_kernel<false, true>, grid, block, smem, s->dev, rays, n, hits, words, flags);
+        else go.next(trace_rays_kernel<false, false>, grid, block, smem, s->dev, rays, n, hits, words, flags);
     }
-    launch_next(finish_hits_kernel, (n + TRACE_BLOCK - 1) / TRACE_BLOCK, block, 0, st, s->dev, rays, n, hits);
-    return cudaGetLastError();
+    // takes the triangle slots and instances that the first kernel left in the records
+    go.next(finish_hits_kernel, (n + TRACE_BLOCK - 1) / TRACE_BLOCK, block, 0, s->dev, rays, n, hits);
+    return go.status();
 }
 
 int run_trace(const lam_scene* s, cudaStream_t st, const char* who, TraceLaunch launch, const void* arg) {
@@ -496,10 +499,10 @@ int run_trace(const lam_scene* s, cudaStream_t st, const char* who, TraceLaunch 
         uint32_t* own = nullptr;
         cudaError_t e = cudaMallocAsync((void**)&own, 3 * sizeof(uint32_t), st);
         if (e != cudaSuccess) return cuda_error(e, who);
-        cudaMemsetAsync(own, 0, 3 * sizeof(uint32_t), st);
         uint32_t flags = 0;
-        e = launch(own, own + 2, arg);
-        if (e == cudaSuccess) cudaMemcpyAsync(&flags, own + 2, sizeof(flags), cudaMemcpyDeviceToHost, st);
+        e = cudaMemsetAsync(own, 0, 3 * sizeof(uint32_t), st);
+        if (e == cudaSuccess) e = launch(own, own + 2, arg);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&flags, own + 2, sizeof(flags), cudaMemcpyDeviceToHost, st);
         cudaFreeAsync(own, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return cuda_error(e, who);

@@ -1,0 +1,29 @@
+"""The host-side sequences of csrc/host_steps.h, compiled alone, with steps and allocations that fail."""
+import os
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "lambent_b200", "csrc")
+
+
+@pytest.fixture
+def run(tmp_path):
+    def compile_and_run(body):
+        src, exe = tmp_path / "t.cpp", tmp_path / "t"
+        src.write_text('#include <cstdio>\n#include <vector>\n#include "host_steps.h"\nusing namespace lam;\n'
+                       "int main() {\n" + body + "\n}\n")
+        subprocess.run(["g++", "-std=c++17", "-Wall", "-I", CSRC, "-o", str(exe), str(src)], check=True)
+        return subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
+    return compile_and_run
+
+
+@pytest.mark.parametrize("fails,taken,status", [(-1, "0123", 0), (0, "0", 7), (1, "01", 7), (3, "0123", 7)])
+def test_no_step_after_one_that_failed(run, fails, taken, status):
+    """A ray query's second kernel indexes triangles with what the first one wrote."""
+    out = run(f"""
+        enum Status {{ OK = 0, BAD = 7 }};
+        Steps<Status> go;
+        for (int k = 0; k < 4; ++k) go([&] {{ std::printf("%d", k); return k == {fails} ? BAD : OK; }});
+        std::printf(" %d", (int)go.status);""")
+    assert out == [taken, str(status)]
