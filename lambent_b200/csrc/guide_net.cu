@@ -684,9 +684,10 @@ static int guide_loss_grad(lam_guide* g, const float* recs, uint32_t n, const fl
     fill_args(g, recs, 13u, n, nullptr, batch, true, 1.0f / (float)n, box, A, U);
     U.grad = grad;
     U.loss = loss;
-    launch_next(net::guide_grad_kernel, U.parts, net::GRAD_THREADS, net::GRAD_SMEM, st, A);
-    launch_next(net::guide_sum_kernel, net::PARAMS / 256, 256, 0, st, U);
-    cudaError_t e = cudaGetLastError();
+    Launches go(st);
+    go.next(net::guide_grad_kernel, U.parts, net::GRAD_THREADS, net::GRAD_SMEM, A);
+    go.next(net::guide_sum_kernel, net::PARAMS / 256, 256, 0, U);
+    const cudaError_t e = go.status();
     if (e != cudaSuccess) return cuda_error(e, "guide gradient launch");
     return LAM_OK;
 }

@@ -1822,23 +1822,23 @@ int ensure_handler(lam_pipeline* pl) {
 }
 
 template <int Q>
-static void launch_guide(bool net, bool markov, int grid, cudaStream_t st, const Args& A) {
+static void launch_guide(bool net, bool markov, int grid, Launches& go, const Args& A) {
     if (markov) {
-        if (net) launch_next(guide_sample_kernel<Q, true, true>, grid, GUIDE_BLOCK, GUIDE_SMEM, st, A);
-        else launch_next(guide_sample_kernel<Q, false, true>, grid, WAVE_BLOCK, 0, st, A);
+        if (net) go.next(guide_sample_kernel<Q, true, true>, grid, GUIDE_BLOCK, GUIDE_SMEM, A);
+        else go.next(guide_sample_kernel<Q, false, true>, grid, WAVE_BLOCK, 0, A);
     } else {
-        if (net) launch_next(guide_sample_kernel<Q, true, false>, grid, GUIDE_BLOCK, GUIDE_SMEM, st, A);
-        else launch_next(guide_sample_kernel<Q, false, false>, grid, WAVE_BLOCK, 0, st, A);
+        if (net) go.next(guide_sample_kernel<Q, true, false>, grid, GUIDE_BLOCK, GUIDE_SMEM, A);
+        else go.next(guide_sample_kernel<Q, false, false>, grid, WAVE_BLOCK, 0, A);
     }
 }
 
 template <int Q>
-static void launch_shade(bool guide, bool learned, dim3 g, dim3 b, cudaStream_t st, const Args& A) {
-    if (guide && learned) launch_next(shade_kernel<Q, true, true, false>, g, b, GUIDE_SHADE_SMEM, st, A);
-    else if (guide) launch_next(shade_kernel<Q, true, false, false>, g, b, GUIDE_SHADE_SMEM, st, A);
-    else if (learned) launch_next(shade_kernel<Q, false, true, false>, g, b, 0, st, A);
-    else if (A.ort) launch_next(shade_kernel<Q, false, false, false, true>, g, b, 0, st, A);
-    else launch_next(shade_kernel<Q, false, false, false>, g, b, 0, st, A);
+static void launch_shade(bool guide, bool learned, dim3 g, dim3 b, Launches& go, const Args& A) {
+    if (guide && learned) go.next(shade_kernel<Q, true, true, false>, g, b, GUIDE_SHADE_SMEM, A);
+    else if (guide) go.next(shade_kernel<Q, true, false, false>, g, b, GUIDE_SHADE_SMEM, A);
+    else if (learned) go.next(shade_kernel<Q, false, true, false>, g, b, 0, A);
+    else if (A.ort) go.next(shade_kernel<Q, false, false, false, true>, g, b, 0, A);
+    else go.next(shade_kernel<Q, false, false, false>, g, b, 0, A);
 }
 
 
@@ -2253,6 +2253,9 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
     auto end = [&](int h) {
         if (h >= 0) cudaEventRecord(pl->timed[h].end, st);
     };
+    // the counters that one kernel leaves bound the next one's queue, and hits index the scene: after a launch
+    // that failed, none of them is this frame's
+    Launches go(st);
     for (uint32_t first = 0; first < pl->opts.samples;) {
         // learned guiding: record training vertices while the guide has seen fewer than train_spp
         // samples per pixel; sample the network once it has taken a training step
@@ -2285,7 +2288,7 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
         A.guide_frac = use_net ? gd->opts.guide_fraction : 0.0f;
         A.first = guide ? 0u : 1u;
         int h = begin(0);
-        launch_next(generate_kernel, gpix, blk, 0, st, A);
+        go.next(generate_kernel, gpix, blk, 0, A);
         end(h);
         ++launches;
         for (uint32_t depth = 0; depth < pl->opts.max_depth; ++depth) {
@@ -2306,30 +2309,32 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
             h = begin(1);
             if (proc) {
                 void* kargs[] = {&A};
-                cudaLaunchKernel((const void*)pl->handler->extend, dim3(w->grid_extend), blk, kargs, instance_smem(A.S), st);
+                go.steps([&] {
+                    return cudaLaunchKernel((const void*)pl->handler->extend, dim3(w->grid_extend), blk, kargs, instance_smem(A.S), st);
+                });
             } else if (alpha) {
-                launch_next(extend_kernel<true>, w->grid_extend, blk, instance_smem(A.S), st, A);
+                go.next(extend_kernel<true>, w->grid_extend, blk, instance_smem(A.S), A);
             } else {
-                launch_next(extend_kernel<false>, w->grid_extend, blk, instance_smem(A.S), st, A);
+                go.next(extend_kernel<false>, w->grid_extend, blk, instance_smem(A.S), A);
             }
             end(h);
             h = begin(2);
             if (sorted) {
-                launch_next(shade_order_kernel<false>, w->grid_sort, blk, 0, st, A);
+                go.next(shade_order_kernel<false>, w->grid_sort, blk, 0, A);
                 ++launches;
             }
             switch (pl->quality) {
-                case LAM_QUALITY_LOW: launch_shade<LAM_QUALITY_LOW>(guide, learned, w->grid_shade, blk, st, A); break;
-                case LAM_QUALITY_HIGH: launch_shade<LAM_QUALITY_HIGH>(guide, learned, w->grid_shade, blk, st, A); break;
-                default: launch_shade<LAM_QUALITY_MEDIUM>(guide, learned, w->grid_shade, blk, st, A); break;
+                case LAM_QUALITY_LOW: launch_shade<LAM_QUALITY_LOW>(guide, learned, w->grid_shade, blk, go, A); break;
+                case LAM_QUALITY_HIGH: launch_shade<LAM_QUALITY_HIGH>(guide, learned, w->grid_shade, blk, go, A); break;
+                default: launch_shade<LAM_QUALITY_MEDIUM>(guide, learned, w->grid_shade, blk, go, A); break;
             }
             launches += 2;
             if (gd) {
                 const int gg = use_net ? w->grid_guide : w->grid_shade;
                 switch (pl->quality) {
-                    case LAM_QUALITY_LOW: launch_guide<LAM_QUALITY_LOW>(use_net, guide, gg, st, A); break;
-                    case LAM_QUALITY_HIGH: launch_guide<LAM_QUALITY_HIGH>(use_net, guide, gg, st, A); break;
-                    default: launch_guide<LAM_QUALITY_MEDIUM>(use_net, guide, gg, st, A); break;
+                    case LAM_QUALITY_LOW: launch_guide<LAM_QUALITY_LOW>(use_net, guide, gg, go, A); break;
+                    case LAM_QUALITY_HIGH: launch_guide<LAM_QUALITY_HIGH>(use_net, guide, gg, go, A); break;
+                    default: launch_guide<LAM_QUALITY_MEDIUM>(use_net, guide, gg, go, A); break;
                 }
                 ++launches;
             }
@@ -2343,13 +2348,14 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
         }
         h = begin(3);
         if (guide) {
-            launch_next(shuffle_kernel, gpix, blk, 0, st, A);
+            go.next(shuffle_kernel, gpix, blk, 0, A);
             ++launches;
         }
         const uint32_t last = first + A.wave_count >= pl->opts.samples ? 1u : 0u;
-        launch_next(accumulate_kernel<0>, gpix, blk, 0, st, A, last);
+        go.next(accumulate_kernel<0>, gpix, blk, 0, A, last);
         end(h);
         ++launches;
+        if (go.status() != cudaSuccess) return cuda_error(go.status(), "lam_render launch");
         if (training) {
             h = begin(4);
             rc = guide_train(gd, gd->records, GUIDE_RECORD_STRIDE, gd->opts.record_capacity, w->ctr + CTR_RECORDS,
@@ -2631,8 +2637,9 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
     }
     const dim3 blk(WAVE_BLOCK);
     uint32_t launches = 0;
+    Launches go(st);  // as in lam_render
     auto record = [&]() {
-        launch_next(batch_start_kernel, 1, 256, 0, st, w->ctr, b->done, b->times, n);
+        go.next(batch_start_kernel, 1, 256, 0, w->ctr, b->done, b->times, n);
         for (size_t wv = 0; wv < P.wave_begin.size(); ++wv) {
             A.segs = b->segs + P.wave_begin[wv];
             A.nsegs = P.wave_nsegs[wv];
@@ -2650,7 +2657,7 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
             A.qacc = aca;
             A.qmisc = mia;
             const dim3 gp((A.pix_threads + WAVE_BLOCK - 1) / WAVE_BLOCK);
-            launch_next(batch_generate_kernel, gp, blk, 0, st, A);
+            go.next(batch_generate_kernel, gp, blk, 0, A);
             for (uint32_t depth = 0; depth < pl->opts.max_depth; ++depth) {
                 A.q_in = qa;
                 A.q_out = qb;
@@ -2665,26 +2672,26 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
                 A.qthr_out = thb;
                 A.qacc_out = acb;
                 A.qmisc_out = mib;
-                if (all_opaque) launch_next(extend_batch_kernel<false>, grid_e, blk, 0, st, A);
-                else launch_next(extend_batch_kernel<true>, grid_e, blk, 0, st, A);
+                if (all_opaque) go.next(extend_batch_kernel<false>, grid_e, blk, 0, A);
+                else go.next(extend_batch_kernel<true>, grid_e, blk, 0, A);
                 if (sorted) {
-                    launch_next(shade_order_kernel<true>, grid_sort, blk, 0, st, A);
+                    go.next(shade_order_kernel<true>, grid_sort, blk, 0, A);
                     ++launches;
                 }
                 switch (pl->quality) {
-                    case LAM_QUALITY_LOW: launch_next(shade_kernel<LAM_QUALITY_LOW, false, false, true>, grid_s, blk, 0, st, A); break;
-                    case LAM_QUALITY_HIGH: launch_next(shade_kernel<LAM_QUALITY_HIGH, false, false, true>, grid_s, blk, 0, st, A); break;
-                    default: launch_next(shade_kernel<LAM_QUALITY_MEDIUM, false, false, true>, grid_s, blk, 0, st, A); break;
+                    case LAM_QUALITY_LOW: go.next(shade_kernel<LAM_QUALITY_LOW, false, false, true>, grid_s, blk, 0, A); break;
+                    case LAM_QUALITY_HIGH: go.next(shade_kernel<LAM_QUALITY_HIGH, false, false, true>, grid_s, blk, 0, A); break;
+                    default: go.next(shade_kernel<LAM_QUALITY_MEDIUM, false, false, true>, grid_s, blk, 0, A); break;
                 }
                 launches += 2;
                 std::swap(qa, qb);
-                    std::swap(rao, rbo);
+                std::swap(rao, rbo);
                 std::swap(rad, rbd);
                 std::swap(tha, thb);
                 std::swap(aca, acb);
                 std::swap(mia, mib);
             }
-            launch_next(batch_accumulate_kernel, gp, blk, 0, st, A);
+            go.next(batch_accumulate_kernel, gp, blk, 0, A);
             launches += 2;
         }
     };
@@ -2699,6 +2706,7 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
             if (e != cudaSuccess) return cuda_error(e, "lam_batch_render capture");
             record();
             e = cudaStreamEndCapture(st, &g);
+            if (go.status() != cudaSuccess) e = go.status();
             if (e == cudaSuccess) e = cudaGraphInstantiate(&b->graph, g, 0);
             if (g) cudaGraphDestroy(g);
             if (e != cudaSuccess) return cuda_error(e, "lam_batch_render graph");
@@ -2711,7 +2719,8 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
     }
     cudaEventRecord(b->ev_out, st);
     cudaStreamWaitEvent(caller, b->ev_out, 0);
-    e = cudaGetLastError();
+    e = go.status();
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(e, "lam_batch_render launch");
     pl->stats.samples = 0;
     for (uint32_t i = 0; i < n; ++i) pl->stats.samples += (uint64_t)reqs[i].targets.width * reqs[i].targets.height * reqs[i].samples;
