@@ -1,5 +1,6 @@
 // host_steps.h - host-side sequences whose failure paths matter, in plain C++ (tested without a device).
 #pragma once
+#include <cstddef>
 
 namespace lam {
 
@@ -13,5 +14,16 @@ struct Steps {
         if (status == Status{}) status = step();
     }
 };
+
+// Two arrays of `count` that are only ever there together: one allocation, so that none is left without
+// the other when memory runs out.  `alloc(T**, n)` returns 0 on success.
+template <class T, class Alloc>
+int alloc_pair(T** a, T** b, size_t count, Alloc alloc) {
+    T* both = nullptr;
+    if (const int rc = alloc(&both, 2 * count)) return rc;
+    *a = both;
+    *b = both + count;
+    return 0;
+}
 
 }  // namespace lam

@@ -1794,10 +1794,8 @@ static int ensure_wave(lam_pipeline* pl, uint32_t width, uint32_t height, bool f
 }
 
 static int ensure_order(WaveBuffers* w, size_t paths) {
-    if (w->order_a && w->order_b) return LAM_OK;
-    if ((!w->order_a && walloc(w, &w->order_a, paths)) || (!w->order_b && walloc(w, &w->order_b, paths)))
-        return LAM_ERR_CUDA;
-    return LAM_OK;
+    if (w->order_a) return LAM_OK;
+    return alloc_pair(&w->order_a, &w->order_b, paths, [&](uint32_t** p, size_t n) { return walloc(w, p, n); });
 }
 
 // The counters of one bounce.
@@ -2198,8 +2196,9 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
     const bool proc = s->dev.has_procedural && !pl->handler_cubin.empty();
     if (proc) {
         if ((rc = ensure_handler(pl))) return rc;
-        if (!w->phit_a && (walloc(w, &w->phit_a, w->paths) || walloc(w, &w->phit_b, w->paths)))
-            return LAM_ERR_CUDA;
+        if (!w->phit_a && (rc = alloc_pair(&w->phit_a, &w->phit_b, w->paths,
+                                           [&](float4** p, size_t n) { return walloc(w, p, n); })))
+            return rc;
         A.phit_a = w->phit_a;
         A.phit_b = w->phit_b;
     }

@@ -27,3 +27,19 @@ def test_no_step_after_one_that_failed(run, fails, taken, status):
         for (int k = 0; k < 4; ++k) go([&] {{ std::printf("%d", k); return k == {fails} ? BAD : OK; }});
         std::printf(" %d", (int)go.status);""")
     assert out == [taken, str(status)]
+
+
+@pytest.mark.parametrize("room,want", [(0, "3 1 1"), (15, "3 1 1"), (16, "0 0 0")])
+def test_a_pair_is_allocated_whole_or_not_at_all(run, room, want):
+    """The class order's two lists: with one of them alone, the next batch wrote through the other."""
+    out = run(f"""
+        std::vector<int> store(16);
+        int *a = nullptr, *b = nullptr;
+        int rc = alloc_pair(&a, &b, 8, [&](int** p, size_t n) {{
+            if (n > {room}) return 3;
+            *p = store.data();
+            return 0;
+        }});
+        std::printf("%d %d %d", rc, a == nullptr, b == nullptr);
+        return a && b != a + 8;""")
+    assert " ".join(out) == want
