@@ -2501,8 +2501,11 @@ static int batch_wave_buffers(BatchState* b, uint32_t capacity, bool order) {
     return LAM_OK;
 }
 
+// What the launches of a batch depend on.  A request names its scene by address, where another scene may be by
+// the next call; of the scenes themselves, whose tables are uploaded for each call, the launches take only
+// whether all geometry is opaque.
 static void batch_key(const lam_batch_request* r, uint32_t n, const lam_batch_tuning& t, uint64_t generation,
-                      bool sorted, std::vector<char>& key) {
+                      bool sorted, bool all_opaque, std::vector<char>& key) {
     const size_t base = sizeof(uint32_t) + n * sizeof(lam_batch_request) + sizeof(t) + sizeof(generation);
     key.resize(base + 1);
     char* k = key.data();
@@ -2510,7 +2513,7 @@ static void batch_key(const lam_batch_request* r, uint32_t n, const lam_batch_tu
     std::memcpy(k + sizeof(n), r, n * sizeof(lam_batch_request));
     std::memcpy(k + sizeof(n) + n * sizeof(lam_batch_request), &t, sizeof(t));
     std::memcpy(k + sizeof(n) + n * sizeof(lam_batch_request) + sizeof(t), &generation, sizeof(generation));
-    k[base] = sorted ? 1 : 0;
+    k[base] = (char)((sorted ? 1 : 0) | (all_opaque ? 2 : 0));
 }
 
 }  // namespace lam
@@ -2696,7 +2699,7 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
     };
     if (t.use_graph) {
         std::vector<char> key;
-        batch_key(reqs, n, t, b->generation, sorted, key);
+        batch_key(reqs, n, t, b->generation, sorted, all_opaque, key);
         if (!b->graph || key != b->graph_key) {
             if (b->graph) cudaGraphExecDestroy(b->graph);
             b->graph = nullptr;
