@@ -2574,7 +2574,7 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
         b->generation++;  // a captured graph does not know the new buffers
         if ((rc = ensure_order(w, b->capacity))) return rc;
     }
-    // device tables (uploaded before any capture)
+    // device tables and pools
     if (dgrow(b, &b->reqs, &b->reqs_cap, n) || dgrow(b, &b->segs, &b->segs_cap, P.segs.size()) ||
         dgrow(b, &b->done, &b->done_cap, n) || dgrow(b, &b->times, &b->times_cap, n + 1) ||
         dgrow(b, &b->pix_color, &b->pix_cap, P.pixels) || dgrow(b, &b->pixel_seed, &b->seed_cap, P.pixels))
@@ -2596,10 +2596,7 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
         q.out_normal = (float4*)r.targets.normal;
         q.out_albedo = (float4*)r.targets.albedo;
     }
-    cudaError_t e = cudaMemcpy(b->reqs, hr.data(), n * sizeof(BatchReq), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(b->segs, P.segs.data(), P.segs.size() * sizeof(BatchSeg), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return cuda_error(e, "lam_batch_render tables");
-    b->last_n = n;
+    cudaError_t e = cudaSuccess;
     if (!b->stream) {
         if ((e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking)) != cudaSuccess ||
             (e = cudaEventCreateWithFlags(&b->ev_in, cudaEventDisableTiming)) != cudaSuccess ||
@@ -2608,6 +2605,13 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
     }
     cudaStream_t caller = (cudaStream_t)stream;
     cudaStream_t st = b->stream;
+    // in the batch's stream: its last batch may still be reading the tables (the copies take the pageable
+    // source before they return)
+    e = cudaMemcpyAsync(b->reqs, hr.data(), n * sizeof(BatchReq), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(b->segs, P.segs.data(), P.segs.size() * sizeof(BatchSeg), cudaMemcpyHostToDevice, st);
+    if (e != cudaSuccess) return cuda_error(e, "lam_batch_render tables");
+    b->last_n = n;
     cudaEventRecord(b->ev_in, caller);
     cudaStreamWaitEvent(st, b->ev_in, 0);
 

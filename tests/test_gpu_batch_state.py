@@ -70,3 +70,24 @@ def test_graph_of_opaque_scenes_is_not_replayed_for_a_cutout_at_the_same_address
     second = render(cutouts[-1])
     assert torch.equal(second, _single(cutouts[-1], cutout, 2, 3))
     assert not torch.equal(first, second)
+
+
+@pytest.mark.parametrize("graph", [0, 1])
+def test_batches_issued_back_to_back(cuda, graph):
+    """Different requests with no wait between the calls: a batch's tables stay as they are until it
+    has run."""
+    import torch
+    s = [scenes.cornell_box(160, 120), scenes.textured_cornell(64, 48), scenes.occluded_cornell(33, 47)]
+    g = [lb.GpuScene(x) for x in s]
+    batches = [[(0, 16, 1), (1, 7, 2)], [(2, 3, 3)], [(1, 5, 4), (2, 2, 5), (0, 1, 6), (1, 1, 7)]] * 2
+    cols = [[torch.full((s[k].height, s[k].width, 4), -1.0, device="cuda") for k, _, _ in b] for b in batches]
+    pipe = _pipe()
+    torch.cuda.synchronize()
+    for b, out in zip(batches, cols):
+        pipe.batch_render([(g[k], s[k].camera, lb.targets_from(o), spp, seed) for (k, spp, seed), o in zip(b, out)],
+                          _abi.BatchTuning(wave_paths=64 * 1024, use_graph=graph))
+    torch.cuda.synchronize()
+    assert pipe.stats().error_flags == 0
+    for b, out in zip(batches, cols):
+        for (k, spp, seed), o in zip(b, out):
+            assert torch.equal(o, _single(g[k], s[k], spp, seed))
