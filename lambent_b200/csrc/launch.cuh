@@ -3,7 +3,9 @@
 // A kernel launched with launch_next may be set up, and its blocks started, as the previous kernel's last
 // blocks exit; its wait_previous() holds it until that kernel's results are complete and visible.  Every
 // kernel launched so calls it before it touches memory that another kernel writes or reads.  Without the
-// launch attribute, and after a kernel that was launched otherwise, it does nothing.
+// launch attribute, and after a kernel that was launched otherwise, it does nothing.  Such memory is read by
+// plain loads: the read-only path (__ldg, const __restrict__ parameters) is for what no kernel writes while
+// this one exists, and it exists while the previous one still writes.
 //
 // It trims the 2-3 us between dependent kernels: 128x128, 1 spp, 5 bounces 158 -> 133 us; 256x256, 16 spp, 8
 // bounces 1,417 -> 1,366.  Letting the next kernel start earlier, when all blocks of the previous one have

@@ -102,11 +102,10 @@ LAM_DEV uint32_t div_by(uint32_t x, uint64_t m) { return (uint32_t)__umul64hi(m,
 // a neighbour's four words are requested together.  With 8 neighbours at 1280x720: 219 -> 117 us, bound
 // by issue and the gathers' latency (56 registers; held to 48 or 40 for more warps: 139.6, 144 against
 // 136.6 us for both passes).
-__global__ void __launch_bounds__(PASS_BLOCK) spatial_kernel(const lam_reservoir* __restrict__ cur,
-                                                             const lam_info* __restrict__ info, uint32_t width,
+__global__ void __launch_bounds__(PASS_BLOCK) spatial_kernel(const lam_reservoir* cur, const lam_info* info, uint32_t width,
                                                              uint32_t height, uint32_t is_samples, uint32_t is_space,
                                                              uint64_t space_m, uint64_t max_m, uint32_t seed_offset,
-                                                             float4* __restrict__ out) {
+                                                             float4* out) {
     wait_previous();
     const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= width * height) return;

@@ -408,16 +408,14 @@ namespace lam {
 
 template <bool ANY, bool ALPHA>
 __global__ void __launch_bounds__(TRACE_BLOCK, ALPHA ? 6 : 7) trace_rays_kernel(const __grid_constant__ DevScene S,
-                                                                 const lam_ray* __restrict__ rays, uint32_t n,
-                                                                 lam_hit* __restrict__ hits,
-                                                                 uint32_t* __restrict__ counter,
-                                                                 uint32_t* __restrict__ err_out) {
+                                                                 const lam_ray* rays, uint32_t n, lam_hit* hits,
+                                                                 uint32_t* counter, uint32_t* err_out) {
     const DevInstance* in = stage_instances(S);  // the scene is no kernel's output
     wait_previous();
     uint32_t err = 0u;
     auto load = [&](uint32_t i, float3& o, float3& d, float& t0, float& t1) {
-        const float4 r0 = __ldg(reinterpret_cast<const float4*>(rays + i));
-        const float4 r1 = __ldg(reinterpret_cast<const float4*>(rays + i) + 1);
+        const float4* r = reinterpret_cast<const float4*>(rays + i);
+        const float4 r0 = r[0], r1 = r[1];
         o = make_float3(r0.x, r0.y, r0.z);
         d = make_float3(r1.x, r1.y, r1.z);
         t0 = r0.w;
@@ -436,8 +434,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, ALPHA ? 6 : 7) trace_rays_kernel(
 // FP64 re-evaluation of each hit's triangle.  Inside the traversal loop it ran for the one or two lanes
 // whose rays had finished, and its registers (96) cost two CTAs per SM: 4.2M rays 2,490 -> 1,890 us.
 __global__ void __launch_bounds__(TRACE_BLOCK) finish_hits_kernel(const __grid_constant__ DevScene S,
-                                                                  const lam_ray* __restrict__ rays, uint32_t n,
-                                                                  lam_hit* hits) {
+                                                                  const lam_ray* rays, uint32_t n, lam_hit* hits) {
     wait_previous();
     const uint32_t i = blockIdx.x * TRACE_BLOCK + threadIdx.x;
     if (i >= n) return;
@@ -449,8 +446,8 @@ __global__ void __launch_bounds__(TRACE_BLOCK) finish_hits_kernel(const __grid_c
         h.instance_index = NO_HIT;
         h.kind = LAM_HIT_NONE;
     } else {
-        const float4 r0 = __ldg(reinterpret_cast<const float4*>(rays + i));
-        const float4 r1 = __ldg(reinterpret_cast<const float4*>(rays + i) + 1);
+        const float4* r = reinterpret_cast<const float4*>(rays + i);
+        const float4 r0 = r[0], r1 = r[1];
         float m[12];
         for (int q = 0; q < 12; ++q) m[q] = S.inst[inst].inv[q];
         float3 oo, od;

@@ -22,3 +22,25 @@ def test_kernels_that_read_one_another_are_launched_in_a_chain(name):
     assert "launch_next(" not in text
     assert "<<<" not in text
     assert ".next(" in text
+
+
+def functions(text):
+    """(signature, body) of every kernel definition."""
+    for m in re.finditer(r"__global__ void[^{;]*\{", text):
+        depth, k = 1, m.end()
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[k], 0)
+            k += 1
+        yield m.group(0), text[m.end():k]
+
+
+@pytest.mark.parametrize("name", sorted(f for f in os.listdir(CSRC) if f.endswith(".cu")))
+def test_dependent_kernels_read_other_kernels_output_by_plain_loads(name):
+    """A kernel that waits for the previous one exists while that one writes, so what it reads is not
+    read-only for its lifetime: no const __restrict__ parameter, and __ldg for the scene alone."""
+    for head, body in functions(source(name)):
+        if "wait_previous()" not in body:
+            continue
+        assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", head), head
+        for arg in re.findall(r"__ldg\(([^;]*)", body):
+            assert re.match(r"(tp\b|S[.\[]|reinterpret_cast<const uint32_t\*>\(S\[q\]->materials)", arg), (head, arg)
