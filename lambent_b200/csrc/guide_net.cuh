@@ -133,6 +133,10 @@ LAM_DEV bool group_or(uint32_t g, bool flag) {
     return r != 0u;
 }
 
+// Barrier of a block of two threads per row of a tile, which its halves reach at different calls (a
+// __syncthreads must be the same one for all threads of the block).
+LAM_DEV void halves_meet() { asm volatile("barrier.cta.sync 1, %0;" ::"n"(2 * TILE) : "memory"); }
+
 // 32 lanes x 16 consecutive f32 columns: this thread's row, columns [col, col + 16).  The wait is in
 // the same statement so that no use of the registers can be scheduled before the load completes.
 LAM_DEV void tmem_ld16(uint32_t taddr, float* v) {
@@ -344,7 +348,7 @@ LAM_DEV v3 mixture_sample(const Lobes& L, float u0, float u1, float u2) {
 
 // Gradient of  scale * (-weight * log q(w))  with respect to the 40 head outputs; returns the loss term.
 // Two threads share a row, HALF = 0 or 1 of its lobes each (1,500 instructions of one warp per scheduler
-// otherwise): the lobes' log terms meet in `terms` (LOBES floats of the row) at a barrier of the block,
+// otherwise): the lobes' log terms meet in `terms` (LOBES floats of the row) at a barrier of the two,
 // the mixture sums are formed by both, in lobe order.  g: outputs 8 k + 4 HALF + 0..3 as g[4 k + 0..3].
 template <int HALF>
 LAM_DEV float head_grad(const float* raw, v3 w, float weight, float scale, float* terms, float* g) {
@@ -357,7 +361,7 @@ LAM_DEV float head_grad(const float* raw, v3 w, float weight, float scale, float
         lf[j] = __logf(fmaxf(L.pi[j], 1e-30f)) + vmf_log_pdf(L.kappa[j], dot(L.mu[j], w));
         terms[j] = lf[j];
     }
-    __syncthreads();
+    halves_meet();
 #pragma unroll
     for (int j = 0; j < LOBES; ++j) {
         lf[j] = terms[j];

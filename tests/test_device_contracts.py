@@ -44,3 +44,12 @@ def test_dependent_kernels_read_other_kernels_output_by_plain_loads(name):
         assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", head), head
         for arg in re.findall(r"__ldg\(([^;]*)", body):
             assert re.match(r"(tp\b|S[.\[]|reinterpret_cast<const uint32_t\*>\(S\[q\]->materials)", arg), (head, arg)
+
+
+def test_block_barriers_are_not_in_functions_that_halves_of_a_block_call_apart():
+    """head_grad<0> and head_grad<1> run at once in the two halves of a block: __syncthreads in one
+    and __syncthreads in the other are different barriers to the language."""
+    text = source("guide_net.cuh")
+    body = text[text.index("float head_grad("):]
+    body = body[:body.index("\n}")]
+    assert "__syncthreads" not in body and "halves_meet();" in body
