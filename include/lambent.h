@@ -602,14 +602,17 @@ int lam_guide_loss_grad(lam_guide* guide, const lam_guide_record* records, uint3
 /* steps Adam steps on minibatches of options.batch records drawn from the n device records. */
 int lam_guide_train(lam_guide* guide, const lam_guide_record* records, uint32_t n, uint32_t steps,
                     const float box[6], void* stream);
-/* Number of Adam steps taken and samples per pixel trained so far.  Also reports, once, a
- * tensor-core completion wait of the guide's kernels that gave up: LAM_ERR_DEVICE_TIMEOUT. */
+/* Number of Adam steps asked for and samples per pixel trained so far.  Also reports, once, a
+ * tensor-core completion wait of the guide's kernels, or a wait of the training kernel's thread blocks
+ * for one another, that gave up: LAM_ERR_DEVICE_TIMEOUT. */
 int lam_guide_progress(const lam_guide* guide, uint64_t* steps, uint32_t* trained_spp);
 /* Bounded device waits: the polls of an mbarrier that the guide's tensor-core kernels
  * (lam_guide_eval, lam_guide_loss_grad, lam_guide_train) make before a wait gives up (default 2^20).
  * A CTA whose wait gives up lets its MMAs in flight finish, frees its tensor memory, records the
- * timeout and returns; its outputs are then undefined.  0 makes every wait give up at once, which
- * exercises that path without a stalled device. */
+ * timeout and returns; its outputs are then undefined.  Training takes each Adam step as a whole or not
+ * at all: after a wait that gave up, that step and the others of its launch (at most 64) are left out.
+ * Its thread blocks poll for one another 4 times as often as the limit, 64 times until all have started.
+ * 0 makes every wait give up at once, which exercises that path without a stalled device. */
 int lam_guide_set_wait_limit(lam_guide* guide, uint32_t tries);
 /* Attaches the guide used by lam_render when guide_mode is LAM_GUIDE_LEARNED (NULL detaches). */
 int lam_pipeline_set_guide(lam_pipeline* pipeline, lam_guide* guide);

@@ -20,7 +20,7 @@
 namespace lam {
 namespace net {
 
-constexpr uint32_t ERR_MMA_TIMEOUT = 1u << 8;
+constexpr uint32_t ERR_MMA_TIMEOUT = 1u << 8, ERR_MEETING_TIMEOUT = 1u << 9;
 // Evaluation: two warpgroups per CTA share the weights; each runs pairs of tiles, tile B's MMAs under tile
 // A's epilogue, with its own tiles, barriers and 128 TMEM columns (as the render's sampling kernel does).
 constexpr uint32_t EVAL_GROUPS = 2u, EVAL_THREADS = EVAL_GROUPS * TILE;
@@ -474,29 +474,53 @@ __global__ void guide_sum_kernel(UpdateArgs A) {
     A.grad[p] = trainable(l, o) ? g : 0.0f;
 }
 
-// All CTAs of the (cooperatively launched) grid meet: the k-th call waits for (k + 1) * gridDim arrivals.
-// Bounded: false, on every thread of the CTA, once the wait has given up.
-constexpr uint32_t GRID_TRIES = 1u << 22;
-LAM_DEV void grid_arrive(uint32_t* count) {
+// Meetings of all CTAs of the (cooperatively launched) grid, in one word: the arrivals at all meetings so
+// far and, above them, 0 or 1 + the meeting that was given up.  A meeting takes place for all CTAs or for
+// none, so that an Adam step is taken by all or by none: it is off once that is written before the last
+// arrival, and a CTA that stopped waiting, or that cannot go on, writes it by an exchange that fails if
+// anyone arrived in between.
+enum : uint32_t { MEET_OPEN, MEET_MET, MEET_OFF };
+LAM_DEV unsigned long long meet_load(const unsigned long long* word) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(word) : "memory");
+    return v;
+}
+LAM_DEV uint32_t meet_state(unsigned long long v, uint32_t k) {
+    const uint32_t off = (uint32_t)(v >> 32);  // a meeting after k that is off: all were at k
+    if (off) return off - 1u > k ? MEET_MET : MEET_OFF;
+    return (uint32_t)v >= (k + 1u) * gridDim.x ? MEET_MET : MEET_OPEN;
+}
+// Calls meeting k off unless it has taken place; by one thread.  Each exchange that fails follows another
+// CTA's arrival or its giving up, at most gridDim.x of them.
+LAM_DEV uint32_t meet_give_up(unsigned long long* word, uint32_t k) {
+    unsigned long long v = meet_load(word);
+    for (uint32_t t = 0; t <= gridDim.x && meet_state(v, k) == MEET_OPEN; ++t) {
+        const unsigned long long off = v | ((unsigned long long)(k + 1u) << 32);
+        const unsigned long long seen = atomicCAS(word, v, off);
+        v = seen == v ? off : seen;
+    }
+    return meet_state(v, k);
+}
+LAM_DEV void grid_arrive(unsigned long long* word) {
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        atomicAdd(count, 1u);
+        atomicAdd(word, 1ull);
     }
 }
-LAM_DEV bool grid_wait(const uint32_t* count, uint32_t k) {
-    uint32_t ok = 1u;
+// Waits, at most `tries` polls, for the others to arrive at meeting k; false on every thread if it is off.
+LAM_DEV bool grid_wait(unsigned long long* word, uint32_t k, uint32_t tries, uint32_t* err) {
+    uint32_t state = MEET_MET;
     if (threadIdx.x == 0) {
-        const uint32_t target = (k + 1u) * gridDim.x;
-        ok = 0u;
-        for (uint32_t t = 0; t < GRID_TRIES && !ok; ++t) {
-            uint32_t v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
-            ok = v >= target;
+        state = MEET_OPEN;
+        for (uint32_t t = 0; t < tries && state == MEET_OPEN; ++t) state = meet_state(meet_load(word), k);
+        if (state == MEET_OPEN) {
+            state = meet_give_up(word, k);
+            if (state != MEET_MET) atomicOr(err, ERR_MEETING_TIMEOUT);
         }
         __threadfence();
     }
-    return __syncthreads_and(ok != 0u) != 0;
+    return __syncthreads_and(state == MEET_MET ? 1 : 0) != 0;
 }
 
 // Adam steps A.step .. A.step + steps - 1 in one launch.  Per step a CTA runs its tiles and writes its
@@ -511,7 +535,9 @@ struct TrainArgs {
     GradArgs g;
     UpdateArgs u;
     uint32_t steps;
-    uint32_t* count;  // arrivals, zero at launch
+    unsigned long long* meet;  // zero at launch
+    // polls of a meeting; the first one also waits for CTAs that cannot start while other kernels hold their SMs
+    uint32_t meet_tries, start_tries;
     float lr[TRAIN_STEPS];
 };
 __global__ void __launch_bounds__(GRAD_THREADS, 1) guide_train_kernel(const __grid_constant__ TrainArgs T) {
@@ -546,13 +572,16 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) guide_train_kernel(const __gr
         fence_before();
         c.failed = __syncthreads_or(c.failed ? 1 : 0) != 0;
         fence_after();
+        if (c.failed) {  // no CTA takes this step or another one of this launch
+            if (threadIdx.x == 0) meet_give_up(T.meet, 2u * s);
+            break;
+        }
         grad_write(c, A.partial + (size_t)blockIdx.x * PARAMS, any);
         fence_before();
-        // a CTA whose waits gave up keeps meeting the others, with partials of zero
-        grid_arrive(T.count);
+        grid_arrive(T.meet);
         const bool more = s + 1u < T.steps;
         // under the others' tails: the next step's records, and the state of this thread's first parameter
-        if (more && !c.failed) {
+        if (more) {
             R = grad_record(A, n, A.step + s + 1u, blockIdx.x);
             grad_encode(S, R, A.box);
         }
@@ -560,10 +589,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) guide_train_kernel(const __gr
         const bool mine = threadIdx.x < TILE && q0 < (uint32_t)PARAMS;
         AdamState x{0.0f, 0.0f, 0.0f};
         if (mine) x = adam_load(T.u, partial_param(q0));
-        if (!grid_wait(T.count, 2u * s)) {
-            c.failed = true;
-            break;
-        }
+        if (!grid_wait(T.meet, 2u * s, s ? T.meet_tries : T.start_tries, A.err)) break;
         // 128 parameters per CTA at the grid of a 16,384-record batch
         for (uint32_t q = q0; threadIdx.x < TILE && q < (uint32_t)PARAMS; q += gridDim.x * TILE) {
             const uint32_t p = partial_param(q);
@@ -571,11 +597,8 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) guide_train_kernel(const __gr
             adam_step(T.u, p, q == q0 ? x : adam_load(T.u, p), g, T.lr[s]);
         }
         if (!more) break;
-        grid_arrive(T.count);
-        if (!grid_wait(T.count, 2u * s + 1u)) {
-            c.failed = true;
-            break;
-        }
+        grid_arrive(T.meet);
+        if (!grid_wait(T.meet, 2u * s + 1u, T.meet_tries, A.err)) break;
     }
     grad_end(c, A.err);
 }
@@ -698,7 +721,10 @@ int guide_train(lam_guide* g, const float* recs, uint32_t stride, uint32_t n, co
     int rc = setup_kernels(g);
     if (rc) return rc;
     net::TrainArgs T;
-    T.count = g->err + 8;
+    T.meet = reinterpret_cast<unsigned long long*>(g->err + 8);
+    // a poll of a meeting is a load that goes to L2; at the default limit of 2^20, some 2 s and 30 s
+    T.meet_tries = (uint32_t)std::min<uint64_t>(0xFFFFFFFFull, (uint64_t)g->wait_tries * 4u);
+    T.start_tries = (uint32_t)std::min<uint64_t>(0xFFFFFFFFull, (uint64_t)g->wait_tries * 64u);
     while (steps) {
         T.steps = std::min(steps, net::TRAIN_STEPS);
         fill_args(g, recs, stride, n, n_dev, g->opts.batch, false, 1.0f / (float)g->opts.batch, box, T.g, T.u);
@@ -707,7 +733,7 @@ int guide_train(lam_guide* g, const float* recs, uint32_t stride, uint32_t n, co
             T.lr[k] = (float)(g->opts.learning_rate * std::sqrt(1.0 - std::pow((double)T.u.b2, t)) /
                               (1.0 - std::pow((double)T.u.b1, t)));
         }
-        cudaError_t e = cudaMemsetAsync(T.count, 0, sizeof(uint32_t), st);
+        cudaError_t e = cudaMemsetAsync(T.meet, 0, sizeof(*T.meet), st);
         if (e != cudaSuccess) return cuda_error(e, "guide training");
         void* args[] = {&T};
         // cooperative: the CTAs wait for one another (at most one per SM)
@@ -745,11 +771,13 @@ int guide_check_error(const lam_guide* g) {
     uint32_t h = 0;
     cudaError_t e = cudaMemcpy(&h, g->err, sizeof(h), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_error(e, "lam_guide error flags");
-    if (h & net::ERR_MMA_TIMEOUT) {
+    if (h & (net::ERR_MMA_TIMEOUT | net::ERR_MEETING_TIMEOUT)) {
         // reported once: the flags start clear again for the next kernels
         e = cudaMemset(g->err, 0, sizeof(h));
         if (e != cudaSuccess) return cuda_error(e, "lam_guide error flags");
-        return set_error(LAM_ERR_DEVICE_TIMEOUT, "guide network: a tensor-core completion wait gave up");
+        return set_error(LAM_ERR_DEVICE_TIMEOUT, h & net::ERR_MMA_TIMEOUT
+                                                     ? "guide network: a tensor-core completion wait gave up"
+                                                     : "guide training: the wait for the other thread blocks gave up");
     }
     return LAM_OK;
 }
