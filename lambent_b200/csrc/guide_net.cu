@@ -736,8 +736,14 @@ int guide_train(lam_guide* g, const float* recs, uint32_t stride, uint32_t n, co
         cudaError_t e = cudaMemsetAsync(T.meet, 0, sizeof(*T.meet), st);
         if (e != cudaSuccess) return cuda_error(e, "guide training");
         void* args[] = {&T};
-        // cooperative: the CTAs wait for one another (at most one per SM)
-        e = cudaLaunchCooperativeKernel((const void*)net::guide_train_kernel, dim3(T.u.parts), dim3(net::GRAD_THREADS), args, net::GRAD_SMEM, st);
+        // cooperative: the CTAs wait for one another (at most one per SM).  The kernel takes any grid; a smaller one
+        // adds the partials of fewer, longer CTAs.
+        e = launch_resident(T.u.parts, cudaErrorCooperativeLaunchTooLarge, [&](unsigned grid) {
+            const cudaError_t s = cudaLaunchCooperativeKernel((const void*)net::guide_train_kernel, dim3(grid),
+                                                              dim3(net::GRAD_THREADS), args, net::GRAD_SMEM, st);
+            if (s == cudaErrorCooperativeLaunchTooLarge) (void)cudaGetLastError();
+            return s;
+        });
         if (e != cudaSuccess) return cuda_error(e, "guide training launch");
         g->steps += T.steps;
         steps -= T.steps;

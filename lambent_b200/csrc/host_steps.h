@@ -26,4 +26,13 @@ int alloc_pair(T** a, T** b, size_t count, Alloc alloc) {
     return 0;
 }
 
+// Launches a grid whose blocks wait for one another with at most `grid` blocks: halved while the launch says
+// that so many are not resident together (a partition of the device holds fewer than the device).
+template <class Status, class Launch>
+Status launch_resident(unsigned grid, Status too_large, Launch launch) {
+    Status s = launch(grid);
+    while (s == too_large && grid > 1) s = launch(grid = (grid + 1) / 2);
+    return s;
+}
+
 }  // namespace lam

@@ -43,3 +43,17 @@ def test_a_pair_is_allocated_whole_or_not_at_all(run, room, want):
         std::printf("%d %d %d", rc, a == nullptr, b == nullptr);
         return a && b != a + 8;""")
     assert " ".join(out) == want
+
+
+@pytest.mark.parametrize("fits,tried,status", [(148, "148", 0), (147, "148,74", 0), (40, "148,74,37", 0),
+                                               (0, "148,74,37,19,10,5,3,2,1", 9), (-1, "148", 4)])
+def test_a_grid_that_must_be_resident_shrinks_to_fit(run, fits, tried, status):
+    """Training on a partition of the device with fewer multiprocessors; other errors (-1) stay."""
+    out = run(f"""
+        enum Status {{ OK = 0, OTHER = 4, TOO_LARGE = 9 }};
+        const Status s = launch_resident(148u, TOO_LARGE, [](unsigned grid) {{
+            std::printf(grid == 148 ? "%u" : ",%u", grid);
+            return {fits} < 0 ? OTHER : (int)grid <= {fits} ? OK : TOO_LARGE;
+        }});
+        std::printf(" %d", (int)s);""")
+    assert out == [tried, str(status)]
