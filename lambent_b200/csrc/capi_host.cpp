@@ -24,6 +24,7 @@ int set_error(int code, const std::string& msg) {
 }
 
 int cuda_error(cudaError_t e, const char* what) {
+    (void)cudaGetLastError();  // returned by this call, so not the next one's to find
     g_last_error = std::string(what) + ": " + cudaGetErrorString(e);
     return LAM_ERR_CUDA;
 }
