@@ -505,12 +505,21 @@ int run_trace(const lam_scene* s, cudaStream_t st, const char* who, TraceLaunch 
         if (e != cudaSuccess) return cuda_error(e, who);
         return flags & ERR_STACK_OVERFLOW ? set_error(LAM_ERR_STACK_OVERFLOW, "traversal stack overflow") : LAM_OK;
     }
+    // whether the stream is being captured, or is the legacy stream while another one is (then refused); the
+    // wait below fails in either
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const bool captured = cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone;
+    if (captured) (void)cudaGetLastError();
     volatile uint32_t* flags = s->trace_flags + slot;
     cudaError_t e = launch(s->trace_words + slot * TRACE_SLOT_WORDS, s->trace_flags_dev + slot, arg);
-    // also after a launch that failed: a kernel before it may run.  A wait that failed (a stream being captured)
-    // says nothing about the kernels: the slot stays taken
+    // also after a launch that failed: a kernel before it may run
     const cudaError_t wait = cudaStreamSynchronize(st);
-    if (wait != cudaSuccess) return cuda_error(e != cudaSuccess ? e : wait, who);
+    if (wait != cudaSuccess) {
+        // in a capture nothing of the call ran; after any other failed wait its kernels still may, and the slot
+        // stays taken
+        if (captured) s->trace_busy.fetch_and(~(1ull << slot), std::memory_order_release);
+        return cuda_error(e != cudaSuccess ? e : wait, who);
+    }
     const uint32_t got = *flags;
     *flags = 0u;
     s->trace_busy.fetch_and(~(1ull << slot), std::memory_order_release);

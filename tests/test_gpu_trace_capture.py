@@ -38,3 +38,29 @@ def test_an_error_that_was_returned_is_not_the_next_calls(cuda):
     torch.cuda.synchronize()
     captured_query(g, rays, hits, torch.cuda.Stream())
     assert (hits == -1).all()  # captured, not run
+
+
+def test_queries_refused_in_a_capture_keep_no_slot(cuda):
+    """With its 64 scratch slots taken, a scene's queries allocate from the device's memory pool."""
+    import torch
+    from cuda.bindings import driver
+    _, g, rays = box_and_rays(torch)
+    want, got = (torch.full((256, 6), -1, dtype=torch.int32, device="cuda") for _ in range(2))
+    g.trace(rays, want)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    for _ in range(70):
+        captured_query(g, rays, got, side)
+    torch.cuda.synchronize()
+    assert (got == -1).all()
+    err, pool = driver.cuDeviceGetDefaultMemPool(0)
+    assert err == driver.CUresult.CUDA_SUCCESS
+    attr = driver.CUmemPool_attribute.CU_MEMPOOL_ATTR_USED_MEM_HIGH
+    driver.cuMemPoolSetAttribute(pool, attr, driver.cuuint64_t(0))
+    for _ in range(4):
+        got.fill_(-1)
+        g.trace(rays, got)
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
+    err, high = driver.cuMemPoolGetAttribute(pool, attr)
+    assert err == driver.CUresult.CUDA_SUCCESS and int(high) == 0
