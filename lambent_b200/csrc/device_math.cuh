@@ -86,7 +86,7 @@ LAM_DEV uint32_t f2u(float f) {
 // a branch each, and a bounce has some twenty of them): q = x * (1 / c), then one correction by the
 // exact residual x - q * c (P. Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000 processor", IBM J. R&D 34, 1990).  Whether one correction rounds correctly depends on
-// c: checked against the IEEE quotient for every byte / 255 and every 24-bit mantissa / pi.
+// c: checked on the device against the IEEE quotient for every byte / 255 and every float / pi.
 LAM_DEV float byte_over_255(uint32_t b) {
     const float x = (float)b, rc = 1.0f / 255.0f;
     const float q = __fmul_rn(x, rc);
@@ -95,7 +95,8 @@ LAM_DEV float byte_over_255(uint32_t b) {
 
 constexpr float PI_F = 3.14159265358979323846f;
 LAM_DEV float over_pi(float x) {
-    if (!(fabsf(x) > 1.0e-30f)) return x / PI_F;  // zeros, NaN, and residuals that could be subnormal
+    // zeros, NaN, infinities (whose residual is NaN), and residuals that could be subnormal
+    if (!(fabsf(x) > 1.0e-30f && fabsf(x) < 1.0e30f)) return x / PI_F;
     const float rc = 1.0f / PI_F;
     const float q = __fmul_rn(x, rc);
     return __fmaf_rn(__fmaf_rn(-q, PI_F, x), rc, q);

@@ -104,12 +104,15 @@ LAM_DEV bool wbw_f32(const TriRay& r, float4 a, float4 b, float4 c, float limit,
 }
 
 // a / b rounded to nearest from b's rounded reciprocal: the quotient estimate is corrected twice by its
-// exact residual (P. Markstein, IBM J. R&D 34, 1990).  For a and b that came from f32, whose quotients
-// and residuals stay far inside the FP64 range; a zero keeps the sign that the first product gives.
+// exact residual (P. Markstein, IBM J. R&D 34, 1990).  For |a| <= |b| that came from f32, whose quotients
+// and residuals stay far inside the FP64 range; a zero keeps the sign that the first product gives, and so
+// does the zero over an infinite b, whose residual is taken with 0 for b (with b it would be NaN).
 LAM_DEV double quotient_f64(double a, double b, double rcp_b) {
+    const int hi = __double2hiint(b);
+    const double br = __hiloint2double((hi & 0x7FF00000) == 0x7FF00000 ? 0 : hi, __double2loint(b));
     const double q0 = __dmul_rn(a, rcp_b);
-    const double q1 = __fma_rn(__fma_rn(-b, q0, a), rcp_b, q0);
-    const double q2 = __fma_rn(__fma_rn(-b, q1, a), rcp_b, q1);
+    const double q1 = __fma_rn(__fma_rn(-br, q0, a), rcp_b, q0);
+    const double q2 = __fma_rn(__fma_rn(-br, q1, a), rcp_b, q1);
     return a == 0.0 ? q0 : q2;
 }
 
