@@ -9,6 +9,7 @@
 #include <cstring>
 #include <vector>
 
+#include "arena.h"
 #include "device_math.cuh"
 #include "guide.cuh"
 #include "launch.cuh"
@@ -234,29 +235,16 @@ static void free_blocks(std::vector<void*>& blocks) {
     blocks.clear();
 }
 
-// Cleared device memory for the buffers of `sizes`: one block, or an allocation each if none is over 1 MB
-// (the driver serves those from memory that it has mapped already).
-static int alloc_blocks(std::vector<void*>& blocks, void** const* buffers, const size_t* sizes, int n) {
-    size_t total = 0, largest = 0;
-    for (int k = 0; k < n; ++k) {
-        total += (sizes[k] + 255u) / 256u * 256u;
-        largest = std::max(largest, sizes[k]);
-    }
-    const bool single = largest <= (1u << 20);
-    char* at = nullptr;
-    for (int k = 0; k < n; ++k) {
-        if (single || k == 0) {
-            const size_t bytes = single ? sizes[k] : total;
-            cudaError_t e = cudaMalloc((void**)&at, bytes);
-            if (e != cudaSuccess) return cuda_error(e, "cudaMalloc (data buffers)");
-            blocks.push_back(at);
-            e = cudaMemset(at, 0, bytes);
-            if (e != cudaSuccess) return cuda_error(e, "cudaMemset (data buffers)");
-        }
-        *buffers[k] = at;
-        at += (sizes[k] + 255u) / 256u * 256u;
-    }
-    return LAM_OK;
+// Cleared device memory for what `layout` takes.
+template <class Layout>
+static int alloc_blocks(std::vector<void*>& blocks, Layout layout) {
+    return place([&](void** p, size_t bytes) {
+        cudaError_t e = cudaMalloc(p, bytes);
+        if (e != cudaSuccess) return cuda_error(e, "cudaMalloc (data buffers)");
+        blocks.push_back(*p);
+        e = cudaMemset(*p, 0, bytes);
+        return e == cudaSuccess ? (int)LAM_OK : cuda_error(e, "cudaMemset (data buffers)");
+    }, layout);
 }
 
 static void free_window(lam_data_buffers* b) {
@@ -272,10 +260,14 @@ static int alloc_window(lam_data_buffers* b, uint32_t w, uint32_t h) {
     // reservoirs are always per pixel: rt_main writes gi_reservoirs[idx] in every ReSTIR mode
     b->reservoir_len = pix;
     b->chain_len = (b->types & LAM_BUFFER_MARKOV_CHAIN_SCREEN_SPACE) ? pix : 1;
-    void** const buffers[] = {&b->reservoirs, &b->old_reservoirs, &b->info, &b->chains, &b->old_chains, &b->pixel_seed};
-    const size_t res = b->reservoir_len * sizeof(lam_reservoir), chain = b->chain_len * sizeof(lam_markov_chain);
-    const size_t sizes[] = {res, res, pix * sizeof(lam_info), chain, chain, pix * sizeof(uint32_t)};
-    return alloc_blocks(b->window, buffers, sizes, 6) ? LAM_ERR_CUDA : LAM_OK;
+    return alloc_blocks(b->window, [&](Arena& a) {
+        a.take((lam_reservoir**)&b->reservoirs, b->reservoir_len);
+        a.take((lam_reservoir**)&b->old_reservoirs, b->reservoir_len);
+        a.take((lam_info**)&b->info, pix);
+        a.take((lam_markov_chain**)&b->chains, b->chain_len);
+        a.take((lam_markov_chain**)&b->old_chains, b->chain_len);
+        a.take((uint32_t**)&b->pixel_seed, pix);
+    });
 }
 
 }  // namespace lam
@@ -294,9 +286,10 @@ extern "C" int lam_data_buffers_new(uint32_t width, uint32_t height, uint32_t wo
     b->world_len = (types & LAM_BUFFER_MARKOV_CHAIN_WORLD_SPACE) ? b->world_size : 1;
     int rc = alloc_window(b, width, height);
     if (!rc) {
-        void** const buffers[] = {&b->world, &b->old_world};
-        const size_t grid = b->world_len * sizeof(lam_world_markov_chain), sizes[] = {grid, grid};
-        rc = alloc_blocks(b->grids, buffers, sizes, 2);
+        rc = alloc_blocks(b->grids, [&](Arena& a) {
+            a.take((lam_world_markov_chain**)&b->world, b->world_len);
+            a.take((lam_world_markov_chain**)&b->old_world, b->world_len);
+        });
     }
     if (rc) {
         free_window(b);

@@ -13,6 +13,7 @@
 #include <cstring>
 #include <vector>
 
+#include "arena.h"
 #include "guide.cuh"
 #include "guide_net.cuh"
 #include "launch.cuh"
@@ -267,40 +268,11 @@ static int walloc(WaveBuffers* w, T** p, size_t count) {
     return LAM_OK;
 }
 
-// Lays arrays out in device memory: a first pass measures, a second one places them in one block.  An
-// allocation per array, some 25 of them, was most of a pipeline's first render: 8.5 -> 1.8 ms at 256x256 with
-// 16 spp, 13.7 -> 3.0 ms for a ReSTIR frame at 1080p.  Arrays of up to ARENA_SMALL bytes are allocated one by
-// one: the driver serves those from memory that it has mapped already.
-struct Arena {
-    WaveBuffers* w = nullptr;
-    char* base = nullptr;
-    size_t used = 0, largest = 0;
-    bool single = false;  // one allocation per array
-    int rc = LAM_OK;
-    template <class T>
-    void take(T** p, size_t count) {
-        if (single) {
-            rc |= walloc(w, p, count);
-            return;
-        }
-        *p = base && count ? reinterpret_cast<T*>(base + used) : nullptr;
-        used += (count * sizeof(T) + 255u) / 256u * 256u;
-        largest = std::max(largest, count * sizeof(T));
-    }
-};
-constexpr size_t ARENA_SMALL = 1u << 20;
-
-// Allocates what `layout` takes.
+// Allocates what `layout` takes.  An allocation per array, some 25 of them, was most of a pipeline's first
+// render: 8.5 -> 1.8 ms at 256x256 with 16 spp, 13.7 -> 3.0 ms for a ReSTIR frame at 1080p.
 template <class Layout>
 static int alloc_arena(WaveBuffers* w, Layout layout) {
-    Arena a;
-    a.w = w;
-    layout(a);
-    if (a.largest <= ARENA_SMALL) a.single = true;
-    else if (int rc = walloc(w, &a.base, a.used)) return rc;
-    a.used = 0;
-    layout(a);
-    return a.rc ? LAM_ERR_CUDA : LAM_OK;
+    return place([w](void** p, size_t bytes) { return walloc(w, reinterpret_cast<char**>(p), bytes); }, layout);
 }
 
 LAM_DEV void create_ray(const Args& A, uint32_t x, uint32_t y, v3* o, v3* d) {
