@@ -1571,11 +1571,6 @@ __global__ void shuffle_kernel(const __grid_constant__ Args A) {
     mc_store(A.tent_snap + p, t);
 }
 
-// Device bytes of wave state per path: rays of two queues (64), live state of two queues (96), hit (8), two
-// queue entries (8), radiance (16), class order (8); ReSTIR / Markov / learned-guide extras.
-constexpr uint64_t WAVE_BYTES_PER_PATH = 200, WAVE_BYTES_FULL = 96, WAVE_BYTES_GUIDE = 32, WAVE_BYTES_LEARNED = 136,
-                   WAVE_BYTES_THREE_WAY = 20 * MIX_LOBES;
-
 // Path state of P paths: what single and batched renders both keep.
 static void layout_paths(Arena& a, WaveBuffers* w, size_t P, bool order) {
     a.take(&w->ray_o, P);
@@ -1599,49 +1594,49 @@ static void layout_paths(Arena& a, WaveBuffers* w, size_t P, bool order) {
     }
 }
 
-static int alloc_wave(WaveBuffers* w, uint32_t npix, bool full, bool guide, bool learned, bool order) {
-    return alloc_arena(w, [&](Arena& a) {
-        const size_t P = w->paths;
-        layout_paths(a, w, P, order);
-        a.take(&w->pix_color, npix);
-        if (full) {
-            a.take(&w->ort, P);
-            a.take(&w->orad, P);
-            a.take(&w->ppoint, P);
-            a.take(&w->pnormal, P);
-            a.take(&w->vpoint, P);
-            a.take(&w->vnormal, P);
-            a.take(&w->pix_orad, npix);
-            a.take(&w->pix_emission, npix);
-            a.take(&w->pix_albedo, npix);
-        }
+// The wave of a single render.  A path takes 192 bytes (rays of two queues 64, live state of two queues 96, hit
+// 8, two queue entries 8, radiance 16), 8 in class order, and what the options add.
+static void layout_wave(Arena& a, WaveBuffers* w, uint32_t npix, bool full, bool guide, bool learned, bool order) {
+    const size_t P = w->paths;
+    layout_paths(a, w, P, order);
+    a.take(&w->pix_color, npix);
+    if (full) {
+        a.take(&w->ort, P);
+        a.take(&w->orad, P);
+        a.take(&w->ppoint, P);
+        a.take(&w->pnormal, P);
+        a.take(&w->vpoint, P);
+        a.take(&w->vnormal, P);
+        a.take(&w->pix_orad, npix);
+        a.take(&w->pix_emission, npix);
+        a.take(&w->pix_albedo, npix);
+    }
+    if (guide) {
+        a.take(&w->lnormal, P);
+        a.take(&w->ldir, P);
+        a.take(&w->tent_snap, npix);
+        a.take(&w->tent_live, npix);
+    }
+    if (learned) {
+        a.take(&w->thr, P);
+        a.take(&w->brdf, P);
+        a.take(&w->seed, P);
+        a.take(&w->flags, P);
+        a.take(&w->dq, P);
+        a.take(&w->def_n, P);
+        a.take(&w->def_t, P);
+        a.take(&w->def_c, P);
+        a.take(&w->def_o, P);
+        a.take(&w->def_d, P);
+        a.take(&w->def_a, P);
+        a.take(&w->rec_head, P);
+        a.take(&w->def_r, P);
+        a.take(&w->def_kind, P);
         if (guide) {
-            a.take(&w->lnormal, P);
-            a.take(&w->ldir, P);
-            a.take(&w->tent_snap, npix);
-            a.take(&w->tent_live, npix);
+            a.take(&w->def_lobe, P * MIX_LOBES);
+            a.take(&w->def_lw, P * MIX_LOBES);
         }
-        if (learned) {
-            a.take(&w->thr, P);
-            a.take(&w->brdf, P);
-            a.take(&w->seed, P);
-            a.take(&w->flags, P);
-            a.take(&w->dq, P);
-            a.take(&w->def_n, P);
-            a.take(&w->def_t, P);
-            a.take(&w->def_c, P);
-            a.take(&w->def_o, P);
-            a.take(&w->def_d, P);
-            a.take(&w->def_a, P);
-            a.take(&w->rec_head, P);
-            a.take(&w->def_r, P);
-            a.take(&w->def_kind, P);
-            if (guide) {
-                a.take(&w->def_lobe, P * MIX_LOBES);
-                a.take(&w->def_lw, P * MIX_LOBES);
-            }
-        }
-    });
+    }
 }
 
 // Whether a wave of `paths` is shaded in material order (lam_pipeline_set_shade_order): the automatic order
@@ -1672,11 +1667,16 @@ static int ensure_wave(lam_pipeline* pl, uint32_t width, uint32_t height, bool f
     bool capped = false;
     size_t free_b = 0, total_b = 0;
     if (spp_wave > 1 && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
-        const uint64_t per_path = WAVE_BYTES_PER_PATH + (full ? WAVE_BYTES_FULL : 0) + (guide ? WAVE_BYTES_GUIDE : 0) +
-                                  (learned ? WAVE_BYTES_LEARNED : 0) + (guide && learned ? WAVE_BYTES_THREE_WAY : 0);
-        const uint64_t fit = (uint64_t)(free_b / 2) / (per_path * std::max(1u, npix));
-        if (fit < spp_wave) {
-            spp_wave = (uint32_t)std::max<uint64_t>(1, fit);
+        const bool order = sorts(pl, guide, (uint64_t)npix * spp_wave);
+        auto bytes = [&](uint32_t samples) -> uint64_t {
+            WaveBuffers m;
+            m.paths = (uint64_t)npix * samples;
+            return arena_bytes([&](Arena& a) { layout_wave(a, &m, npix, full, guide, learned, order); });
+        };
+        const uint64_t room = free_b / 2, all = bytes(spp_wave);
+        if (all > room) {
+            const uint64_t one = bytes(1), more = std::max<uint64_t>(1, (all - one) / (spp_wave - 1u));
+            spp_wave = room > one ? (uint32_t)std::min<uint64_t>(spp_wave - 1u, 1u + (room - one) / more) : 1u;
             capped = true;
         }
     }
@@ -1690,7 +1690,8 @@ static int ensure_wave(lam_pipeline* pl, uint32_t width, uint32_t height, bool f
         w->full = full;
         w->guide = guide;
         w->learned = learned;
-        if (alloc_wave(w, npix, full, guide, learned, sorts(pl, guide, w->paths)) == LAM_OK) break;
+        const bool order = sorts(pl, guide, w->paths);
+        if (alloc_arena(w, [&](Arena& a) { layout_wave(a, w, npix, full, guide, learned, order); }) == LAM_OK) break;
         free_wave(w);
         if (spp_wave == 1) return LAM_ERR_CUDA;  // the failed allocation set the error message
         (void)cudaGetLastError();                // an out-of-memory error is not sticky
