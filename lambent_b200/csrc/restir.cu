@@ -252,22 +252,38 @@ static void free_window(lam_data_buffers* b) {
     b->reservoirs = b->old_reservoirs = b->info = b->chains = b->old_chains = b->pixel_seed = nullptr;
 }
 
-static int alloc_window(lam_data_buffers* b, uint32_t w, uint32_t h) {
+static void set_window(lam_data_buffers* b, uint32_t w, uint32_t h) {
     const size_t pix = (size_t)w * h;
     b->width = w;
     b->height = h;
     b->pixels = pix;
     // reservoirs are always per pixel: rt_main writes gi_reservoirs[idx] in every ReSTIR mode
     b->reservoir_len = pix;
-    b->chain_len = (b->types & LAM_BUFFER_MARKOV_CHAIN_SCREEN_SPACE) ? pix : 1;
-    return alloc_blocks(b->window, [&](Arena& a) {
+    b->chain_len = (b->types & LAM_BUFFER_MARKOV_CHAIN_SCREEN_SPACE) ? pix : std::min<size_t>(pix, 1);
+}
+
+// The buffers of a w x h window; where their memory is not to be had, those of an empty one, which no pass takes.
+static int alloc_window(lam_data_buffers* b, uint32_t w, uint32_t h) {
+    set_window(b, w, h);
+    const int rc = alloc_blocks(b->window, [&](Arena& a) {
         a.take((lam_reservoir**)&b->reservoirs, b->reservoir_len);
         a.take((lam_reservoir**)&b->old_reservoirs, b->reservoir_len);
-        a.take((lam_info**)&b->info, pix);
+        a.take((lam_info**)&b->info, b->pixels);
         a.take((lam_markov_chain**)&b->chains, b->chain_len);
         a.take((lam_markov_chain**)&b->old_chains, b->chain_len);
-        a.take((uint32_t**)&b->pixel_seed, pix);
+        a.take((uint32_t**)&b->pixel_seed, b->pixels);
     });
+    if (rc) {
+        free_window(b);
+        set_window(b, 0, 0);
+    }
+    return rc;
+}
+
+// What a pass over the buffers is refused for, or null.
+static const char* refused(const lam_data_buffers* b) {
+    if (!b) return "null buffers";
+    return b->pixels ? nullptr : "the buffers hold no window (a resize failed)";
 }
 
 }  // namespace lam
@@ -311,7 +327,7 @@ extern "C" int lam_data_buffers_resize(lam_data_buffers* b, uint32_t width, uint
 }
 
 extern "C" int lam_data_buffers_advance_frame(lam_data_buffers* b, uint32_t adv, uint32_t cap, void* stream) {
-    if (!b) return set_error(LAM_ERR_INVALID_ARGUMENT, "null buffers");
+    if (const char* why = refused(b)) return set_error(LAM_ERR_INVALID_ARGUMENT, why);
     if (cap == 0 || cap > 0xFFFF) return set_error(LAM_ERR_INVALID_ARGUMENT, "confidence_cap must be a NonZeroU16");
     cudaStream_t st = (cudaStream_t)stream;
     const size_t res_bytes = b->reservoir_len * sizeof(lam_reservoir);
@@ -371,7 +387,7 @@ extern "C" int lam_data_buffers_destroy(lam_data_buffers* b) {
 
 extern "C" int lam_temporal_resampling(lam_data_buffers* b, uint32_t width, uint32_t height, uint32_t seed_offset,
                                        void* stream) {
-    if (!b) return set_error(LAM_ERR_INVALID_ARGUMENT, "null buffers");
+    if (const char* why = refused(b)) return set_error(LAM_ERR_INVALID_ARGUMENT, why);
     if (width != b->width || height != b->height) return set_error(LAM_ERR_INVALID_ARGUMENT, "size differs from the buffers");
     uint32_t n = width * height;
     launch_next(temporal_kernel, (n + PASS_BLOCK - 1) / PASS_BLOCK, PASS_BLOCK, 0, (cudaStream_t)stream,
@@ -383,6 +399,7 @@ extern "C" int lam_temporal_resampling(lam_data_buffers* b, uint32_t width, uint
 extern "C" int lam_spatial_resampling(lam_data_buffers* b, const lam_frame_targets* tg, uint32_t is_samples,
                                       uint32_t is_space, uint32_t seed_offset, void* stream) {
     if (!b || !tg || !tg->color) return set_error(LAM_ERR_INVALID_ARGUMENT, "null argument");
+    if (const char* why = refused(b)) return set_error(LAM_ERR_INVALID_ARGUMENT, why);
     if (tg->width != b->width || tg->height != b->height) return set_error(LAM_ERR_INVALID_ARGUMENT, "size differs from the buffers");
     if (is_samples > 128) return set_error(LAM_ERR_INVALID_ARGUMENT, "IS_SAMPLES must be <= 128 (Q[129] in the reference)");
     if (is_space < 2) return set_error(LAM_ERR_INVALID_ARGUMENT, "IS_SPACE must be >= 2");
