@@ -235,16 +235,19 @@ static void free_blocks(std::vector<void*>& blocks) {
     blocks.clear();
 }
 
-// Cleared device memory for what `layout` takes.
+// Cleared device memory for what `layout` takes; the clears are waited for, since the passes run in any stream.
 template <class Layout>
 static int alloc_blocks(std::vector<void*>& blocks, Layout layout) {
-    return place([&](void** p, size_t bytes) {
+    const int rc = place([&](void** p, size_t bytes) {
         cudaError_t e = cudaMalloc(p, bytes);
         if (e != cudaSuccess) return cuda_error(e, "cudaMalloc (data buffers)");
         blocks.push_back(*p);
         e = cudaMemset(*p, 0, bytes);
         return e == cudaSuccess ? (int)LAM_OK : cuda_error(e, "cudaMemset (data buffers)");
     }, layout);
+    if (rc) return rc;
+    const cudaError_t e = cudaStreamSynchronize(cudaStreamLegacy);
+    return e == cudaSuccess ? LAM_OK : cuda_error(e, "clearing the data buffers");
 }
 
 static void free_window(lam_data_buffers* b) {

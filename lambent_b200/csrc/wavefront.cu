@@ -1646,7 +1646,8 @@ static bool sorts(const lam_pipeline* pl, bool guide, uint64_t paths) {
            (pl->shade_order == LAM_SHADE_ORDER_AUTO && !guide && paths >= SORT_MIN_PATHS);
 }
 
-static int ensure_wave(lam_pipeline* pl, uint32_t width, uint32_t height, bool full, bool guide, bool learned) {
+static int ensure_wave(lam_pipeline* pl, uint32_t width, uint32_t height, bool full, bool guide, bool learned,
+                       cudaStream_t st) {
     const uint32_t npix = width * height;
     uint32_t spp_wave = 1;
     if (!guide && pl->opts.restir_temporal != LAM_RESTIR_PER_SAMPLE) {
@@ -1699,7 +1700,8 @@ static int ensure_wave(lam_pipeline* pl, uint32_t width, uint32_t height, bool f
         capped = true;
     }
     w->mem_capped = capped;
-    cudaMemset(w->ctr, 0, CTR_WORDS * sizeof(uint32_t));
+    // in the render's stream: the legacy stream's work may come at any time between a non-blocking one's kernels
+    cudaMemsetAsync(w->ctr, 0, CTR_WORDS * sizeof(uint32_t), st);
     pl->total_segments = 0;
     pl->prof_segments_base = 0;
     cudaDeviceGetAttribute(&w->sms, cudaDevAttrMultiProcessorCount, pl->device);
@@ -2101,10 +2103,10 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
     const bool full = guide || restir != LAM_RESTIR_DISABLED;
     pl->stats_ctr = nullptr;  // the counters may move with the wave buffers
     pl->stats_pending = false;
-    int rc = ensure_wave(pl, tg->width, tg->height, full, guide, learned);
+    cudaStream_t st = (cudaStream_t)stream;
+    int rc = ensure_wave(pl, tg->width, tg->height, full, guide, learned, st);
     if (rc) return rc;
     WaveBuffers* w = pl->wave;
-    cudaStream_t st = (cudaStream_t)stream;
     Args A;
     std::memset(&A, 0, sizeof(A));
     A.S = s->dev;
@@ -2468,7 +2470,7 @@ static int batch_wave_buffers(BatchState* b, uint32_t capacity, bool order) {
         free_wave(w);
         return rc;
     }
-    cudaMemset(w->ctr, 0, CTR_WORDS * sizeof(uint32_t));
+    cudaMemsetAsync(w->ctr, 0, CTR_WORDS * sizeof(uint32_t), b->stream);
     b->wave = w;
     b->capacity = capacity;
     return LAM_OK;
@@ -2521,6 +2523,13 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
     t.wave_paths = std::max(t.wave_paths, max_pix);
     if (!pl->batch) pl->batch = new BatchState();
     BatchState* b = pl->batch;
+    cudaError_t e = cudaSuccess;
+    if (!b->stream) {
+        if ((e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking)) != cudaSuccess ||
+            (e = cudaEventCreateWithFlags(&b->ev_in, cudaEventDisableTiming)) != cudaSuccess ||
+            (e = cudaEventCreateWithFlags(&b->ev_out, cudaEventDisableTiming)) != cudaSuccess)
+            return cuda_error(e, "batch stream");
+    }
     pl->stats_ctr = nullptr;  // the counters may move with the batch buffers
     pl->stats_pending = false;
     const BatchPlan P = plan_batch(reqs, n, t.wave_paths);
@@ -2568,13 +2577,6 @@ extern "C" int lam_batch_render(lam_pipeline* pl, const lam_batch_request* reqs,
         q.out_color = (float4*)r.targets.color;
         q.out_normal = (float4*)r.targets.normal;
         q.out_albedo = (float4*)r.targets.albedo;
-    }
-    cudaError_t e = cudaSuccess;
-    if (!b->stream) {
-        if ((e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking)) != cudaSuccess ||
-            (e = cudaEventCreateWithFlags(&b->ev_in, cudaEventDisableTiming)) != cudaSuccess ||
-            (e = cudaEventCreateWithFlags(&b->ev_out, cudaEventDisableTiming)) != cudaSuccess)
-            return cuda_error(e, "batch stream");
     }
     cudaStream_t caller = (cudaStream_t)stream;
     cudaStream_t st = b->stream;
