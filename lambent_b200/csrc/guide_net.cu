@@ -715,9 +715,10 @@ static int guide_loss_grad(lam_guide* g, const float* recs, uint32_t n, const fl
     return LAM_OK;
 }
 
-// `steps` Adam steps on minibatches of options.batch records drawn from n (or *n_dev, if fewer).
+// `steps` Adam steps on minibatches of options.batch records drawn from n (or *n_dev, if fewer); counts its
+// kernels in *launches.
 int guide_train(lam_guide* g, const float* recs, uint32_t stride, uint32_t n, const uint32_t* n_dev, uint32_t steps,
-                const float box[6], cudaStream_t st) {
+                const float box[6], cudaStream_t st, uint32_t* launches) {
     int rc = setup_kernels(g);
     if (rc) return rc;
     net::TrainArgs T;
@@ -745,6 +746,7 @@ int guide_train(lam_guide* g, const float* recs, uint32_t stride, uint32_t n, co
             return s;
         });
         if (e != cudaSuccess) return cuda_error(e, "guide training launch");
+        ++*launches;
         g->steps += T.steps;
         steps -= T.steps;
     }
@@ -881,7 +883,8 @@ extern "C" int lam_guide_train(lam_guide* g, const lam_guide_record* records, ui
                                const float box[6], void* stream) {
     if (!g || !box || (n && !records)) return set_error(LAM_ERR_INVALID_ARGUMENT, "lam_guide_train: null argument");
     if (!n) return LAM_OK;
-    return guide_train(g, reinterpret_cast<const float*>(records), 13u, n, nullptr, steps, box, (cudaStream_t)stream);
+    uint32_t launches = 0;
+    return guide_train(g, reinterpret_cast<const float*>(records), 13u, n, nullptr, steps, box, (cudaStream_t)stream, &launches);
 }
 
 extern "C" int lam_guide_set_wait_limit(lam_guide* g, uint32_t tries) {

@@ -101,7 +101,7 @@ namespace lam {
 // path throughput and accumulated colour at the vertex, and the previous record of the same path.
 constexpr uint32_t GUIDE_RECORD_STRIDE = 20;
 int guide_train(lam_guide* g, const float* recs, uint32_t stride, uint32_t n, const uint32_t* n_dev, uint32_t steps,
-                const float box[6], cudaStream_t st);
+                const float box[6], cudaStream_t st, uint32_t* launches);
 int guide_check_error(const lam_guide* g);
 
 int set_intersection_handler(lam_tracer* t, const char* src);

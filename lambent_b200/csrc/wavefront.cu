@@ -2333,9 +2333,8 @@ extern "C" int lam_render(lam_pipeline* pl, const lam_scene* s, lam_data_buffers
         if (training) {
             h = begin(4);
             rc = guide_train(gd, gd->records, GUIDE_RECORD_STRIDE, gd->opts.record_capacity, w->ctr + CTR_RECORDS,
-                             gd->opts.steps_per_wave, s->bounds, st);
+                             gd->opts.steps_per_wave, s->bounds, st, &launches);
             if (rc) return rc;
-            ++launches;
             end(h);
             gd->trained_spp += A.wave_count;
         }

@@ -75,3 +75,23 @@ def test_parameters_are_always_those_of_whole_steps(cuda):
             assert e.code == _abi.ERR_DEVICE_TIMEOUT
             gave_up += 1
     assert gave_up
+
+
+def test_launch_count_of_a_training_render(cuda):
+    """A launch takes at most 64 Adam steps; kernel_launches counts each."""
+    import torch
+    from lambent_b200 import scenes
+    s = scenes.cornell_box(64, 64)
+    g = lb.GpuScene(s)
+    count = {}
+    for steps in (0, 1, 64, 65, 200):
+        guide = lb.Guide(lb.GuideOptions(steps_per_wave=steps, batch=128, record_capacity=4096, train_spp=2))
+        pipe = lb.RayTracer(lb.path_tracing.Medium).create_pipeline(*s.layout_counts(), lb.PathTracerOpts(
+            samples=2, restir_temporal=_abi.RESTIR_DISABLED, max_depth=3, guide_mode=_abi.GUIDE_LEARNED))
+        pipe.set_guide(guide)
+        col = torch.zeros((64, 64, 4), device="cuda")
+        pipe.render(g, lb.DataBuffers(64, 64, 1, 0), s.camera, lb.targets_from(col), 0)
+        torch.cuda.synchronize()
+        assert guide.progress()[0] == steps
+        count[steps] = pipe.stats().kernel_launches
+    assert [count[k] - count[0] for k in (1, 64, 65, 200)] == [1, 1, 2, 4]
