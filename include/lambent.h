@@ -456,7 +456,8 @@ int lam_trace_rays_static(const lam_scene* scene, const lam_ray* rays, uint32_t 
 /* DataBuffers::new, src/data_buffer/mod.rs:150-252 */
 int lam_data_buffers_new(uint32_t width, uint32_t height, uint32_t world_space_buffer_size,
                          uint32_t buffer_types, lam_data_buffers** out);
-/* DataBuffers::resize, src/data_buffer/mod.rs:259-267 */
+/* DataBuffers::resize, src/data_buffer/mod.rs:259-267.  A resize that fails leaves the buffers without a
+ * window: the passes over them return LAM_ERR_INVALID_ARGUMENT until one succeeds. */
 int lam_data_buffers_resize(lam_data_buffers* buffers, uint32_t width, uint32_t height);
 /* DataBuffers::advance_frame, src/data_buffer/mod.rs:272-349 (AdvanceOptions.confidence_cap) */
 int lam_data_buffers_advance_frame(lam_data_buffers* buffers, uint32_t buffers_to_advance,

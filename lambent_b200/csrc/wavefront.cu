@@ -1710,7 +1710,8 @@ static int ensure_wave(lam_pipeline* pl, uint32_t width, uint32_t height, bool f
     w->grid_extend = w->sms * std::max(1, occ);
     occ = 0;
     // the blocks of the shade form that these renders run: its grid-stride loop wants one resident round
-    // (a ReSTIR frame at 1080p 2,294 us, 2,535 with the plain form's count; guided 960x540 at 4 spp 2,492 / 2,688)
+    // (a ReSTIR frame at 1080p 2,294 us, 2,535 with the plain form's count; guided 960x540 at 4 spp 2,492 / 2,688).
+    // Markov-guided renders take the reservoir form's six, of which three of theirs are resident at a time
     const void* shade = full      ? (const void*)shade_kernel<LAM_QUALITY_MEDIUM, false, false, false, true>
                         : learned ? (const void*)shade_kernel<LAM_QUALITY_MEDIUM, false, true, false>
                                   : (const void*)shade_kernel<LAM_QUALITY_MEDIUM, false, false, false>;

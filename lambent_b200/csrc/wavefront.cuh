@@ -56,7 +56,7 @@ struct Args {
     float tmin, tmax;
     uint32_t wave_first, wave_count;
     uint64_t npix_m;         // ~0 / npix + 1: multiplier of pixel_of's division
-    uint32_t first;          // depth 0 of a wave whose generate kernel left only seeds and directions (first_ray)
+    uint32_t first;          // depth 0 of a wave whose generate kernel left only seeds and directions (load_ray)
     uint32_t pdf_at_sample;  // LAM_GUIDE_PDF_AT_SAMPLE: Markov mixture pdf with its cosine term at the chosen direction
     uint32_t guide_metal;    // LAM_GUIDE_METAL: the learned guide is mixed in at rough metallic vertices too
     // wave buffers
