@@ -95,3 +95,26 @@ def test_launch_count_of_a_training_render(cuda):
         assert guide.progress()[0] == steps
         count[steps] = pipe.stats().kernel_launches
     assert [count[k] - count[0] for k in (1, 64, 65, 200)] == [1, 1, 2, 4]
+
+
+@pytest.mark.parametrize("batch", [128 * 100, 128 * 148])
+def test_guides_trained_in_two_streams(cuda, batch):
+    """Each launch fills most of the device with blocks that wait for one another: two at a time run, one
+    after the other or side by side, and neither waits for blocks that cannot start."""
+    import torch
+    rec = records(5000)
+    opts = lb.GuideOptions(batch=batch, record_capacity=0, seed=3)
+    want = lb.Guide(opts)
+    for _ in range(8):
+        want.train(rec, 8, BOX)
+    torch.cuda.synchronize()
+    guides, streams = [lb.Guide(opts) for _ in range(2)], [torch.cuda.Stream() for _ in range(2)]
+    for g in guides:
+        g.set_wait_limit(1 << 16)  # a second or two, should they hold each other up
+    for _ in range(8):
+        for g, st in zip(guides, streams):
+            g.train(rec, 8, BOX, stream=st)
+    torch.cuda.synchronize()
+    for g in guides:
+        assert g.progress() == (64, 0)
+        np.testing.assert_array_equal(np.array(g.params()), np.array(want.params()))
