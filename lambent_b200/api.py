@@ -755,8 +755,8 @@ class Guide:
                                     _stream_ptr(stream)))
 
     def set_wait_limit(self, tries):
-        """Polls of a tensor-core completion barrier before a wait gives up (lam_guide_set_wait_limit);
-        0 makes every wait give up at once."""
+        """Polls of a tensor-core completion barrier before a wait gives up (lam_guide_set_wait_limit); the
+        training kernel's meetings scale with it.  0 makes every wait give up at once."""
         check(lib().lam_guide_set_wait_limit(self._h, int(tries)))
 
     def progress(self):
